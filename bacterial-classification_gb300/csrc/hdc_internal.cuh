@@ -60,6 +60,14 @@ struct hdc_refdb {
     int32_t limb_max[4] = {0, 0, 0, 0};
     int limb_bits = 11;         // limbs are balanced base-2^limb_bits digits (the top one within the cap)
     int32_t max_abs = 0;
+    // The same references for the single-accumulator search, beside the limbs where the values allow it and memory
+    // is left (null otherwise: the limbs serve): base-8 digit tiles for +1/-1 queries, or one fp16 row each for
+    // count-valued queries.
+    void* d_digits = nullptr;
+    int digits = 0;
+    __half* d_rows16 = nullptr;  // d_limbs itself when one limb holds every value
+    int32_t value_max = 0;       // largest |value| and squared norm, measured
+    int64_t norm2_max = 0;
 };
 
 namespace hdc {
@@ -83,7 +91,9 @@ int launch_pack_2bit(hdc_context* ctx, const char* d_bytes, int64_t n_bytes, uin
 int launch_norms(hdc_context* ctx, const void* d_hv, int elem_bytes, int64_t n, int64_t* d_norm2,
                  int32_t* d_maxabs, cudaStream_t stream);
 
+// what the tensor cores take (the most of their forms), and what the CUDA-core kernel needs at least
 size_t plain_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k);
+size_t plain_min_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k);
 
 int launch_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, int64_t nq, int32_t maxq,
                         const int16_t* d_r, const int64_t* d_rn, int64_t nr, int32_t maxr, int k, int mode,
@@ -112,6 +122,9 @@ int tc_default_share();
 int tc_default_scatter();
 int tc_default_kblock();
 int tc_default_pair_mma();
+// Build the forms of the single-accumulator search from the limbs (synchronizes the stream); a form that does not fit
+// in memory is left out.
+int refdb_forms(hdc_refdb* db, cudaStream_t stream);
 // Fill db->d_sqrt (allocated here) from db->d_norm2.
 int refdb_sqrt_table(hdc_refdb* db, cudaStream_t stream);
 int tc_default_tile_n();

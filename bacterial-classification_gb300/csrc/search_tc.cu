@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "hdc_internal.cuh"
+#include "search_mm.cuh"
 #include "tc_ptx.cuh"
 #include "topk.cuh"
 
@@ -751,6 +752,14 @@ __global__ void sqrt_kernel(const int64_t* __restrict__ n2, int64_t n, double* _
     }
 }
 
+__global__ void norm2_max_kernel(const int64_t* __restrict__ n2, int64_t n, unsigned long long* __restrict__ out) {
+    unsigned long long m = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        m = max(m, (unsigned long long)n2[i]);
+    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
 // cuTensorMapEncodeTiled resolved through the runtime, so the library does not
 // link libcuda (it must load on hosts without a driver).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -854,6 +863,7 @@ int refdb_create(hdc_context* ctx, const void* d_ref, int elem_bytes, int64_t nr
         if (e != cudaSuccess) st = cuda_fail(e, "refdb: build");
     }
     cudaFree(d_lmax);
+    if (st == HDC_OK) st = refdb_forms(db, stream);
     if (st != HDC_OK) {
         refdb_destroy(db);
         return st;
@@ -868,7 +878,56 @@ void refdb_destroy(hdc_refdb* db) {
     cudaFree(db->d_norm2);
     cudaFree(db->d_rsq);
     cudaFree(db->d_sqrt);
+    cudaFree(db->d_digits);
+    if (db->d_rows16 != db->d_limbs) cudaFree(db->d_rows16);
     delete db;
+}
+
+int refdb_forms(hdc_refdb* db, cudaStream_t stream) {
+    int64_t* d_max = nullptr;  // the largest value (int32) and the largest squared norm
+    cudaError_t e = cudaMalloc(&d_max, 2 * sizeof(int64_t));
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, 2 * sizeof(int64_t), stream);
+    int st = e == cudaSuccess ? mm_limbs_max(db->d_limbs, db->L, db->limb_bits, db->r_pad, db->dim,
+                                             reinterpret_cast<int32_t*>(d_max), stream)
+                              : cuda_fail(e, "refdb: allocation");
+    if (st == HDC_OK) {
+        norm2_max_kernel<<<(unsigned)std::min<int64_t>((db->nr + 255) / 256, 256), 256, 0, stream>>>(
+            db->d_norm2, db->nr, reinterpret_cast<unsigned long long*>(d_max + 1));
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&db->value_max, d_max, sizeof(int32_t), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&db->norm2_max, d_max + 1, sizeof(int64_t), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) st = cuda_fail(e, "refdb: largest value");
+    }
+    cudaFree(d_max);
+    if (st != HDC_OK) return st;
+    if (db->L == 1) db->d_rows16 = db->d_limbs;
+    // base-2048 limbs are a database for +1/-1 queries, smaller bases one for counts
+    if (db->limb_bits == 11) {
+        const int digits = mm_f4_limbs(db->value_max);
+        const size_t bytes = digits ? mm_f4_ref_bytes(db->nr, db->dim, digits) : 0;
+        if (!digits || bytes / 64 > 0x7fffffff) return HDC_OK;  // TMA coordinates are 32-bit
+        if (cudaMalloc(&db->d_digits, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            db->d_digits = nullptr;
+            return HDC_OK;
+        }
+        db->digits = digits;
+        st = mm_pack_refs(nullptr, db->d_limbs, db->L, db->limb_bits, db->r_pad, db->nr, db->dim, digits, db->d_digits,
+                          stream);
+    } else if (db->L > 1 && db->value_max <= 2048) {
+        if (cudaMalloc(&db->d_rows16, (size_t)db->r_pad * db->dim * sizeof(__half)) != cudaSuccess) {
+            cudaGetLastError();
+            db->d_rows16 = nullptr;
+            return HDC_OK;
+        }
+        st = mm_rows_from_limbs(db->d_limbs, db->L, db->limb_bits, db->r_pad, db->dim, db->d_rows16, stream);
+    }
+    if (st == HDC_OK) {
+        e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) st = cuda_fail(e, "refdb: search forms");
+    }
+    return st;
 }
 
 int refdb_sqrt_table(hdc_refdb* db, cudaStream_t stream) {
@@ -1019,8 +1078,53 @@ static int64_t tc_quad_queries(const hdc_context* ctx, int64_t nq, const hdc_ref
     return nq / rows * rows;
 }
 
+// The single-accumulator search (search_mm.cu) is the automatic schedule wherever the database has a form for the
+// queries; the schedule settings below belong to the limb search, so setting any of them to other than its automatic
+// value (128 references a tile) selects it.
+static bool tc_auto_schedule(const hdc_context* ctx) {
+    return ctx->tc_group == 0 && ctx->tc_policy < 0 && (ctx->tc_tile_n == 0 || ctx->tc_tile_n == 128) && ctx->tc_m_blocks == 0 &&
+           ctx->tc_prefetch < 0 && ctx->tc_cluster == 0 && ctx->tc_share < 0 && ctx->tc_kblock == 0 &&
+           ctx->tc_pair_mma < 0 && ctx->tc_lanes == 0;
+}
+
+// The operand form for queries of magnitude up to maxq, or none: +1/0/-1 queries on the base-8 digits, others on the
+// fp16 rows while a K block's sums stay within 2^24 and a dot within int32.
+static bool mm_form(const hdc_context* ctx, const hdc_refdb* db, int64_t nq, int32_t maxq, MmOperands& op) {
+    if (!tc_auto_schedule(ctx)) return false;
+    const bool f4 = maxq <= 1 && db->d_digits;
+    op.f4 = f4;
+    op.limbs = f4 ? db->digits : 1;
+    op.b = f4 ? db->d_digits : static_cast<const void*>(db->d_rows16);
+    op.ldb = db->dim;
+    op.sum_per_dim = f4 ? mm_f4_sum_per_dim(db->value_max) : (int64_t)std::max(maxq, 1) * std::max(db->value_max, 1);
+    // digits: |q|^2 <= dim; the fp16 rows' queries are measured by the call
+    op.one_segment = f4 && (double)db->dim * (double)db->norm2_max <= mm_f4_norm_limit(op.limbs, db->dim);
+    op.rr = db->d_rsq;
+    op.rs = db->d_sqrt;
+    op.ri = db->d_sqrt + db->nr;
+    if (!op.b || !mm_sums_fit(f4, op.sum_per_dim) || op.sum_per_dim * db->dim > 0x7fffffff) return false;
+    return !f4 || mm_f4_query_bytes(nq, db->dim) / 64 <= 0x7fffffff;
+}
+
+// Workspace of that search: the packed queries (digits only), then its lists.
+static size_t mm_workspace(const hdc_context* ctx, const hdc_refdb* db, int64_t nq, int k, const MmOperands& op) {
+    return (op.f4 ? mm_f4_query_bytes(nq, db->dim) : 0) +
+           mm_list_bytes(ctx, nq, db->nr, db->dim, k, op.f4, op.limbs);
+}
+
+static size_t limb_workspace_bytes(const hdc_context* ctx, int64_t nq, const hdc_refdb* db, int k);
+
 size_t tc_workspace_bytes(const hdc_context* ctx, int64_t nq, const hdc_refdb* db, int k) {
     k = std::max(1, (int)std::min<int64_t>(k, db->nr));
+    size_t need = limb_workspace_bytes(ctx, nq, db, k);
+    for (int32_t maxq = 1; maxq <= 2; ++maxq) {  // the two operand forms
+        MmOperands op;
+        if (k <= kMaxKTC && mm_form(ctx, db, nq, maxq, op)) need = std::max(need, mm_workspace(ctx, db, nq, k, op));
+    }
+    return need;
+}
+
+static size_t limb_workspace_bytes(const hdc_context* ctx, int64_t nq, const hdc_refdb* db, int k) {
     int G4, S4;
     const int64_t n4 = tc_quad_queries(ctx, nq, db, k, G4, S4);
     if (n4 == nq) return tc_part_bytes(tc_plan(ctx, nq, db), nq, k);
@@ -1226,6 +1330,8 @@ static int quad_clusters_fit(const hdc_context* ctx) {
     return fit;
 }
 
+static bool aligned256(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 255) == 0; }
+
 int launch_search_tc(hdc_context* ctx, const hdc_refdb* db, const __half* d_q, const int64_t* d_qn, int64_t nq,
                      int32_t maxq, int k, int mode, float* d_score, int32_t* d_idx, double* d_cos, int64_t* d_dot,
                      void* d_work, size_t work_bytes, int* d_status, cudaStream_t stream) {
@@ -1240,6 +1346,33 @@ int launch_search_tc(hdc_context* ctx, const hdc_refdb* db, const __half* d_q, c
             return fail(HDC_ERR_RANGE, "tc search: dim * max|q| * max|limb| exceeds 2^24 (fp32 accumulators inexact)");
     }
     if ((reinterpret_cast<uintptr_t>(d_q) & 15) != 0) return fail(HDC_ERR_INVALID, "tc search: queries not 16B aligned");
+    MmOperands op;
+    if (mm_form(ctx, db, nq, maxq, op) && d_work && aligned256(d_work) && work_bytes >= mm_workspace(ctx, db, nq, k, op)) {
+        void* lists = d_work;
+        int st = HDC_OK;
+        if (op.f4) {
+            st = mm_pack_queries(d_q, true, nq, ctx->dim, d_work, stream);
+            op.a = d_work;
+            lists = static_cast<uint8_t*>(d_work) + mm_f4_query_bytes(nq, ctx->dim);
+        } else {
+            op.a = d_q;
+            op.lda = ctx->dim;
+        }
+        op.qn = d_qn;
+        if (st == HDC_OK) st = mm_begin(lists, nq, stream);
+        if (st == HDC_OK && !op.f4) {
+            unsigned long long* words = static_cast<unsigned long long*>(lists);
+            st = mm_norm_max(d_q, nq, ctx->dim, (unsigned long long)db->norm2_max, words, stream);
+            op.q_norm_max = words;
+            op.r_norm_max = words + 1;
+        }
+        if (st == HDC_OK)
+            st = mm_search(ctx, op, nq, db->nr, 0, db->nr, ctx->dim, k, mode, lists, true, ctx->tc_last_shape, stream);
+        ctx->tc_last_shape[4] = 3;  // packing or the queries' largest norm, search, merge
+        if (st != HDC_OK) return st;
+        return mm_finish(ctx, nq, db->nr, db->nr, ctx->dim, k, op.f4, op.limbs, d_qn, db->d_norm2, lists, d_score, d_idx,
+                         d_cos, d_dot, stream);
+    }
     int G4, S4;
     const int64_t n4 = tc_quad_queries(ctx, nq, db, k, G4, S4);
     if (n4 == nq)

@@ -191,6 +191,19 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_
         : "memory");
 }
 
+// D[tmem] (+)= (A * 2^sa) (B * 2^sb)^T with packed e2m1 operands (K = 64), one power-of-two
+// scale per row and 32 dims from tensor memory (ue8m0 bytes at sfa / sfb), fp32 accumulators.
+__device__ __forceinline__ void mma_f4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
+                                       uint32_t sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%5], p;\n\t}\n" ::"r"(
+            tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+        : "memory");
+}
+
 // Arrive on `bar` once every previously issued tcgen05.mma of this thread completes.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -309,6 +322,18 @@ __device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t adesc, ui
         : "memory");
 }
 
+// mma_f4 over a CTA pair (rows as mma_f16_pair); each CTA's tensor memory holds the scales.
+__device__ __forceinline__ void mma_f4_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%5], p;\n\t}\n" ::"r"(
+            tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+        : "memory");
+}
+
 // Arrive on the mbarrier at `bar`'s offset in every CTA of cta_mask once the
 // pair MMAs issued so far complete.
 __device__ __forceinline__ void mma_commit_pair_mc(uint64_t* bar, uint16_t cta_mask) {
@@ -363,6 +388,15 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
+// 16 consecutive columns, as tmem_st32.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 // This thread's tcgen05.st have completed.
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -401,6 +435,14 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int m, int n) {
            | (0u << 7) | (0u << 10)         // A, B format: f16
            | (0u << 15) | (0u << 16)        // A, B K-major
            | ((uint32_t)(n >> 3) << 17)     // N / 8
+           | ((uint32_t)(m >> 4) << 24);    // M / 16
+}
+
+// Instruction descriptor of kind::mxf4: e2m1 A and B, ue8m0 scales, fp32 D, both operands K-major, M x N, K = 64.
+__host__ __device__ constexpr uint32_t idesc_f4_f32(int m, int n) {
+    return (1u << 7) | (1u << 10)            // A, B format: e2m1
+           | ((uint32_t)(n >> 3) << 17)     // N / 8
+           | (1u << 23)                      // scales: ue8m0
            | ((uint32_t)(m >> 4) << 24);    // M / 16
 }
 
