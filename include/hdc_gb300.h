@@ -155,11 +155,14 @@ int hdc_norms(hdc_context* ctx, const void* d_hv, int elem_bytes, int64_t n, int
 /* The same for integer-valued fp16 rows (HDC_OUT_F16 / HDC_OUT_BIPOLAR_F16 queries). */
 int hdc_norms_f16(hdc_context* ctx, const void* d_hv, int64_t n, int64_t* d_norm2, int32_t* d_maxabs, void* stream);
 
-/* Workspace the plain search needs for nq queries and top-k. */
+/* Workspace of the plain search for nq queries and top-k (at most 2 GiB beyond
+ * its partial lists): with all of it the search runs on the tensor cores where
+ * the values allow; a smaller one that holds the partial lists of the CUDA-core
+ * kernel is accepted too, and takes that kernel. */
 size_t hdc_search_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k);
 
 /* Plain form: exact integer cosine top-k of int16 queries against int16
- * references on CUDA cores, the drop-in for launch_cosine_topk
+ * references, the drop-in for launch_cosine_topk
  * (src/cosine.cu:441-496) and, with k = 1, launch_cosine_argmax
  * (src/cosine.cu:172-222).  For every query: the k best references by the
  * float score of score_mode (descending), ties to the lower reference index.
@@ -168,7 +171,10 @@ size_t hdc_search_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr
  * optional), d_dot (int64 exact dot; optional).  max_abs_q / max_abs_r bound
  * |element| of queries / references (from hdc_norms); products must satisfy
  * max_abs_q * max_abs_r <= 2^20 (else HDC_ERR_RANGE).  d_qnorm2 / d_rnorm2 come from hdc_norms.
- * d_work must hold hdc_search_workspace_bytes(nq, nr, k) bytes. */
+ * d_work must hold hdc_search_workspace_bytes(nq, nr, k) bytes (256-byte
+ * aligned).  Rows of |v| <= 2048 (and +1/0/-1 queries against |r| <= 18724) are
+ * converted in the workspace and searched on the tensor cores, exactly; larger
+ * values take CUDA cores. */
 int hdc_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, int64_t nq,
                      int32_t max_abs_q, const int16_t* d_r, const int64_t* d_rnorm2, int64_t nr,
                      int32_t max_abs_r, int k, int score_mode, float* d_score, int32_t* d_idx,
@@ -244,7 +250,8 @@ int hdc_search_tc(hdc_context* ctx, const hdc_refdb* db, const void* d_q, const 
  * synchronisation cudaMalloc / cudaFree imply.
  *
  * Limits and behaviour:
- *   - a batch whose workspace (hdc_search_workspace_bytes) exceeds
+ *   - a batch whose partial lists (16 bytes x k x queries x reference ranges,
+ *     about two ranges per SM and query tile) exceed
  *     HDC_NOALLOC_SCRATCH_BYTES is rejected with HDC_ERR_RANGE and a message
  *     naming both sizes; pass fewer queries per call;
  *   - k is checked first (1..32 after clamping to nr, else HDC_ERR_INVALID,
