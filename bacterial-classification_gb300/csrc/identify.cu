@@ -23,16 +23,20 @@
 // One CTA per read: the read's int16 hypervector is staged in shared memory
 // once, and the CTA's warps split each candidate node's rows (coalesced
 // 16-byte loads of a row per warp step); dots are exact int64.
+#include <algorithm>
+
 #include "hdc_internal.cuh"
+#include "identify.cuh"
 #include "topk.cuh"
 
 namespace hdc {
 namespace {
 
-constexpr int kMaxBeam = 8;
-constexpr int kMaxLevels = 8;
+constexpr int kMaxBeam = kIdBeam;
+constexpr int kMaxLevels = kIdLevels;
 constexpr int kIdWarps = 8;
 constexpr int kSimWarps = 8;
+constexpr int64_t kIdBatch = 65536;  // reads of a grouped pass
 
 // exact dot of an int16 row (global) with an int16 vector (shared or global),
 // one warp; dim % 8 == 0 and both 16-byte aligned.  NARROW: every partial sum
@@ -82,24 +86,6 @@ struct Entry {
     int32_t parent_slot;
 };
 
-struct IdentifyArgs {
-    const int16_t* q;         // [nq][dim] whole-read hypervectors
-    const int64_t* qn;        // [nq]
-    const int16_t* rows;      // [n_rows][dim] similarity rows
-    const int64_t* rn;        // [n_rows]
-    const int64_t* node_rows; // [n_nodes+1] CSR: node -> its rows
-    const int64_t* child_ptr;
-    const int32_t* child_idx;
-    const int32_t* roots;
-    int n_roots;
-    int dim, levels, beam, mode;
-    double threshold;
-    int32_t* path;            // [nq][levels]
-    float* path_score;        // [nq][levels]
-    int32_t* depth;           // [nq]
-    int32_t* stop_level;      // [nq] level of an early stop, -1 when all levels ran (may be null)
-};
-
 __global__ void __launch_bounds__(32 * kIdWarps) identify_kernel(const IdentifyArgs a) {
     extern __shared__ __align__(16) int16_t qs[];
     __shared__ int32_t paths[kMaxBeam][kMaxLevels];
@@ -109,6 +95,7 @@ __global__ void __launch_bounds__(32 * kIdWarps) identify_kernel(const IdentifyA
     __shared__ int n_beam_s, done_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r = blockIdx.x;
+    if (a.only_if && *a.only_if == 0) return;
     {
         const uint4* src = reinterpret_cast<const uint4*>(a.q + r * a.dim);
         uint4* dst = reinterpret_cast<uint4*>(qs);
@@ -294,11 +281,24 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
         cudaError_t e = cudaFuncSetAttribute(identify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return cuda_fail(e, "identify: shared memory attribute");
     }
-    IdentifyArgs a{d_q, d_qn, d_rows, d_rn, d_node_rows, d_child_ptr, d_child_idx, d_roots, n_roots, ctx->dim,
-                   levels, beam, mode, threshold, d_path, d_path_score, d_depth, d_stop_level};
-    identify_kernel<<<(unsigned)nq, 32 * kIdWarps, smem, stream>>>(a);
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? HDC_OK : cuda_fail(e, "identify: launch");
+    // Batches of reads grouped by parent on the tensor cores, each followed by the per-read kernel for what does not
+    // fit there (it exits at once otherwise).
+    for (int64_t r0 = 0; r0 < nq; r0 += kIdBatch) {
+        const int64_t n = std::min(kIdBatch, nq - r0);
+        IdentifyArgs a{d_q + r0 * ctx->dim, d_qn + r0, d_rows, d_rn, d_node_rows, d_child_ptr, d_child_idx, d_roots, n_roots,
+                       ctx->dim, levels, beam, mode, threshold, d_path + r0 * levels, d_path_score + r0 * levels,
+                       d_depth + r0, d_stop_level ? d_stop_level + r0 : nullptr, nullptr};
+        int32_t* flag = nullptr;
+        void* ws = nullptr;
+        int st = launch_identify_grouped(ctx, a, n, &flag, &ws, stream);
+        if (st != HDC_OK) return st;
+        a.only_if = flag;
+        identify_kernel<<<(unsigned)n, 32 * kIdWarps, smem, stream>>>(a);
+        cudaError_t e = cudaGetLastError();
+        if (ws) cudaFreeAsync(ws, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "identify: launch");
+    }
+    return HDC_OK;
 }
 
 int launch_similarity(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, const int16_t* d_rows,
