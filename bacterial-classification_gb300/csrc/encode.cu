@@ -21,12 +21,10 @@
 //     also carries the all-ones start value.  A binder word is the XOR of
 //     one 128 W-byte table row per part (conflict-free: the 32 lanes read the
 //     32 W words of one row).
-//   * Per chunk of kChunk positions each lane computes kChunk / 32 canonical
-//     k-mers with a rolling 2-bit code (revcomp = bitwise NOT of the
-//     little-endian code, forward = digit reversal), and writes one entry per
-//     position: the byte offsets of its table rows, so a row's address is one
-//     add.  Invalid k-mers and the chunk tail point at an all-zero row, which
-//     contributes nothing.
+//   * Per chunk of 256 positions the warp turns its bases into bit planes
+//     (ballots); a lane's k-mer is a funnel shift of them, its reverse complement
+//     an inversion and a bit reversal, and the entries of the valid ones (a byte
+//     per digit part) are collected in shared memory, 16 to a bundling step.
 //   * Bundling never unpacks bits: 16 binder words are reduced by a
 //     carry-save adder tree into bit-sliced counters (ones/twos/fours/eights
 //     plus NH higher planes), ~2 logic ops per word; counts are extracted
@@ -34,6 +32,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "hdc_internal.cuh"
 
@@ -42,9 +41,10 @@ namespace {
 
 constexpr int kWarps = 24;
 constexpr int kThreads = kWarps * 32;
-constexpr int kChunk = 64;  // positions per staged chunk
-constexpr int kPerLane = kChunk / 32;
 constexpr int kMaxParts = 4;
+constexpr int kChunk = 256;  // positions per staged chunk
+constexpr int kPerLane = kChunk / 32;
+constexpr int kList = kChunk + 16;  // entries a warp holds: a chunk's and fewer than a group left of the one before
 constexpr size_t kMaxEncodeSmem = 227 * 1024;  // dynamic shared memory a CTA may opt into
 
 struct EncodeArgs {
@@ -54,7 +54,6 @@ struct EncodeArgs {
     int part_first[kMaxParts];  // first digit (0 = first base of the canonical k-mer)
     int part_len[kMaxParts];
     int part_row0[kMaxParts];
-    int zero_row;
     int table_rows;
     const unsigned char* bytes;
     // 2-bit packed input (when set, instead of bytes): base i of the stream at bits 2 (i % 16)
@@ -67,6 +66,7 @@ struct EncodeArgs {
     int64_t n_seqs;
     int window, step;
     int64_t n_segs;
+    uint32_t row_bytes;  // of the table: 128 W
     int out_kind;
     void* out;
     int64_t out_stride;
@@ -102,29 +102,35 @@ __device__ __forceinline__ void get_segment(const EncodeArgs& a, int64_t g, int6
     len = a.window;
 }
 
-// 2-bit code of an ASCII byte (A=0 C=1 G=2 T=3) and whether it is a base.
+// 2-bit code of an ASCII base (A=0 C=1 G=2 T=3).
 __device__ __forceinline__ uint32_t base_code(uint32_t c) { return ((c >> 1) ^ (c >> 2)) & 3u; }
-__device__ __forceinline__ uint32_t is_base(uint32_t c) {
-    return (c == 'A') | (c == 'C') | (c == 'G') | (c == 'T');
+// A k-mer window as bit planes: bit i of lo / hi is the low / high bit of its base i's code.
+struct Planes {
+    uint32_t lo, hi;
+};
+
+// The canonical one of a k-mer and its reverse complement (both planes inverted and bit-reversed): the smaller as a
+// number with base 0 in the most significant digit, decided at the first base where they differ.
+__device__ __forceinline__ Planes canonical(Planes f, int k, uint32_t mask) {
+    const Planes r{__brev(~f.lo & mask) >> (32 - k), __brev(~f.hi & mask) >> (32 - k)};
+    const uint32_t diff = (f.lo ^ r.lo) | (f.hi ^ r.hi);
+    const uint32_t at = diff & (0u - diff);  // the first differing base (none: a palindrome, equal either way)
+    // there: f below r when hi says so, or hi is equal and lo says so
+    const uint32_t below = (~f.hi & r.hi) | (~(f.hi ^ r.hi) & ~f.lo & r.lo);
+    return (below & at) ? f : r;
 }
 
-// A position's table rows, one per digit part, as byte offsets from the start of the table
-// (parts past NP and invalid k-mers point at the all-zero row).
-template <int NP, int W>
-__device__ __forceinline__ uint4 pack_entry(const EncodeArgs& a, uint32_t canon) {
-    constexpr uint32_t kRowBytes = 128u * W;
-    uint32_t f[kMaxParts];
+// A position's table rows, one byte per digit part: the row within the part, its bases' high bits, then their low bits.
+template <int NP>
+__device__ __forceinline__ uint32_t pack_entry(const EncodeArgs& a, Planes c) {
+    uint32_t e = 0;
 #pragma unroll
-    for (int p = 0; p < kMaxParts; ++p) {
-        uint32_t row = (uint32_t)a.zero_row;
-        if (p < NP) {
-            const int len = a.part_len[p];
-            const int shift = 2 * (a.k - a.part_first[p] - len);
-            row = (uint32_t)a.part_row0[p] + ((canon >> shift) & ((1u << (2 * len)) - 1u));
-        }
-        f[p] = row * kRowBytes;
+    for (int p = 0; p < NP; ++p) {
+        const int len = a.part_len[p];
+        const uint32_t m = (1u << len) - 1u;
+        e |= ((((c.hi >> a.part_first[p]) & m) << len) | ((c.lo >> a.part_first[p]) & m)) << (8 * p);
     }
-    return make_uint4(f[0], f[1], f[2], f[3]);
+    return e;
 }
 
 // W consecutive words of a table row from shared memory (32-bit shared address)
@@ -142,8 +148,10 @@ __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&v)[W]) {
 template <int NH>
 __device__ __forceinline__ void write_word(const EncodeArgs& a, int64_t seg, int w32, int nvalid, uint32_t ones,
                                            uint32_t twos, uint32_t fours, uint32_t eights, const uint32_t (&hi)[NH]) {
-    if (a.out_kind == HDC_OUT_SIGN_BITS) {
-        // a row has ceil(dim / 32) words: a word that starts at or past dim writes nothing
+    const int kind = a.out_kind;
+    if (kind == HDC_OUT_SIGN_BITS || kind == HDC_OUT_BIPOLAR_BF16 || kind == HDC_OUT_BIPOLAR_I16 ||
+        kind == HDC_OUT_BIPOLAR_F16 || kind == HDC_OUT_BIPOLAR_I8) {
+        // rows of ceil(dim / 32) words: a word that starts at or past dim writes nothing
         // (the ring of 64-bit words can hold one more 32-bit word than that)
         if (w32 * 32 >= a.dim) return;
         // 2 count - nvalid >= 0, i.e. count >= ceil(nvalid / 2), compared plane by plane
@@ -167,7 +175,47 @@ __device__ __forceinline__ void write_word(const EncodeArgs& a, int64_t seg, int
         uint32_t bits = gt | eq;
         const int nd = min(32, a.dim - w32 * 32);
         if (nd < 32) bits &= (1u << nd) - 1u;
-        reinterpret_cast<uint32_t*>(a.out)[seg * a.out_stride + w32] = bits;
+        if (kind == HDC_OUT_SIGN_BITS) {
+            reinterpret_cast<uint32_t*>(a.out)[seg * a.out_stride + w32] = bits;
+            return;
+        }
+        // +1 / -1 elements straight from the sign bits (extracting the counts first would take ~700 instructions a word)
+        const uint32_t neg = ~bits;
+        if (kind == HDC_OUT_BIPOLAR_I8) {
+            int8_t* o = static_cast<int8_t*>(a.out) + seg * a.out_stride + w32 * 32;
+            uint32_t pk[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)  // four sign bits to the low bits of four bytes; 1 -> 0xff, 0 -> 0x01
+                pk[q] = 0x01010101u | ((((neg >> (4 * q)) & 15u) * 0x00204081u) & 0x01010101u) * 0xffu;
+            if (nd == 32 && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
+                reinterpret_cast<uint4*>(o)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                reinterpret_cast<uint4*>(o)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+            } else {
+#pragma unroll
+                for (int b = 0; b < 32; ++b)
+                    if (b < nd) o[b] = (int8_t)(pk[b >> 2] >> (8 * (b & 3)));
+            }
+            return;
+        }
+        uint16_t* o = static_cast<uint16_t*>(a.out) + seg * a.out_stride + w32 * 32;
+        // two's complement: 1 -> 0xffff; floats: the sign bit of the constant
+        const uint32_t one = kind == HDC_OUT_BIPOLAR_I16 ? 0x00010001u : kind == HDC_OUT_BIPOLAR_F16 ? 0x3c003c00u : 0x3f803f80u;
+        const uint32_t flip = kind == HDC_OUT_BIPOLAR_I16 ? 0xfffeu : 0x8000u;
+        uint32_t pk[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const uint32_t two = neg >> (2 * q);
+            pk[q] = one ^ (((two & 1u) | ((two & 2u) << 15)) * flip);
+        }
+        if (nd == 32 && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                reinterpret_cast<uint4*>(o)[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+        } else {
+#pragma unroll
+            for (int b = 0; b < 32; ++b)
+                if (b < nd) o[b] = (uint16_t)(pk[b >> 1] >> (16 * (b & 1)));
+        }
         return;
     }
 
@@ -203,24 +251,6 @@ __device__ __forceinline__ void write_word(const EncodeArgs& a, int64_t seg, int
             for (int b = 0; b < 32; ++b)
                 if (b < nd) o[b] = 2 * (int)val[b] - nvalid;
         }
-    } else if (a.out_kind == HDC_OUT_BIPOLAR_I8) {
-        int8_t* o = reinterpret_cast<int8_t*>(rowp) + seg * a.out_stride + dbase;
-        uint32_t pk[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            pk[q] = 0;
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                pk[q] |= (2 * (int)val[4 * q + t] - nvalid >= 0 ? 0x01u : 0xffu) << (8 * t);
-        }
-        if (nd == 32 && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
-            reinterpret_cast<uint4*>(o)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            reinterpret_cast<uint4*>(o)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-        } else {
-#pragma unroll
-            for (int b = 0; b < 32; ++b)
-                if (b < nd) o[b] = (int8_t)(pk[b >> 2] >> (8 * (b & 3)));
-        }
     } else {
         uint16_t* o = reinterpret_cast<uint16_t*>(rowp) + seg * a.out_stride + dbase;
         uint32_t pk[16];
@@ -230,16 +260,8 @@ __device__ __forceinline__ void write_word(const EncodeArgs& a, int64_t seg, int
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
                 const int v = 2 * (int)val[2 * q + t] - nvalid;
-                if (a.out_kind == HDC_OUT_I16)
-                    h2[t] = (uint32_t)v & 0xffffu;
-                else if (a.out_kind == HDC_OUT_BIPOLAR_I16)
-                    h2[t] = v >= 0 ? 0x0001u : 0xffffu;
-                else if (a.out_kind == HDC_OUT_BIPOLAR_F16)
-                    h2[t] = v >= 0 ? 0x3c00u : 0xbc00u;  // fp16 +1 / -1
-                else if (a.out_kind == HDC_OUT_F16)
-                    h2[t] = __half_as_ushort(__int2half_rn(v));  // exact: |v| <= 2048
-                else
-                    h2[t] = v >= 0 ? 0x3f80u : 0xbf80u;  // bf16 +1 / -1
+                // fp16 is exact here: |v| <= 2048
+                h2[t] = a.out_kind == HDC_OUT_I16 ? (uint32_t)v & 0xffffu : __half_as_ushort(__int2half_rn(v));
             }
             pk[q] = h2[0] | (h2[1] << 16);
         }
@@ -255,14 +277,19 @@ __device__ __forceinline__ void write_word(const EncodeArgs& a, int64_t seg, int
     }
 }
 
-// W: words a lane owns (a slab is 32 W words; W = 2 halves the per-position work of the
-// entries, addresses and k-mer staging per word, where the wider table fits shared memory)
+// W: words a lane owns (a slab is 32 W words; W = 2 halves the per-position work of the entries, addresses and k-mer
+// staging per word, where the wider table fits shared memory).
+//
+// Bound by shared-memory wavefronts: a position's NP rows take 2 NP of them at W = 2 (128 bytes each), so an entry is
+// four bytes, four entries a load (as 16-byte offsets read one by one they took 2 more: 8.07 a position, 88 % of the
+// pipe busy).  The logic pipe comes next (57 %): a row's address is a byte permute and a multiply-add on the FMA pipe.
+// Ordering a chunk's entries by their third part, to read its row only when it changes, was not faster.
 template <int NP, int NH, int W>
 __global__ void __launch_bounds__(kThreads) encode_kernel(const EncodeArgs a) {
     extern __shared__ __align__(16) uint32_t smem[];
     constexpr int SW = 32 * W;  // words per slab
     uint32_t* table = smem;     // [table_rows][SW]
-    uint4* lists = reinterpret_cast<uint4*>(smem + a.table_rows * SW);
+    uint32_t* lists = smem + a.table_rows * SW;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int slab = blockIdx.y;
 
@@ -270,14 +297,14 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const EncodeArgs a) {
     for (int e = threadIdx.x; e < a.table_rows * SW; e += kThreads) {
         const int row = e / SW, w = slab * SW + (e % SW);
         uint32_t v = 0;
-        if (row < a.zero_row && w < a.W32) {
+        if (w < a.W32) {
             int p = 0;
             while (p + 1 < a.nparts && row >= a.part_row0[p + 1]) ++p;
             const int sub = row - a.part_row0[p], len = a.part_len[p], first = a.part_first[p];
             v = p == 0 ? ~0u : 0u;
             const int wn = (w + 1 == a.W32) ? 0 : w + 1;
             for (int t = 0; t < len; ++t) {
-                const int digit = (sub >> (2 * (len - 1 - t))) & 3;
+                const int digit = ((sub >> (len + t)) & 1) << 1 | ((sub >> t) & 1);
                 const uint32_t* b = a.base32 + digit * a.W32;
                 v ^= __funnelshift_r(b[w], b[wn], first + t);  // rot_{first+t}
             }
@@ -286,12 +313,14 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const EncodeArgs a) {
     }
     __syncthreads();
 
-    // this lane's words of table row 0 (a row's W lane words are contiguous)
-    const uint32_t tbase = (uint32_t)__cvta_generic_to_shared(table) + 4u * W * lane;
-    uint4* list = lists + warp * kChunk;
-    const uint4 zero_entry = pack_entry<0, W>(a, 0);
+    // this lane's words of each part's first row (a row's W lane words are contiguous)
+    uint32_t base[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        base[p] = (uint32_t)__cvta_generic_to_shared(table) + a.row_bytes * (uint32_t)a.part_row0[p] + 4u * W * lane;
+    uint32_t* list = lists + warp * kList;
     const int k = a.k;
-    const uint32_t mask2k = k == 16 ? 0xffffffffu : ((1u << (2 * k)) - 1u);
+    const uint32_t maskk = (1u << k) - 1u;
     const int64_t gw = (int64_t)blockIdx.x * kWarps + warp, nw = (int64_t)gridDim.x * kWarps;
     const int w0 = slab * SW + W * lane;  // this lane's first word
 
@@ -318,100 +347,123 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const EncodeArgs a) {
         }
         int nvalid = 0;
 
+        uint32_t pend[W];  // sixteens of a group, added together with the next one's
+        bool odd = false;
+        auto up = [&](int i, uint32_t x, uint32_t y) {  // two sixteens up the planes
+            uint32_t carry;
+            csa(carry, hi[i][0], hi[i][0], x, y);
+#pragma unroll
+            for (int h = 1; h < NH; ++h) {
+                if (h == 4 && npos <= 255) break;  // no higher plane is reached
+                const uint32_t t = hi[i][h] & carry;
+                hi[i][h] ^= carry;
+                carry = t;
+            }
+        };
+        // ---- bundle a group of 16 entries (the first n of them, in a tail): binder words through a carry-save adder tree ----
+        auto bundle = [&](const uint32_t* ent, auto tail, int n) {
+            uint32_t xw[W][16];
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+                const uint4 e4 = *reinterpret_cast<const uint4*>(ent + j);
+                const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    uint32_t v[W];
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        uint32_t u[W];
+                        // a multiply-add by a number the compiler does not know: on the FMA pipe
+                        lds_words<W>(__byte_perm(e[h], 0, 0x4440 | p) * a.row_bytes + base[p], u);
+#pragma unroll
+                        for (int i = 0; i < W; ++i) v[i] = p ? v[i] ^ u[i] : u[i];
+                    }
+#pragma unroll
+                    for (int i = 0; i < W; ++i) xw[i][j + h] = decltype(tail)::value && j + h >= n ? 0u : v[i];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                uint32_t twosA, twosB, foursA, foursB, eightsA, eightsB, sixteens;
+                csa(twosA, ones[i], ones[i], xw[i][0], xw[i][1]);
+                csa(twosB, ones[i], ones[i], xw[i][2], xw[i][3]);
+                csa(foursA, twos[i], twos[i], twosA, twosB);
+                csa(twosA, ones[i], ones[i], xw[i][4], xw[i][5]);
+                csa(twosB, ones[i], ones[i], xw[i][6], xw[i][7]);
+                csa(foursB, twos[i], twos[i], twosA, twosB);
+                csa(eightsA, fours[i], fours[i], foursA, foursB);
+                csa(twosA, ones[i], ones[i], xw[i][8], xw[i][9]);
+                csa(twosB, ones[i], ones[i], xw[i][10], xw[i][11]);
+                csa(foursA, twos[i], twos[i], twosA, twosB);
+                csa(twosA, ones[i], ones[i], xw[i][12], xw[i][13]);
+                csa(twosB, ones[i], ones[i], xw[i][14], xw[i][15]);
+                csa(foursB, twos[i], twos[i], twosA, twosB);
+                csa(eightsB, fours[i], fours[i], foursA, foursB);
+                csa(sixteens, eights[i], eights[i], eightsA, eightsB);
+                if (odd)
+                    up(i, pend[i], sixteens);
+                else
+                    pend[i] = sixteens;
+            }
+            odd = !odd;
+        };
+
+        int n_list = 0;  // entries at hand: the valid k-mers not bundled yet
         for (int c0 = 0; c0 < npos; c0 += kChunk) {
-            // ---- stage kPerLane canonical k-mers per lane ----
-            const int p0 = c0 + lane * kPerLane;
-            uint32_t x = 0, m = 0;
-            auto push = [&](int pos) {
-                uint32_t code, inv;
+            // ---- stage a chunk's canonical k-mers: lane l those at c0 + l, c0 + 32 + l, ... ----
+            // bit planes of 32 bases a ballot; past the segment every base is bad
+            auto planes = [&](int pos, uint32_t& lo, uint32_t& hp, uint32_t& bad) {
+                uint32_t code = 0;
+                bool ok = pos < len;
                 if (a.words) {  // packed: every position of the segment is a base
                     const int64_t i = start + pos;
-                    code = pos < len ? (__ldg(a.words + (i >> 4)) >> (2 * (int)(i & 15))) & 3u : 0u;
-                    inv = pos < len ? 0u : 1u;
-                } else {
-                    const uint32_t c = pos < len ? (uint32_t)__ldg(s + pos) : 0u;
+                    if (ok) code = (__ldg(a.words + (i >> 4)) >> (2 * (int)(i & 15))) & 3u;
+                } else if (ok) {
+                    const uint32_t c = (uint32_t)__ldg(s + pos);
                     code = base_code(c);
-                    inv = pos < len ? (is_base(c) ^ 1u) : 1u;
+                    ok = c == __byte_perm(0x54474341u, 0, code | 0x4440u);  // "ACGT"[code]
                 }
-                x = (x >> 2) | (code << (2 * (k - 1)));
-                m = (m >> 1) | (inv << (k - 1));
+                lo = __ballot_sync(0xffffffffu, code & 1u);
+                hp = __ballot_sync(0xffffffffu, code & 2u);
+                bad = __ballot_sync(0xffffffffu, !ok);
             };
-            for (int j = 0; j < k - 1; ++j) push(p0 + j);
-#pragma unroll
-            for (int r = 0; r < kPerLane; ++r) {
-                push(p0 + r + k - 1);
-                uint4 e = zero_entry;
-                if (p0 + r < npos && m == 0) {
-                    uint32_t rc = ~x & mask2k;
-                    uint32_t y = __brev(x) >> (32 - 2 * k);
-                    uint32_t fw = ((y & 0x55555555u) << 1) | ((y >> 1) & 0x55555555u);
-                    e = pack_entry<NP, W>(a, fw < rc ? fw : rc);
-                    ++nvalid;
-                }
-                list[lane * kPerLane + r] = e;
+            uint32_t lo0, hp0, bad0;
+            planes(c0 + lane, lo0, hp0, bad0);
+#pragma unroll 2
+            for (int r = 0; r < kPerLane && c0 + 32 * r < npos; ++r) {
+                uint32_t lo1, hp1, bad1;
+                planes(c0 + 32 * (r + 1) + lane, lo1, hp1, bad1);
+                // k bases from this lane's position
+                const bool valid = (__funnelshift_r(bad0, bad1, lane) & maskk) == 0;
+                const Planes f{__funnelshift_r(lo0, lo1, lane) & maskk, __funnelshift_r(hp0, hp1, lane) & maskk};
+                const uint32_t e = pack_entry<NP>(a, canonical(f, k, maskk));
+                const uint32_t on = __ballot_sync(0xffffffffu, valid);
+                if (valid) list[n_list + __popc(on & ((1u << lane) - 1u))] = e;
+                n_list += __popc(on);
+                lo0 = lo1;
+                hp0 = hp1;
+                bad0 = bad1;
             }
             __syncwarp();
-
-            // ---- bundle: binder words through a carry-save adder tree ----
-            const int groups = (min(kChunk, npos - c0) + 15) >> 4;
-            for (int g = 0; g < groups; ++g) {
-                uint32_t xw[W][16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const uint4 e = list[g * 16 + j];
-                    uint32_t v[W];
-                    lds_words<W>(tbase + e.x, v);
-                    if (NP > 1) {
-                        uint32_t u[W];
-                        lds_words<W>(tbase + e.y, u);
-#pragma unroll
-                        for (int i = 0; i < W; ++i) v[i] ^= u[i];
-                    }
-                    if (NP > 2) {
-                        uint32_t u[W];
-                        lds_words<W>(tbase + e.z, u);
-#pragma unroll
-                        for (int i = 0; i < W; ++i) v[i] ^= u[i];
-                    }
-                    if (NP > 3) {
-                        uint32_t u[W];
-                        lds_words<W>(tbase + e.w, u);
-#pragma unroll
-                        for (int i = 0; i < W; ++i) v[i] ^= u[i];
-                    }
-#pragma unroll
-                    for (int i = 0; i < W; ++i) xw[i][j] = v[i];
-                }
-#pragma unroll
-                for (int i = 0; i < W; ++i) {
-                    uint32_t twosA, twosB, foursA, foursB, eightsA, eightsB, sixteens;
-                    csa(twosA, ones[i], ones[i], xw[i][0], xw[i][1]);
-                    csa(twosB, ones[i], ones[i], xw[i][2], xw[i][3]);
-                    csa(foursA, twos[i], twos[i], twosA, twosB);
-                    csa(twosA, ones[i], ones[i], xw[i][4], xw[i][5]);
-                    csa(twosB, ones[i], ones[i], xw[i][6], xw[i][7]);
-                    csa(foursB, twos[i], twos[i], twosA, twosB);
-                    csa(eightsA, fours[i], fours[i], foursA, foursB);
-                    csa(twosA, ones[i], ones[i], xw[i][8], xw[i][9]);
-                    csa(twosB, ones[i], ones[i], xw[i][10], xw[i][11]);
-                    csa(foursA, twos[i], twos[i], twosA, twosB);
-                    csa(twosA, ones[i], ones[i], xw[i][12], xw[i][13]);
-                    csa(twosB, ones[i], ones[i], xw[i][14], xw[i][15]);
-                    csa(foursB, twos[i], twos[i], twosA, twosB);
-                    csa(eightsB, fours[i], fours[i], foursA, foursB);
-                    csa(sixteens, eights[i], eights[i], eightsA, eightsB);
-                    uint32_t carry = sixteens;
-#pragma unroll
-                    for (int h = 0; h < NH; ++h) {
-                        const uint32_t t = hi[i][h] & carry;
-                        hi[i][h] ^= carry;
-                        carry = t;
-                    }
-                }
-            }
+            int g = 0;
+            for (; g + 16 <= n_list; g += 16) bundle(list + g, std::false_type{}, 16);
+            nvalid += g;
+            n_list -= g;
+            __syncwarp();
+            if (g && lane < n_list) list[lane] = list[g + lane];  // fewer than 16, read before any is written over
             __syncwarp();
         }
-        nvalid = __reduce_add_sync(0xffffffffu, nvalid);
+        if (n_list) {
+            if (lane >= n_list && lane < 16) list[lane] = 0;  // any row: masked
+            __syncwarp();
+            bundle(list, std::true_type{}, n_list);
+            nvalid += n_list;
+            __syncwarp();
+        }
+        if (odd) {
+#pragma unroll
+            for (int i = 0; i < W; ++i) up(i, pend[i], 0u);
+        }
         if (a.nkmers && lane == 0 && slab == 0) a.nkmers[seg] = nvalid;
         // next segment: from the queue, or a fixed stride over the grid
         if (a.queue) {
@@ -449,15 +501,16 @@ int launch_np_nh(const hdc_context* ctx, const EncodeArgs& a, int n_slabs, size_
 
 // Shared memory of a CTA whose lanes own W words: the slab's table rows and the warps' lists
 size_t encode_smem(const EncodeArgs& a, int w) {
-    return (size_t)a.table_rows * 32 * w * 4 + (size_t)kWarps * kChunk * sizeof(uint4);
+    return (size_t)a.table_rows * 32 * w * 4 + (size_t)kWarps * kList * sizeof(uint32_t);
 }
 
 // Two words a lane where that table fits a CTA's shared memory, else one
 template <int NP>
-int launch_np(const hdc_context* ctx, const EncodeArgs& a, int nh, cudaStream_t stream) {
+int launch_np(const hdc_context* ctx, EncodeArgs a, int nh, cudaStream_t stream) {
     const bool w2 = encode_smem(a, 2) <= kMaxEncodeSmem;
     const int n_slabs = (a.W32 + 32 * (w2 ? 2 : 1) - 1) / (32 * (w2 ? 2 : 1));
     const size_t smem = encode_smem(a, w2 ? 2 : 1);
+    a.row_bytes = w2 ? 256 : 128;
     if (w2) {
         if (nh <= 4) return launch_np_nh<NP, 4, 2>(ctx, a, n_slabs, smem, stream);
         if (nh <= 8) return launch_np_nh<NP, 8, 2>(ctx, a, n_slabs, smem, stream);
@@ -537,8 +590,7 @@ int launch_encode(hdc_context* ctx, const char* d_bytes, const int64_t* d_seg_of
         first += len;
         row0 += 1 << (2 * len);
     }
-    a.zero_row = row0;
-    a.table_rows = row0 + 1;
+    a.table_rows = row0;
     a.bytes = reinterpret_cast<const unsigned char*>(d_bytes);
     a.words = d_words;
     a.seg_off = d_seg_off;
