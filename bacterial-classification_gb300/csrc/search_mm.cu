@@ -606,16 +606,16 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
                 }
                 kth = skeys[(k - 1) * kMmQueryTile];
             }
-            int ended = 0;  // halves that have flushed
+            int ended = 0;  // bit h: half h has flushed; what follows in its ring belongs to the next group
             long long c0 = clock64();
             uint32_t seen = sh.beat;
             while (true) {
                 int h = -1;
-                if (ended < 2)
-                    h = ld_acquire_shared(&sh.head[0][row]) != tail[0]   ? 0
-                        : ld_acquire_shared(&sh.head[1][row]) != tail[1] ? 1
-                                                                         : -1;
-                if (__all_sync(0xffffffffu, ended == 2)) break;
+                if (!(ended & 1) && ld_acquire_shared(&sh.head[0][row]) != tail[0])
+                    h = 0;
+                else if (!(ended & 2) && ld_acquire_shared(&sh.head[1][row]) != tail[1])
+                    h = 1;
+                if (__all_sync(0xffffffffu, ended == 3)) break;
                 if (!__any_sync(0xffffffffu, h >= 0)) {
                     bool stop = err_s != 0;
                     if (sh.beat != seen) {
@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
                         ++tail[0];
                     st_release_shared(&sh.tail[h][row], at + 1);
                     if ((uint32_t)cand.y == kFlush) {
-                        ++ended;
+                        ended |= 1 << h;
                     } else {
                         const double rsc = __ldg(a.rs + (uint32_t)cand.y), ric = __ldg(a.ri + (uint32_t)cand.y);
                         const float s = exact_score_recip(cand.x, my_sq, rsc, my_iq, ric, a.mode);

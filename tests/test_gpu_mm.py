@@ -140,3 +140,26 @@ def test_saved_database_searches_the_same(hdc, cuda, tmp_path):
         assert ctx.tc_last_shape()[4] == 3
         for x, y in zip(a, b):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("nr,k", [(300, 10), (100, 5)])
+def test_tc_many_groups_of_few_tiles(hdc, cuda, nr, k):
+    """Far more query tiles than SMs against one or two reference tiles: a drain warp may be a whole group of query tiles
+    ahead of the other half's, and its candidates wait for their own group.  Equal to the limb search bit for bit."""
+    import torch
+    g = torch.Generator(device=cuda).manual_seed(nr)
+    dim, nq = 256, 60001
+    r = torch.randint(-200, 201, (nr, dim), dtype=torch.int16, device=cuda, generator=g)
+    q = (torch.randint(0, 2, (nq, dim), device=cuda, generator=g) * 2 - 1).to(torch.float16)
+    ctx = hdc.Context(dim, 10, 250, 10)
+    db = ctx.refdb(r, 200)
+    qn = torch.full((nq,), dim, dtype=torch.int64, device=cuda)
+    a = ctx.search_tc(db, q, qn, 1, k)
+    torch.cuda.synchronize()
+    assert ctx.tc_last_shape()[4] == 3
+    ctx.tc_option(hdc.TC_CLUSTER, 1)
+    b = ctx.search_tc(db, q, qn, 1, k)
+    torch.cuda.synchronize()
+    assert ctx.status() == 0 and ctx.tc_last_shape()[0] == 1
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
