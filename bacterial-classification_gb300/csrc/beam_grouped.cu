@@ -1162,7 +1162,7 @@ __device__ void tc_phase(const GArgs& a, const TcItems& t, TcShared& sm, TcRun& 
                 acc_phase ^= 1;
             }
         }
-    } else if (lane == 0) {
+    } else if (tc::elect_one()) {
         // ------------------------------------------------ MMA issuer
         // the limb tiles of B are 64 or 96 consecutive rows of shared memory and their
         // accumulators as many consecutive columns: one N = 64 or 96 MMA covers them all
@@ -1211,7 +1211,7 @@ __device__ void tc_phase(const GArgs& a, const TcItems& t, TcShared& sm, TcRun& 
 template <class Lay>
 __device__ void tc_teardown(TcShared& sm, int* status) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp == Lay::kMmaWarp && lane == 0) {
+    if (warp == Lay::kMmaWarp && tc::elect_one()) {
         tc::mma_commit(&sm.drain_bar);
         const long long c0 = clock64();
         while (!tc::mbar_try_wait(tc::smem_u32(&sm.drain_bar), 0) && clock64() - c0 < tc::kWaitCycles) {

@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
             use += (uint32_t)n_kb;
         }
     } else if (warp == kMmaWarp) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
 
     if (warp < 4) {
         regs_down<kRegsLoad>();
-        if (warp == 0 && lane == 0) {
+        if (warp == 0 && tc::elect_one()) {
             // -------------------------------------------- TMA producer
             int stage = 0;
             uint32_t phase = 0;
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
                 while (!tc::mbar_try_wait(tc::smem_u32(bar), ph) && clock64() - c0 < tc::kWaitCycles) {
                 }
             }
-        } else if (warp == 1 && lane == 0 && crank == 0) {
+        } else if (warp == 1 && crank == 0 && tc::elect_one()) {
             // -------------------------------------------- MMA issuer (the even CTA's, in a pair)
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
@@ -973,9 +973,10 @@ struct MmPlan {
 // G query tiles at a time on S = SMs / G reference lanes each.  All G x S CTAs step through the same reference tiles
 // together, so DRAM sees the references once a group.  The choice minimises
 //     groups x (tiles of a lane x cycles of a tile + the start of the lists)
-// with cycles a column and K step as measured.  Pairs: 0.57 for digits (D = 10,240, 4 digits: 79.6K to 81K cycles a
-// tile of 224, of which the MMAs take 71.7K), 0.6 for fp16.  Single CTAs load as many operand bytes for half the MMA
-// work or less and are bound by L2: 1.1 (112 columns) and 1.7 (64 columns: 515 TFLOP/s where pairs run 1,750).  More
+// with cycles a column and K step as measured.  Pairs run at the tensor pipe's rate: 0.53 (digits) and 0.5 (fp16: 514
+// cycles a K block of 4 steps and 256 columns).  Single CTAs load as many operand bytes for half the MMA work or less:
+// 0.9 (112 columns, 95 cycles a step) and 1.4 (64 columns: 328 cycles a K block where 32 CTAs run, bound by the MMA
+// issuer's waits and commits; 400 on all SMs, bound by L2).  More
 // lanes cost a little each (their lists start empty; 38 lanes none to speak of, 76 lanes 13 %), and a group whose
 // query tiles fill L2 about 5 % (60,000 references, 38,912 queries: 22.4 ms with 38 tiles a group, 23.6 with 152).
 MmPlan mm_plan(int sms, int64_t nq, int64_t nr, int dim, bool f4, int limbs) {
@@ -1004,8 +1005,8 @@ MmPlan mm_plan(int sms, int64_t nq, int64_t nr, int dim, bool f4, int limbs) {
             }
         }
     };
-    if (qt >= 2) consider(2, f4 ? MmTile<true, 2>::N : MmTile<false, 2>::N, f4 ? 0.57 : 0.6);
-    consider(1, f4 ? MmTile<true, 1>::N : MmTile<false, 1>::N, f4 ? 1.1 : 1.7);
+    if (qt >= 2) consider(2, f4 ? MmTile<true, 2>::N : MmTile<false, 2>::N, f4 ? 0.53 : 0.5);
+    consider(1, f4 ? MmTile<true, 1>::N : MmTile<false, 1>::N, f4 ? 0.9 : 1.4);
     return best;
 }
 

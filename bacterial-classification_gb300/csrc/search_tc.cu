@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (tc::elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             int64_t issued = 0;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer (the even CTA's, with pair MMAs)
-        if (lane == 0 && (!PAIR_MMA || (crank & 1) == 0)) {
+        if ((!PAIR_MMA || (crank & 1) == 0) && tc::elect_one()) {
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
