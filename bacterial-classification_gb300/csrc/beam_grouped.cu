@@ -619,7 +619,7 @@ __global__ void output_kernel(const GArgs a, int32_t* __restrict__ path, float* 
 // beam slot) whose beam row is node P are scored against P's children (a childless P
 // against itself) as one dense [entries] x [children] product.  A work item is up to 128
 // entries x 32 children of one parent.  Producer warps, in groups of four taking every G-th K
-// block (TcLayout: three groups in the level kernel, two in the one-launch kernel), write the
+// block (TcLayout: three groups, two in the one-launch kernel that streams its leaf level too), write the
 // entries' +1/-1 signs (from the packed bits) as fp16 straight into TMEM with tcgen05.st (the
 // A operand: lane = entry, two signs a column), and the children's int32
 // prototype rows, split into three balanced base-2048 fp16 limbs, into 128-byte-swizzled
@@ -652,12 +652,19 @@ constexpr int kTcMaxStages = 6;
 // g, g + G, ...): warps 0 .. 4G-1 produce, 4G .. 4G+3 run the epilogue, lane 0 of warp 4G+4
 // issues the MMAs.  A warp's registers come from its SM sub-partition's quarter of the file,
 // so 17 warps (G = 3: five on one sub-partition) get 96 registers a thread, 13 warps (G = 2)
-// 128: the level kernel takes three groups, the one-launch kernel, whose other phases need the
-// registers, two.
+// 128: only the one-launch kernel with the streamed leaf level in it, whose scoring needs the
+// registers, takes two.
+//
+// What bounds a level is the producers' sequence per K block, mostly half-rate integer
+// instructions (64 dims: two a sign column, three a value and limb pair).  The K order within 32
+// dims is theirs to choose: a column holds dims j and j + 16, so one shift and one and-xor of a
+// word of signs make it, and a thread's 8 values of a row are one 16-byte store a limb.  100,000
+// leaves, 20,000 reads, D = 16,384: levels 0-4 2.85 ms with columns of neighbouring dims and two
+// groups, 2.06 so, 1.79 with three groups.
 template <int G>
 struct TcLayout {
     static constexpr int kGroups = G;
-    static constexpr int kStages = 2 * G;  // two stages in flight per group
+    static constexpr int kStages = 6;  // two or three in flight per group
     static constexpr int kProducers = 128 * G;
     static constexpr size_t kStageArea = (size_t)kTcDepth * 5 * kProducers * 16;  // 4 x 16 B values + 16 B bits
     static constexpr int kEpiWarp = 4 * G;
@@ -668,7 +675,8 @@ struct TcLayout {
     static_assert(kTcACol + 32 * kStages <= kTcTmemCols, "the A stages fit the TMEM allocation");
 };
 using TcLevel = TcLayout<3>;  // descent_tc_kernel: 544 threads
-using TcOne = TcLayout<2>;    // descent_one_kernel: 416 threads
+template <bool LEAF>
+using TcOne = TcLayout<LEAF ? 2 : 3>;  // descent_one_kernel: 416 threads with the streamed leaf level in it
 
 struct TcItems {
     int32_t* ent_read;    // [entries] grouped by parent
@@ -865,29 +873,48 @@ __global__ void items_level0_kernel(const GArgs a, TcItems t) {
     items_level0_range(a, t, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
-// v = l0 + 2048 l1 with l0 in [-1024, 1023] and |l1| <= 1024, for |v| <= 2^21
-__device__ __forceinline__ void limbs2(int32_t v, int32_t& l0, int32_t& l1) {
-    l1 = (v >> 11) + (((v & 2047) + 1024) >> 11);  // floor((v + 1024) / 2048)
-    l0 = (int32_t)((uint32_t)v - ((uint32_t)l1 << 11));
+// Two small floats as an fp16 pair (one cvt.rn.f16x2.f32; exact for integers of magnitude <= 2048).
+__device__ __forceinline__ uint32_t half2_of(float x, float y) {
+    const __half2 h = __floats2half2_rn(x, y);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// x and y as fp16 pairs of limbs v = l0 + 2048 l1 with l0 in [-1024, 1023] and |l1| <= 1024, for |v| <= 2^21.  A limb
+// becomes an fp32 by a magic number, its bits below 2^23's exponent: three integer instructions a value, the half-rate
+// ones that bound the producers.
+__device__ __forceinline__ void limbs2(int32_t x, int32_t y, uint32_t& h0, uint32_t& h1) {
+    const uint32_t t = (uint32_t)(x + (1 << 22) + 1024), s = (uint32_t)(y + (1 << 22) + 1024);  // 0 < t < 2^23
+    auto low = [](uint32_t v) { return __uint_as_float((v & 2047u) | 0x4B000000u) - (8388608.0f + 1024.0f); };
+    // v >> 11 below the exponent (0x4B000000 = 600 * 2^21)
+    auto high = [](uint32_t v) { return __uint_as_float(__funnelshift_r(v, 600u, 11)) - (8388608.0f + 2048.0f); };
+    h0 = half2_of(low(t), low(s));
+    h1 = half2_of(high(t), high(s));
 }
 
 // v = l0 + 2048 l1 + 2048^2 l2 with l0, l1 in [-1024, 1023] and |l2| <= 512, for every int32 v
-__device__ __forceinline__ void limbs3(int32_t v, int32_t& l0, int32_t& l1, int32_t& l2) {
+__device__ __forceinline__ void limbs3(int32_t v, float& l0, float& l1, float& l2) {
+    // |x| < 2^22: exact, one integer and one float add
+    auto small = [](int32_t x) { return __int_as_float(0x4B400000 + x) - 12582912.0f; };
     const int32_t q1 = (v >> 11) + (((v & 2047) + 1024) >> 11);  // floor((v + 1024) / 2048)
-    l0 = (int32_t)((uint32_t)v - ((uint32_t)q1 << 11));
     const int32_t q2 = (q1 >> 11) + (((q1 & 2047) + 1024) >> 11);
-    l1 = q1 - q2 * 2048;
-    l2 = q2;
+    l0 = small((int32_t)((uint32_t)v - ((uint32_t)q1 << 11)));
+    l1 = small(q1 - q2 * 2048);
+    l2 = small(q2);
+}
+__device__ __forceinline__ void limbs3(int32_t x, int32_t y, uint32_t& h0, uint32_t& h1, uint32_t& h2) {
+    float a0, a1, a2, b0, b1, b2;
+    limbs3(x, a0, a1, a2);
+    limbs3(y, b0, b1, b2);
+    h0 = half2_of(a0, b0);
+    h1 = half2_of(a1, b1);
+    h2 = half2_of(a2, b2);
 }
 
-// Two small integers (|x| <= 2048) as an fp16 pair: each becomes an fp32 by the magic
-// number 1.5 * 2^23 (exact for |x| < 2^22: one integer and one float add, no conversion
-// unit), and the pair is packed with one cvt.rn.f16x2.f32 (exact: both fit 11 bits).
-__device__ __forceinline__ uint32_t half2_bits(int32_t x, int32_t y) {
-    const float fx = __int_as_float(0x4B400000 + x) - 12582912.0f;
-    const float fy = __int_as_float(0x4B400000 + y) - 12582912.0f;
-    const __half2 h = __floats2half2_rn(fx, fy);
-    return *reinterpret_cast<const uint32_t*>(&h);
+__device__ __forceinline__ void four_int16(const uint4& p, int32_t (&x)[4]) {
+    x[0] = (int32_t)(p.x << 16) >> 16;
+    x[1] = (int32_t)p.x >> 16;
+    x[2] = (int32_t)(p.y << 16) >> 16;
+    x[3] = (int32_t)p.y >> 16;
 }
 
 // cp.async of 16 / 8 bytes global -> shared; with src_bytes 0 nothing is read and zeros land
@@ -976,9 +1003,10 @@ __device__ void tc_phase(const GArgs& a, const TcItems& t, TcShared& sm, TcRun& 
     if (warp < Lay::kEpiWarp) {
         // ------------------------------------------------ producers: group g takes K blocks g, g + 3, ...
         // Row tid of A is this thread's entry.  The valid children's values of a K block are
-        // groups of 4 (group 16 v + u: the item's v-th valid child, dims 4u..4u+3); group x
-        // goes to the thread with tb = x mod 128, so the limb split is spread over the whole
-        // group.  tb is tid rotated so that the groups past the first 128 (a warp that has any
+        // groups of 8 (group 8 v + u: the item's v-th valid child, dims d..d+3 and d+16..d+19
+        // with d = 32 (u / 4) + 4 (u % 4), interleaved in the row's 16-byte chunk u as A's
+        // columns have them); group x goes to the thread with tb = x mod 128, so the limb split
+        // is spread over the whole group.  tb is tid rotated so that the groups past the first 128 (a warp that has any
         // takes a second pass) fall to warp 1, 6 or 11, not to the warps that share their SM
         // sub-partition with the MMA issuer.  Nothing
         // is written for an unused row or child slot: an accumulator row or column depends only
@@ -1002,42 +1030,45 @@ __device__ void tc_phase(const GArgs& a, const TcItems& t, TcShared& sm, TcRun& 
             } else {
                 n0 = min(kTcC, n_children(a, ip) - ij0);
             }
-            const int ngroups = (n0 + n1) * 16;
-            const char* gsrc[4];  // this group's 4 values in K block 0: 16 bytes of an int32 row or 8 of an int16 row
-            int gdst[4];          // child slot * 16 + u
-            bool g16[4];
+            const int ngroups = (n0 + n1) * 8;
+            const char* gsrc[2];  // this group's first 4 values in K block 0: 16 bytes of an int32 row or 8 of an int16 row
+            int gdst[2];          // child slot * 8 + u
+            bool g16[2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 2; ++i) {
                 const int x = tb + kTcE * i;
                 gsrc[i] = reinterpret_cast<const char*>(a.proto);
                 gdst[i] = 0;
                 g16[i] = false;
                 if (x < ngroups) {
-                    const int v = x >> 4, u = x & 15;
+                    const int v = x >> 3, u = x & 7;
                     const int js = v < n0 ? v : kTcHalfC + (v - n0);
                     const int64_t c = item_child(a, t, it, js);
+                    const int d = 32 * (u >> 2) + 4 * (u & 3);
                     g16[i] = c >= a.n32;
-                    gsrc[i] = g16[i] ? reinterpret_cast<const char*>(a.proto16 + (c - a.n32) * a.dim + 4 * u)
-                                     : reinterpret_cast<const char*>(a.proto + c * a.dim + 4 * u);
-                    gdst[i] = js * 16 + u;
+                    gsrc[i] = g16[i] ? reinterpret_cast<const char*>(a.proto16 + (c - a.n32) * a.dim + d)
+                                     : reinterpret_cast<const char*>(a.proto + c * a.dim + d);
+                    gdst[i] = js * 8 + u;
                 }
             }
             // a warp whose groups are all int32 rows runs the int32-only body
-            bool my16 = false;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) my16 |= g16[i];
+            const bool my16 = g16[0] || g16[1];
             auto body = [&](auto rows16) {
                 constexpr bool R16 = decltype(rows16)::value;
                 auto issue = [&](int kb, int slot) {  // this thread's slices of K block kb, into staging slot `slot`
                     if (kb < kblocks) {
                         uint4* sb = staging + (size_t)slot * 5 * Lay::kProducers;
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
+                        for (int i = 0; i < 2; ++i)
                             if (tb + kTcE * i < ngroups) {
-                                if (R16 && g16[i])
-                                    cp_async8(sb + i * Lay::kProducers + ptid, gsrc[i] + kb * 128, 8);
-                                else
-                                    cp_async16(sb + i * Lay::kProducers + ptid, gsrc[i] + kb * 256, 16);
+                                uint4* to = sb + 2 * i * Lay::kProducers + ptid;
+                                if (R16 && g16[i]) {
+                                    cp_async8(to, gsrc[i] + kb * 128, 8);
+                                    cp_async8(to + Lay::kProducers, gsrc[i] + kb * 128 + 32, 8);
+                                } else {
+                                    cp_async16(to, gsrc[i] + kb * 256, 16);
+                                    cp_async16(to + Lay::kProducers, gsrc[i] + kb * 256 + 64, 16);
+                                }
                             }
                         if (rrow >= 0) cp_async8(sb + 4 * Lay::kProducers + ptid, bits_row + kb, 8);
                     }
@@ -1045,69 +1076,68 @@ __device__ void tc_phase(const GArgs& a, const TcItems& t, TcShared& sm, TcRun& 
                 };
 #pragma unroll
                 for (int i = 0; i < kTcDepth; ++i) issue(g + Lay::kGroups * i, i);
+                int stage = (int)((nbase + g) % Lay::kStages);
+                uint32_t phase = (uint32_t)((nbase + g) / Lay::kStages & 1);
                 for (int kb = g, i = 0; kb < kblocks; kb += Lay::kGroups, ++i) {
                     cp_async_wait<kTcDepth - 1>();  // this thread's copies of block kb have landed
                     const int slot = i % kTcDepth;
                     const uint4* sb = staging + (size_t)slot * 5 * Lay::kProducers;
                     uint4 pv[4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) pv[j] = tb + kTcE * j < ngroups ? sb[j * Lay::kProducers + ptid] : make_uint4(0, 0, 0, 0);
+                    for (int j = 0; j < 4; ++j)
+                        pv[j] = tb + kTcE * (j >> 1) < ngroups ? sb[j * Lay::kProducers + ptid] : make_uint4(0, 0, 0, 0);
                     const uint2 w = rrow >= 0 ? *reinterpret_cast<const uint2*>(sb + 4 * Lay::kProducers + ptid) : make_uint2(0, 0);
                     issue(kb + Lay::kGroups * kTcDepth, slot);  // the slot is free again: refill it kTcDepth blocks ahead
-                    const int64_t n = nbase + kb;
-                    const int stage = (int)(n % Lay::kStages);
-                    const uint32_t phase = (uint32_t)((n / Lay::kStages) & 1);
                     const bool got = tc::mbar_wait(&sm.empty_bar[stage], phase ^ 1, &sm.err, 11, a.wait_cycles);
                     if (__any_sync(0xffffffffu, !got)) {
                         ok = false;
                         break;
                     }
                     uint8_t* st = ring + (size_t)stage * kTcStageBytes;
-                    // A: this entry's 64 signs, two fp16 to a column, into TMEM lane tid (an unused
-                    // row's garbage only reaches its own accumulator row, which is never read)
+                    // A: this entry's 64 signs, dims j and j + 16 of a word to a column, into TMEM lane tid (an
+                    // unused row's garbage only reaches its own accumulator row, which is never read)
                     {
                         uint32_t col[32];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const uint32_t t = (j < 16 ? w.x : w.y) >> (2 * (j & 15));
-                            col[j] = 0xBC00BC00u ^ ((t & 1u) << 15) ^ ((t & 2u) << 30);
-                        }
+                        for (int j = 0; j < 32; ++j)
+                            col[j] = (((j < 16 ? w.x : w.y) << (15 - (j & 15))) & 0x80008000u) ^ 0xBC00BC00u;
                         tc::tmem_st32(tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(kTcACol + 32 * stage), col);
                     }
-                    // B: this thread's groups of 4 prototype values, each in two or three limbs (8
-                    // bytes per limb)
+                    // B: this thread's groups of 8 prototype values in the columns' order, each in two or three
+                    // limbs (16 bytes per limb)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < 2; ++j) {
                         if (tb + kTcE * j >= ngroups) break;
-                        int32_t l0[4], l1[4], l2[4];
-                        int32_t x[4] = {(int32_t)pv[j].x, (int32_t)pv[j].y, (int32_t)pv[j].z, (int32_t)pv[j].w};
+                        int32_t x[4] = {(int32_t)pv[2 * j].x, (int32_t)pv[2 * j].y, (int32_t)pv[2 * j].z, (int32_t)pv[2 * j].w};
+                        int32_t y[4] = {(int32_t)pv[2 * j + 1].x, (int32_t)pv[2 * j + 1].y, (int32_t)pv[2 * j + 1].z,
+                                        (int32_t)pv[2 * j + 1].w};
                         if (R16 && g16[j]) {  // four int16 values in the first 8 bytes
-                            x[0] = (int32_t)(pv[j].x << 16) >> 16;
-                            x[1] = (int32_t)pv[j].x >> 16;
-                            x[2] = (int32_t)(pv[j].y << 16) >> 16;
-                            x[3] = (int32_t)pv[j].y >> 16;
+                            four_int16(pv[2 * j], x);
+                            four_int16(pv[2 * j + 1], y);
                         }
-                        const int js = gdst[j] >> 4, u = gdst[j] & 15;
-                        const int off = (u & 1) * 8;
+                        const int js = gdst[j] >> 3, u = gdst[j] & 7;
+                        uint32_t h0[4], h1[4], h2[4];
                         if (two) {
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) limbs2(x[e], l0[e], l1[e]);
+                            for (int e = 0; e < 4; ++e) limbs2(x[e], y[e], h0[e], h1[e]);
                         } else {
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) limbs3(x[e], l0[e], l1[e], l2[e]);
-                            *reinterpret_cast<uint2*>(swz(st + 2 * kTcBBytes, js, u >> 1) + off) =
-                                make_uint2(half2_bits(l2[0], l2[1]), half2_bits(l2[2], l2[3]));
+                            for (int e = 0; e < 4; ++e) limbs3(x[e], y[e], h0[e], h1[e], h2[e]);
+                            *reinterpret_cast<uint4*>(swz(st + 2 * kTcBBytes, js, u)) = make_uint4(h2[0], h2[1], h2[2], h2[3]);
                         }
-                        *reinterpret_cast<uint2*>(swz(st, js, u >> 1) + off) =
-                            make_uint2(half2_bits(l0[0], l0[1]), half2_bits(l0[2], l0[3]));
-                        *reinterpret_cast<uint2*>(swz(st + kTcBBytes, js, u >> 1) + off) =
-                            make_uint2(half2_bits(l1[0], l1[1]), half2_bits(l1[2], l1[3]));
+                        *reinterpret_cast<uint4*>(swz(st, js, u)) = make_uint4(h0[0], h0[1], h0[2], h0[3]);
+                        *reinterpret_cast<uint4*>(swz(st + kTcBBytes, js, u)) = make_uint4(h1[0], h1[1], h1[2], h1[3]);
                     }
                     tc::tmem_st_wait();       // the A columns are written
                     tc::fence_before();       // ... before the arrive below (tcgen05 ordering)
                     tc::fence_proxy_async();  // the B writes above are read by the tensor cores
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&sm.full_bar[stage]);
+                    stage += Lay::kGroups;
+                    if (stage >= Lay::kStages) {
+                        stage -= Lay::kStages;
+                        phase ^= 1;
+                    }
                 }
             };
             if (__any_sync(0xffffffffu, my16))
@@ -1251,10 +1281,10 @@ __global__ void __launch_bounds__(TcLevel::kThreads, 1) descent_tc_kernel(const 
 // scoring keeps its TMEM columns and mbarrier ring positions from one level to the next.
 
 constexpr int kCodeGridBarrier = 20;  // status 100 + this: a grid barrier gave up
-// Dynamic shared memory of the one-launch kernel: the tensor-core levels use the first TcOne::kSmem
+// Dynamic shared memory of the one-launch kernel: the tensor-core levels use the first TcLayout::kSmem
 // bytes; the streamed leaf level uses all of it (row slots + the consumers' bit buffers).
 constexpr size_t kOneSmem = 225 * 1024;
-static_assert(kOneSmem >= TcOne::kSmem, "the one-launch kernel also runs the tensor-core levels");
+static_assert(kOneSmem >= TcOne<true>::kSmem && kOneSmem >= TcOne<false>::kSmem, "the one-launch kernel also runs the tensor-core levels");
 constexpr int kMaxPhaseTs = 64;       // phase timestamps kept of a launch (hdc_beam_phase_times)
 
 struct OneArgs {
@@ -1270,7 +1300,6 @@ struct OneArgs {
     float* out_score;
     int32_t* out_depth;
     unsigned long long* phase_ts;  // [kMaxPhaseTs] CTA 0's clock at the start and after every barrier
-    int leaf_apart;                // 1: stop at the last level's node-ordered pairs (scored by leaf_kernel)
     long long wait_cycles;         // limit of every bounded wait (SM cycles)
     int late_cta;                  // test hook: CTA 0 reaches its first grid barrier 4 limits late
 };
@@ -1741,7 +1770,11 @@ __global__ void __launch_bounds__(kScoreThreads, ROWS16 ? kScoreBlocks16 : kLeaf
     select_reads<16>(a, l.L, w, a.nq, nw, [&](int64_t r) { output_one(a, r, l.path, l.path_score, l.depth); });
 }
 
-__global__ void __launch_bounds__(TcOne::kThreads, 1) descent_one_kernel(const GArgs a, const TcItems t, const OneArgs o) {
+// LEAF: the last level too (streamed); without it, the registers of that phase free, three producer groups fit.
+template <bool LEAF>
+__global__ void __launch_bounds__(TcOne<LEAF>::kThreads, 1)
+    descent_one_kernel(const GArgs a, const TcItems t, const OneArgs o) {
+    using Lay = TcOne<LEAF>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ TcShared sm;
     __shared__ int32_t sh[32];
@@ -1752,9 +1785,9 @@ __global__ void __launch_bounds__(TcOne::kThreads, 1) descent_one_kernel(const G
         n_ts = 0;
         if (blockIdx.x == 0) o.phase_ts[n_ts++] = global_ns();
     }
-    uint4* staging = reinterpret_cast<uint4*>(ring + (size_t)TcOne::kStages * kTcStageBytes);
+    uint4* staging = reinterpret_cast<uint4*>(ring + (size_t)Lay::kStages * kTcStageBytes);
     if (o.use_tc) {
-        tc_setup<TcOne>(sm);
+        tc_setup<Lay>(sm);
     } else {
         if (threadIdx.x == 0) sm.err = 0;
         __syncthreads();
@@ -1847,7 +1880,7 @@ __global__ void __launch_bounds__(TcOne::kThreads, 1) descent_one_kernel(const G
                 if (!(ok = grid_barrier(o, sm, &ok_s, &n_ts))) break;
             }
             // G: the level's pairs scored on the tensor cores
-            tc_phase<TcOne>(a, t, sm, run, ring, staging);
+            tc_phase<Lay>(a, t, sm, run, ring, staging);
         } else {
             // C: pairs per node, summed per CTA
             sum = cta_sum(a.node_cnt, n0, n1, sh);
@@ -1861,14 +1894,14 @@ __global__ void __launch_bounds__(TcOne::kThreads, 1) descent_one_kernel(const G
             // E: the pairs in node order
             scatter_range(a, gtid, gstride);
             if (!(ok = grid_barrier(o, sm, &ok_s, &n_ts))) break;
-            if (o.leaf_apart && L == a.levels - 1) {
+            if (!LEAF && L == a.levels - 1) {
                 // the last level is scored and selected by leaf_kernel
                 apart_done = true;
                 break;
             }
             // F: the pairs scored on the CUDA cores: the leaf level's rows streamed through shared
             // memory, other levels (every level without the tensor cores) one warp per pair
-            if (o.use_tc)
+            if (LEAF && o.use_tc)
                 stream_phase(a, sm, run, ring, kOneSmem - 1024);
             else if (rows16)
                 score_pairs<true>(a, gtid >> 5, gstride >> 5);
@@ -1877,11 +1910,12 @@ __global__ void __launch_bounds__(TcOne::kThreads, 1) descent_one_kernel(const G
         }
         if (!(ok = grid_barrier(o, sm, &ok_s, &n_ts))) break;
         // H: the beams of this CTA's reads (after a streamed level, their pairs' keys first)
-        if (o.use_tc && !tcl && r0 < r1) {
+        if (LEAF && o.use_tc && !tcl && r0 < r1) {
             keys_from_parts(a, r0, r1);
             __syncthreads();
         }
-        select_reads(a, L, r0 + (tid >> 5), r1, nt >> 5, [](int64_t) {});
+        // (16 lanes a read where the producer groups leave no registers for 8 keys a lane)
+        select_reads<LEAF ? kSelLanes : 16>(a, L, r0 + (tid >> 5), r1, nt >> 5, [](int64_t) {});
         __syncthreads();
     }
     if (ok && !apart_done)
@@ -1891,10 +1925,19 @@ __global__ void __launch_bounds__(TcOne::kThreads, 1) descent_one_kernel(const G
         for (int i = n_ts; i < kMaxPhaseTs; ++i) o.phase_ts[i] = 0;
     }
     if (o.use_tc) {
-        tc_teardown<TcOne>(sm, o.status);
+        tc_teardown<Lay>(sm, o.status);
     } else if (tid == 0 && sm.err) {
         atomicCAS(o.status, 0, 100 + sm.err);
     }
+}
+
+struct OneLaunch {
+    const void* kernel;
+    int threads;
+};
+OneLaunch one_launch(bool leaf) {
+    if (leaf) return {(const void*)descent_one_kernel<true>, TcOne<true>::kThreads};
+    return {(const void*)descent_one_kernel<false>, TcOne<false>::kThreads};
 }
 
 // The one-launch descent needs every CTA (one per SM) resident at once; checked once per
@@ -1903,10 +1946,14 @@ bool one_launch_fits(hdc_context* ctx) {
     if (ctx->beam_one == 0) return false;
     if (ctx->beam_one_fit < 0) {
         int per_sm = 0;
-        cudaError_t e = cudaFuncSetAttribute(descent_one_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kOneSmem);
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, descent_one_kernel, TcOne::kThreads, kOneSmem);
+        cudaError_t e = cudaSuccess;
+        for (const bool leaf : {false, true}) {
+            const OneLaunch l = one_launch(leaf);
+            int n = 0;
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOneSmem);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, l.kernel, l.threads, kOneSmem);
+            per_sm = leaf ? std::min(per_sm, n) : n;
+        }
         int coop = 0;
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
         cudaGetLastError();
@@ -2062,13 +2109,14 @@ int launch_beam_grouped(hdc_context* ctx, const int8_t* d_q, const uint32_t* d_q
         o.phase_ts = ctx->d_phase_ts;
         o.wait_cycles = a.wait_cycles;
         o.late_cta = ctx->test_withhold_loads == 2 ? 1 : 0;
-        o.leaf_apart = ctx->beam_one != 1 ? 1 : 0;  // automatic: the last level in a launch of its own
+        const bool with_leaf = ctx->beam_one == 1;  // automatic: the last level in a launch of its own
+        const OneLaunch launch = one_launch(with_leaf);
         e = cudaMemsetAsync(one_state, 0, 4 * sizeof(uint32_t), stream);
         void* args[] = {(void*)&a, (void*)&t, (void*)&o};
         if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel((const void*)descent_one_kernel, dim3((unsigned)ctx->num_sms),
-                                            dim3(TcOne::kThreads), args, kOneSmem, stream);
-        if (e == cudaSuccess && o.leaf_apart) {
+            e = cudaLaunchCooperativeKernel(launch.kernel, dim3((unsigned)ctx->num_sms), dim3(launch.threads), args, kOneSmem,
+                                            stream);
+        if (e == cudaSuccess && !with_leaf) {
             LeafArgs l{levels - 1, d_path, d_path_score, d_depth, o.bar_count, o.bar_gen, o.abort, o.status};
             void* largs[] = {(void*)&a, (void*)&l};
             const bool r16 = n32 < n_nodes;
