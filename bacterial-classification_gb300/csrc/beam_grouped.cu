@@ -1986,7 +1986,7 @@ int launch_beam_grouped(hdc_context* ctx, const int8_t* d_q, const uint32_t* d_q
     int32_t maxc = max_children;
     if (maxc <= 0) {
         int32_t* d_maxc = nullptr;
-        if ((e = cudaMallocAsync(&d_maxc, sizeof(int32_t), stream)) != cudaSuccess)
+        if ((e = scratch_alloc(ctx, reinterpret_cast<void**>(&d_maxc), sizeof(int32_t), stream)) != cudaSuccess)
             return cuda_fail(e, "beam: workspace");
         cudaMemsetAsync(d_maxc, 0, sizeof(int32_t), stream);
         max_children_kernel<<<mc_grid, 256, 0, stream>>>(d_child_ptr, n_nodes, d_maxc);
@@ -2077,7 +2077,7 @@ int launch_beam_grouped(hdc_context* ctx, const int8_t* d_q, const uint32_t* d_q
     };
     const size_t bytes = carve_all(nullptr);
     uint8_t* ws = nullptr;
-    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&ws), bytes, stream)) != cudaSuccess)
+    if ((e = scratch_alloc(ctx, reinterpret_cast<void**>(&ws), bytes, stream)) != cudaSuccess)
         return cuda_fail(e, "beam: workspace");
     carve_all(ws);
     a.bits = d_qbits ? d_qbits : bits;

@@ -530,7 +530,7 @@ int launch_fasta_parse(hdc_context* ctx, const char* d_in, int64_t n, char* d_ou
     // tiles, then (after the scan) the records
     uint8_t* ws = nullptr;
     const size_t b_tiles = ((size_t)a.n_tiles * sizeof(TileSum) + 255) & ~(size_t)255;
-    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&ws), b_tiles + 256, stream)) != cudaSuccess)
+    if ((e = scratch_alloc(ctx, reinterpret_cast<void**>(&ws), b_tiles + 256, stream)) != cudaSuccess)
         return cuda_fail(e, "fasta: workspace");
     a.tiles = reinterpret_cast<TileSum*>(ws);
     a.totals = reinterpret_cast<int64_t*>(ws + b_tiles);
@@ -560,7 +560,7 @@ int launch_fasta_parse(hdc_context* ctx, const char* d_in, int64_t n, char* d_ou
         return (size_t)(cur - base);
     };
     const size_t bytes = carve_all(nullptr);
-    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&rs), bytes, stream)) != cudaSuccess) {
+    if ((e = scratch_alloc(ctx, reinterpret_cast<void**>(&rs), bytes, stream)) != cudaSuccess) {
         cudaFreeAsync(ws, stream);
         return cuda_fail(e, "fasta: record workspace");
     }

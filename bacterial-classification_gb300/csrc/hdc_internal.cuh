@@ -19,6 +19,7 @@ struct hdc_context {
     int words32 = 0;  // 2 * words64: the 64*HV_WORDS-bit ring in 32-bit words
     int device = 0;
     int num_sms = 0;
+    cudaMemPool_t scratch = nullptr;  // workspaces of the calls (null: the device's default pool)
     uint64_t* host_base = nullptr;  // [4][words64], A,C,G,T
     uint32_t* d_base32 = nullptr;   // [4][words32] on the device
     int* d_status = nullptr;        // device status word written by kernels that can give up
@@ -75,6 +76,9 @@ namespace hdc {
 // Records a message for hdc_last_error() and returns the status.
 int fail(int status, const std::string& msg);
 int cuda_fail(cudaError_t e, const char* what);
+
+// A call's workspace, freed with cudaFreeAsync on the same stream.
+cudaError_t scratch_alloc(const hdc_context* ctx, void** out, size_t bytes, cudaStream_t stream);
 
 inline bool valid_score_mode(int m) { return m == HDC_SCORE_NORM || m == HDC_SCORE_COS || m == HDC_SCORE_DOT; }
 

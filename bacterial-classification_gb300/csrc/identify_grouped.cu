@@ -748,7 +748,7 @@ int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t 
     };
     const size_t bytes = carve_all(nullptr);
     uint8_t* ws = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&ws), bytes, stream) != cudaSuccess) {
+    if (scratch_alloc(ctx, reinterpret_cast<void**>(&ws), bytes, stream) != cudaSuccess) {
         cudaGetLastError();
         return HDC_OK;  // no room: the per-read kernel needs none
     }

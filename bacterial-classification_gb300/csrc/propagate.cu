@@ -327,7 +327,7 @@ int propagate_scored(hdc_context* ctx, const int16_t* d_hv, const int64_t* d_nor
     auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t b_prev = align((size_t)n_slots * 4), b_tri = align((size_t)std::max<int64_t>(max_tri, 1) * 4),
                  b_na = align((size_t)n_parents * 4);
-    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&ws), b_prev + b_tri + b_na, stream)) != cudaSuccess)
+    if ((e = scratch_alloc(ctx, reinterpret_cast<void**>(&ws), b_prev + b_tri + b_na, stream)) != cudaSuccess)
         return cuda_fail(e, "propagate: workspace");
     GScoredArgs a{};
     a.hv = d_hv;
@@ -376,7 +376,7 @@ int propagate_scored(hdc_context* ctx, const int16_t* d_hv, const int64_t* d_nor
         }
         const size_t bytes = (ft.size() + tt.size()) * sizeof(GTile) + parents.size() * 4 + toff.size() * 8 + 64;
         uint8_t* tb = nullptr;
-        if ((e = cudaMallocAsync(reinterpret_cast<void**>(&tb), bytes, stream)) != cudaSuccess) {
+        if ((e = scratch_alloc(ctx, reinterpret_cast<void**>(&tb), bytes, stream)) != cudaSuccess) {
             st = cuda_fail(e, "propagate: tile list");
             break;
         }

@@ -98,3 +98,40 @@ def test_identify_under_capture(hdc, cuda):
         torch.cuda.synchronize()
         for a, b in zip(got, w):
             assert torch.equal(a, b)
+
+
+def test_workspaces_of_contexts_in_threads(hdc, cuda):
+    """Contexts that come and go in three threads share a workspace pool: every call on its own stream, same results."""
+    import threading
+    import torch
+    g = np.random.default_rng(11)
+    rows, node_rows, ptr, idx, roots = _tree(g, 3, 3, lambda rank, node: 10, 256, 140)
+    t = lambda a: torch.from_numpy(a).to(cuda)
+    tr, tree = t(rows), (t(node_rows), t(ptr), t(idx), torch.tensor(roots, dtype=torch.int32, device=cuda))
+    qs = [t(g.integers(-140, 141, (n, 256)).astype(np.int16)) for n in (3, 50, 400)]
+
+    def call(q):
+        ctx = hdc.Context(256, 8, 150, 10)
+        out = ctx.identify(q, ctx.norms(q), tr, ctx.norms(tr), *tree, 3, 5, -2.0)
+        torch.cuda.current_stream().synchronize()
+        assert ctx.status() == 0
+        return out
+    want = [call(q) for q in qs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for j in range(12):
+                    n = (i + j) % 3
+                    if not all(torch.equal(a, b) for a, b in zip(call(qs[n]), want[n])):
+                        bad.append((i, j))
+        except Exception as e:
+            bad.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not bad
