@@ -67,8 +67,8 @@ struct hdc_refdb {
     void* d_digits = nullptr;
     int digits = 0;
     __half* d_rows16 = nullptr;  // d_limbs itself when one limb holds every value
-    int32_t value_max = 0;       // largest |value| and squared norm, measured
-    int64_t norm2_max = 0;
+    int32_t value_max = 0;       // largest |value| and squared norms, measured: a row's, 64 dims' of a row (fp16 rows)
+    int64_t norm2_max = 0, block2_max = 0;
 };
 
 namespace hdc {

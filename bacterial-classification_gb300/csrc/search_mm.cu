@@ -11,10 +11,11 @@
 // Exactness.  fp32 adds integers exactly while every partial sum stays within 2^24.  By Cauchy-Schwarz no partial sum of
 // a dot exceeds |q| |r|, so one accumulator holds a whole dot wherever the largest norms (of the rows themselves) allow
 // it, as encoded reads and references do by far (D = 8,192: 3.8e6 for a 150 bp read and a 1,500 bp sequence).  Otherwise
-// the K loop runs in segments of at most 2^24 / sum_per_dim dims (the largest |q| times the largest |r|), each in a
-// fresh accumulator that the drain warps add to int32 registers while the next one fills (count-valued queries,
-// 19,456 x 50,000 at D = 8,192: 1,651 TFLOP/s whole, 1,204 in 9 segments).  Either way it needs neither smaller limbs
-// (more MMAs) nor CUDA-core arithmetic.
+// the K loop runs in segments, each in a fresh accumulator that the drain warps add to int32 registers while the next one
+// fills: of as many K blocks as the same inequality on the largest norms of 64 dims allows, or at least of 2^24 /
+// sum_per_dim dims (the largest |q| times the largest |r|), down to one MMA.  Count-valued reads of 250 bp against
+// references bundled of eight sequences, 4,000 x 50,000 at D = 10,240: six segments, 2.5 ms (1,626 TFLOP/s); a segment a
+// K block as the values alone have it 11.3 ms; three exact limbs of the smaller base they need 10.8 ms.
 //
 // Kernel (one CTA per SM, persistent, 4 warpgroups with their registers redistributed by setmaxnreg):
 //   * warp 0 TMA producer, warp 1 MMA issuer;
@@ -58,8 +59,9 @@ struct MmArgs {
     int64_t nq, nr, r0;
     int k, mode, limbs;
     int n_kb, kb_per_seg;  // K blocks of a tile, and of a segment
-    const unsigned long long* q_norm_max;  // largest squared norms of the queries and references (null: not used)
-    const unsigned long long* r_norm_max;
+    int mma_per_seg;       // F16: MMAs of a segment where a K block's four sum to too much (1 or 2, else 0)
+    const MmNorms* q_norms;  // largest squared norms of the queries and references (null: not used)
+    const MmNorms* r_norms;
     int n_qtiles, n_rtiles, G, S, n_groups, t_stride;
     double norm_limit;
     int stages;
@@ -170,6 +172,18 @@ struct MmShared {
 };
 constexpr uint32_t kFlush = 0xffffffffu;  // in a candidate's reference: the group's columns are all drained
 
+// sum += x + kAddWhole (modulo 2^32), for a whole |x| <= 2^24, in three float adds, one integer multiply-add and one
+// integer add: x + 1.5 * 2^34 rounds x to a multiple of 2^11, whose quotient and remainder are then read off the bits
+// below an exponent.  A segment's drain is bound by conversions at 16 a cycle and SM; with every other one made so, the
+// two pipes share them (4,000 x 20,000 queries and references of magnitude 100 and 2,000, D = 8,192, a segment a K
+// block: 4.40 -> 3.72 ms).
+constexpr uint32_t kAddWhole = 0x50C00000u * 2048u + 0x4B400000u;
+__device__ __forceinline__ void add_whole(int32_t& sum, float x) {
+    const float high = __fadd_rn(x, 25769803776.0f);                         // 0x50C00000 = 1.5 * 2^34
+    const float low = __fsub_rn(x, __fsub_rn(high, 25769803776.0f + 12582912.0f));  // remainder + 0x4B400000 = 1.5 * 2^23
+    sum = (int32_t)((uint32_t)sum + __float_as_uint(high) * 2048u + __float_as_uint(low));
+}
+
 // KR: a list's keys in KR registers (k <= KR) with its dots in shared memory; 0: lists in shared memory.
 template <bool F4, int CL, int KR>
 __global__ void __launch_bounds__(kThreadsMm, 1)
@@ -185,6 +199,7 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
     __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], accf_bar[2], acce_bar[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int err_s;
+    __shared__ int seg_s[2];  // K blocks of a segment; MMAs of one, where less than a K block
     const int stages = a.stages;
     const uint32_t stage_bytes = (uint32_t)mm_stage_bytes(T::A_BYTES, T::B_BYTES, a.limbs);
     MmShared& sh = *reinterpret_cast<MmShared*>(ring + (size_t)stages * stage_bytes);
@@ -205,6 +220,29 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
         tc::fence_mbar_init();
         tc::prefetch_tmap(&tmA);
         tc::prefetch_tmap(&tmB);
+    }
+    if (threadIdx.x == kThreadsMm - 1) {  // (a warp that sets nothing else up)
+        // One segment when the norms allow it: no partial sum of a dot, over whatever dims, exceeds |q| |r|
+        // (Cauchy-Schwarz).  Otherwise as many K blocks a segment as theirs allow: m of them sum to at most m |q_b| |r_b|.
+        int kbs = a.kb_per_seg, mmas = a.mma_per_seg;
+        if (a.q_norms) {
+            if ((double)a.q_norms->row * (double)a.r_norms->row <= a.norm_limit) {
+                kbs = a.n_kb;
+                mmas = 0;
+            } else if (!F4 && a.q_norms->block && a.r_norms->block) {
+                const double b = (double)a.q_norms->block * (double)a.r_norms->block;
+                const double room = (double)kMmMaxSum * (double)kMmMaxSum * (1 - 1e-9);  // (products are rounded)
+                int m = min(a.n_kb, (int)(kMmMaxSum * rsqrtf((float)b)) + 1);
+                while (m > 0 && (double)m * m * b > room) --m;
+                if (m > (mmas ? 0 : kbs)) {
+                    const int n = (a.n_kb + m - 1) / m;
+                    kbs = (a.n_kb + n - 1) / n;  // of even length
+                    mmas = 0;
+                }
+            }
+        }
+        seg_s[0] = kbs;
+        seg_s[1] = mmas;
     }
     if (threadIdx.x < kMmQueryTile) {
         for (int h = 0; h < 2; ++h) sh.head[h][threadIdx.x] = sh.tail[h][threadIdx.x] = 0;
@@ -237,9 +275,8 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
         tc::fence_after();
     }
     if constexpr (PAIR) tc::cluster_sync();  // the peer's barriers and scales exist before anything uses them
-    // One segment when the norms allow it: no partial sum of a dot, over whatever dims, exceeds |q| |r| (Cauchy-Schwarz)
-    int kb_per_seg = a.kb_per_seg;
-    if (a.q_norm_max && (double)*a.q_norm_max * (double)*a.r_norm_max <= a.norm_limit) kb_per_seg = a.n_kb;
+    const int kb_per_seg = seg_s[0], mma_per_seg = F4 ? 0 : seg_s[1];
+    const int n_segs = mma_per_seg ? a.n_kb * (4 / mma_per_seg) : (a.n_kb + kb_per_seg - 1) / kb_per_seg;
     const int crank = PAIR ? (int)tc::cluster_ctarank() : 0;
     const int gslot = (int)(blockIdx.x % a.G), lane_j = (int)(blockIdx.x / a.G);
     const int lead_slot = gslot & ~(CL - 1);  // a pair takes part in a group when its first CTA has a query tile
@@ -309,16 +346,59 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
             int64_t segs = 0;
+            auto acc_free = [&]() {  // the next accumulator is drained
+                const bool got = PAIR ? tc::mbar_wait_cluster(&acce_bar[acc], acc_phase ^ 1, &err_s, 2, a.wait_cycles)
+                                      : tc::mbar_wait(&acce_bar[acc], acc_phase ^ 1, &err_s, 2, a.wait_cycles);
+                tc::fence_after();
+                return got;
+            };
+            auto acc_done = [&]() {
+                if constexpr (PAIR)
+                    tc::mma_commit_pair_mc(&accf_bar[acc], 3);
+                else
+                    tc::mma_commit(&accf_bar[acc]);
+                ++segs;
+                if (++acc == 2) {
+                    acc = 0;
+                    acc_phase ^= 1;
+                }
+            };
+            auto stage_done = [&]() {
+                if constexpr (PAIR)
+                    tc::mma_commit_pair_mc(&empty_bar[stage], 3);
+                else
+                    tc::mma_commit(&empty_bar[stage]);
+                if (++stage == stages) {
+                    stage = 0;
+                    phase ^= 1;
+                }
+            };
+            auto mma16 = [&](uint32_t d0, uint64_t adesc, uint64_t bdesc, uint32_t on) {  // K = 16 fp16 = 32 bytes
+                if constexpr (PAIR)
+                    tc::mma_f16_pair(d0, adesc, bdesc, IDESC, on);
+                else
+                    tc::mma_f16(d0, adesc, bdesc, IDESC, on);
+            };
             for (int grp = 0; ok && grp < a.n_groups; ++grp) {
                 if (grp * a.G + lead_slot >= a.n_qtiles) continue;
                 for (int t0 = lane_j; ok && t0 < a.n_rtiles; t0 += a.S) {
-                    for (int k0 = 0; ok && k0 < a.n_kb; k0 += kb_per_seg) {
-                        if (!(PAIR ? tc::mbar_wait_cluster(&acce_bar[acc], acc_phase ^ 1, &err_s, 2, a.wait_cycles)
-                                   : tc::mbar_wait(&acce_bar[acc], acc_phase ^ 1, &err_s, 2, a.wait_cycles))) {
-                            ok = false;
-                            break;
-                        }
+                    for (int kb = 0; mma_per_seg && ok && kb < a.n_kb; ++kb) {
+                        if (!(ok = tc::mbar_wait(&full_bar[stage], phase, &err_s, 3, a.wait_cycles))) break;
                         tc::fence_after();
+                        const uint32_t sa = tc::smem_u32(ring + (size_t)stage * stage_bytes);
+                        const uint64_t adesc = tc::kmajor_desc(sa, T::SBO, T::LAYOUT);
+                        const uint64_t bdesc = tc::kmajor_desc(sa + (uint32_t)T::A_BYTES, T::SBO, T::LAYOUT);
+                        for (int kk = 0; ok && kk < 4; kk += mma_per_seg) {
+                            if (!(ok = acc_free())) break;
+                            const uint32_t d0 = tmem + (uint32_t)(acc * BN);
+                            for (int j = 0; j < mma_per_seg; ++j)
+                                mma16(d0, adesc + 2 * (kk + j), bdesc + 2 * (kk + j), j ? 1u : 0u);
+                            acc_done();
+                        }
+                        if (ok) stage_done();
+                    }
+                    for (int k0 = 0; !mma_per_seg && ok && k0 < a.n_kb; k0 += kb_per_seg) {
+                        if (!(ok = acc_free())) break;
                         const uint32_t d0 = tmem + (uint32_t)(acc * BN);
                         const int k1 = min(k0 + kb_per_seg, a.n_kb);
                         for (int kb = k0; kb < k1; ++kb) {
@@ -347,33 +427,13 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
                                 }
                             } else {
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk) {  // K = 16 fp16 per MMA = 32 bytes
-                                    const uint32_t on = (kb - k0) | kk ? 1u : 0u;
-                                    if constexpr (PAIR)
-                                        tc::mma_f16_pair(d0, adesc + 2 * kk, bdesc + 2 * kk, IDESC, on);
-                                    else
-                                        tc::mma_f16(d0, adesc + 2 * kk, bdesc + 2 * kk, IDESC, on);
-                                }
+                                for (int kk = 0; kk < 4; ++kk)
+                                    mma16(d0, adesc + 2 * kk, bdesc + 2 * kk, (kb - k0) | kk ? 1u : 0u);
                             }
-                            if constexpr (PAIR)
-                                tc::mma_commit_pair_mc(&empty_bar[stage], 3);
-                            else
-                                tc::mma_commit(&empty_bar[stage]);
-                            if (++stage == stages) {
-                                stage = 0;
-                                phase ^= 1;
-                            }
+                            stage_done();
                         }
                         if (!ok) break;
-                        if constexpr (PAIR)
-                            tc::mma_commit_pair_mc(&accf_bar[acc], 3);
-                        else
-                            tc::mma_commit(&accf_bar[acc]);
-                        ++segs;
-                        if (++acc == 2) {
-                            acc = 0;
-                            acc_phase ^= 1;
-                        }
+                        acc_done();
                     }
                 }
             }
@@ -400,7 +460,7 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
         const int row = quarter * 32 + lane;
         const int n_chunks = half ? T::NCH - T::NCH2 : T::NCH2;
         const uint32_t col_addr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * T::NCH2 * 16);
-        const bool multi = kb_per_seg < a.n_kb;
+        const bool multi = n_segs > 1;
         const int k = a.k;
         int acc = 0;
         uint32_t acc_phase = 0;
@@ -451,29 +511,36 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
                     for (int i = 0; i < T::NCH2; ++i)
 #pragma unroll
                         for (int c = 0; c < 16; ++c) sum[i][c] = 0;
-                    for (int k0 = 0; k0 < a.n_kb; k0 += kb_per_seg) {
+                    for (int s = 0; s < n_segs; ++s) {
                         if (!tc::mbar_wait(&accf_bar[acc], acc_phase, &err_s, 4, a.wait_cycles)) {
                             ok = false;
                             break;
                         }
                         tc::fence_after();
                         d0 = col_addr + (uint32_t)(acc * BN);
+                        uint32_t v[2][16];  // the next chunk is on its way while one is added
+                        tc::tmem_ld16(d0, v[0]);
 #pragma unroll
                         for (int i = 0; i < T::NCH2; ++i) {
-                            uint32_t v[16];
-                            tc::tmem_ld16(d0 + 16u * i, v);
                             tc::tmem_ld_wait();
+                            if (i + 1 < T::NCH2) tc::tmem_ld16(d0 + 16u * (i + 1), v[(i + 1) & 1]);
 #pragma unroll
-                            for (int c = 0; c < 16; ++c) sum[i][c] += __float2int_rn(__uint_as_float(v[c]));
+                            for (int c = 0; c < 16; ++c) {
+                                const float x = __uint_as_float(v[i & 1][c]);
+                                if (c & 1)
+                                    add_whole(sum[i][c], x);
+                                else
+                                    sum[i][c] += __float2int_rn(x);
+                            }
                         }
-                        if (k0 + kb_per_seg < a.n_kb) release();
+                        if (s + 1 < n_segs) release();
                     }
                     if (!ok) break;
 #pragma unroll
                     for (int i = 0; i < T::NCH2; ++i) {
                         uint32_t v[16];
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) v[c] = (uint32_t)sum[i][c];
+                        for (int c = 0; c < 16; ++c) v[c] = (uint32_t)sum[i][c] - (c & 1 ? (uint32_t)n_segs * kAddWhole : 0u);
                         if (i < n_chunks) tc::tmem_st16(d0 + 16u * i, v);
                     }
                     tc::tmem_st_wait();
@@ -857,15 +924,35 @@ __global__ void pack_refs_kernel(const int16_t* __restrict__ r16, const __half* 
     }
 }
 
-// A CTA's sum of squares, as the largest so far.
-__device__ __forceinline__ void block_norm_max(unsigned long long s, unsigned long long* out) {
-    __shared__ unsigned long long part[kRowThreads / 32];
+// Eight threads' sums of squares of 8 dims each, as the K block's (the lanes of `group` take part).
+template <typename T>
+__device__ __forceinline__ T kblock_norm(T s, uint32_t group) {
+    for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(group, s, o);
+    return s;
+}
+
+__device__ __forceinline__ uint32_t warp_most(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+__device__ __forceinline__ unsigned long long warp_most(unsigned long long v) {
+    for (int o = 16; o; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// A CTA's sum of squares and its threads' largest of a K block, as the largest so far.
+template <typename T>
+__device__ __forceinline__ void block_norm_max(unsigned long long s, T most, MmNorms* out) {
+    __shared__ MmNorms part[kRowThreads / 32];
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    unsigned long long b = warp_most(most);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = {s, b};
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < kRowThreads / 32; ++w) s += part[w];
-        if (s > *reinterpret_cast<volatile unsigned long long*>(out)) atomicMax(out, s);
+        for (int w = 1; w < kRowThreads / 32; ++w) {
+            s += part[w].row;
+            b = max(b, part[w].block);
+        }
+        const ulonglong2 now = __ldcg(reinterpret_cast<const ulonglong2*>(out));  // (both only ever grow)
+        if (s > now.x) atomicMax(&out->row, s);
+        if (b > now.y) atomicMax(&out->block, b);
     }
 }
 
@@ -873,10 +960,11 @@ __device__ __forceinline__ void block_norm_max(unsigned long long s, unsigned lo
 // a row, 8 elements a thread and step.  Bound by the bytes: 2 read and 2 written a value.
 template <bool VEC>
 __global__ void __launch_bounds__(kRowThreads) rows_f16_kernel(const int16_t* __restrict__ v, int dim, int64_t ld,
-                                                               __half* __restrict__ out,
-                                                               unsigned long long* __restrict__ norm_max) {
+                                                               __half* __restrict__ out, MmNorms* __restrict__ norms) {
     const int64_t row = blockIdx.x;
+    const uint32_t group = 0xffu << (threadIdx.x & 24);  // (ld is a multiple of 64: the eight run a step together)
     unsigned long long s = 0;
+    uint32_t most = 0;  // (64 values of magnitude <= 2048: 2^28)
     for (int d0 = threadIdx.x * 8; d0 < ld; d0 += kRowThreads * 8) {
         const int16_t* src = v + row * dim + d0;
         int16_t x[8];
@@ -887,33 +975,39 @@ __global__ void __launch_bounds__(kRowThreads) rows_f16_kernel(const int16_t* __
             for (int u = 0; u < 8; ++u) x[u] = d0 + u < dim ? src[u] : (int16_t)0;
         }
         __half h[8];
+        uint32_t p = 0;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             h[u] = __short2half_rn(x[u]);
-            s += (uint32_t)((int)x[u] * (int)x[u]);
+            p += (uint32_t)((int)x[u] * (int)x[u]);
         }
         *reinterpret_cast<uint4*>(out + row * ld + d0) = *reinterpret_cast<const uint4*>(h);
+        s += p;
+        most = max(most, kblock_norm(p, group));
     }
-    block_norm_max(s, norm_max);
+    block_norm_max(s, most, norms);
 }
 
-// the largest squared norm of fp16 integer rows (dim % 8 == 0, 16-byte aligned)
-__global__ void __launch_bounds__(kRowThreads) norm_max_kernel(const __half* __restrict__ v, int dim,
-                                                               unsigned long long other,
-                                                               unsigned long long* __restrict__ norm_max) {
-    unsigned long long s = 0;
+// the largest squared norms of fp16 integer rows (dim % 8 == 0, 16-byte aligned)
+__global__ void __launch_bounds__(kRowThreads) norm_max_kernel(const __half* __restrict__ v, int dim, MmNorms other,
+                                                               MmNorms* __restrict__ norms) {
+    const uint32_t group = 0xffu << (threadIdx.x & 24);
+    unsigned long long s = 0, most = 0;
     const uint4* src = reinterpret_cast<const uint4*>(v + (int64_t)blockIdx.x * dim);
-    for (int i = threadIdx.x; i < dim / 8; i += kRowThreads) {
-        const uint4 x = __ldg(src + i);
+    for (int i = threadIdx.x; i < (dim / 8 + 7) / 8 * 8; i += kRowThreads) {  // whole K blocks
+        const uint4 x = i < dim / 8 ? __ldg(src + i) : make_uint4(0, 0, 0, 0);
         const __half* h = reinterpret_cast<const __half*>(&x);
+        unsigned long long p = 0;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int e = __half2int_rn(h[u]);
-            s += (unsigned long long)((long long)e * e);
+            p += (unsigned long long)((long long)e * e);
         }
+        s += p;
+        most = max(most, kblock_norm(p, group));
     }
-    block_norm_max(s, norm_max);
-    if (blockIdx.x == 0 && threadIdx.x == 0) norm_max[1] = other;
+    block_norm_max(s, most, norms);
+    if (blockIdx.x == 0 && threadIdx.x == 0) norms[1] = other;
 }
 
 // the values of a database's limbs (dim % 8 == 0), 8 elements a thread
@@ -1144,7 +1238,7 @@ size_t mm_f4_ref_bytes(int64_t nr, int dim, int limbs) {
     return (size_t)((nr + 2 * kMmF4Half - 1) / (2 * kMmF4Half)) * 2 * kMmF4Half * n_kblocks(dim, true) * 64 * limbs;
 }
 
-bool mm_sums_fit(bool f4, int64_t sum_per_dim) { return sum_per_dim * (f4 ? kMmF4Dims : 64) <= kMmMaxSum; }
+bool mm_sums_fit(bool f4, int64_t sum_per_dim) { return sum_per_dim * (f4 ? kMmF4Dims : 16) <= kMmMaxSum; }
 
 int mm_pack_queries(const void* d_q, bool is_f16, int64_t nq, int dim, void* out, cudaStream_t stream) {
     const int n_kb = n_kblocks(dim, true);
@@ -1193,20 +1287,19 @@ int mm_pack_refs(const int16_t* d_r, const __half* limbs16, int L16, int bits, i
     }, "mm search: pack references");
 }
 
-int mm_rows_f16(const int16_t* d_v, int64_t n, int dim, int64_t ld, __half* out, unsigned long long* norm_max,
+int mm_rows_f16(const int16_t* d_v, int64_t n, int dim, int64_t ld, __half* out, MmNorms* norms,
                 cudaStream_t stream) {
     return check_launch([&] {
         if (dim % 8 == 0 && aligned16(d_v))
-            rows_f16_kernel<true><<<(unsigned)n, kRowThreads, 0, stream>>>(d_v, dim, ld, out, norm_max);
+            rows_f16_kernel<true><<<(unsigned)n, kRowThreads, 0, stream>>>(d_v, dim, ld, out, norms);
         else
-            rows_f16_kernel<false><<<(unsigned)n, kRowThreads, 0, stream>>>(d_v, dim, ld, out, norm_max);
+            rows_f16_kernel<false><<<(unsigned)n, kRowThreads, 0, stream>>>(d_v, dim, ld, out, norms);
     }, "mm search: fp16 rows");
 }
 
-int mm_norm_max(const __half* d_v, int64_t n, int dim, unsigned long long other, unsigned long long* norm_max,
-                cudaStream_t stream) {
+int mm_norm_max(const __half* d_v, int64_t n, int dim, MmNorms other, MmNorms* norms, cudaStream_t stream) {
     return check_launch([&] {
-        norm_max_kernel<<<(unsigned)n, kRowThreads, 0, stream>>>(d_v, dim, other, norm_max);
+        norm_max_kernel<<<(unsigned)n, kRowThreads, 0, stream>>>(d_v, dim, other, norms);
     }, "mm search: largest norm");
 }
 
@@ -1253,6 +1346,7 @@ int mm_search(hdc_context* ctx, const MmOperands& op, int64_t nq, int64_t nr, in
     const int64_t most = std::max<int64_t>(1, kMmMaxSum / (op.sum_per_dim * kb_dims));  // K blocks of a segment
     const int64_t segs = (a.n_kb + most - 1) / most;
     a.kb_per_seg = (int)((a.n_kb + segs - 1) / segs);
+    if (!op.f4 && op.sum_per_dim * 64 > kMmMaxSum) a.mma_per_seg = op.sum_per_dim * 32 > kMmMaxSum ? 1 : 2;
     a.n_qtiles = p.n_qtiles;
     const int n = p.CL == 2 ? (op.f4 ? MmTile<true, 2>::N : MmTile<false, 2>::N)
                             : (op.f4 ? MmTile<true, 1>::N : MmTile<false, 1>::N);
@@ -1272,10 +1366,11 @@ int mm_search(hdc_context* ctx, const MmOperands& op, int64_t nq, int64_t nr, in
     a.ws_dot = reinterpret_cast<int64_t*>(a.ws_key + (size_t)p.S * nq * k);
     a.status = ctx->d_status;
     a.wait_cycles = ctx->wait_cycles > 0 ? ctx->wait_cycles : tc::kWaitCycles;
-    if (segs > 1 && op.one_segment) a.kb_per_seg = a.n_kb;
-    if (segs > 1 && !op.one_segment && op.q_norm_max) {
-        a.q_norm_max = op.q_norm_max;
-        a.r_norm_max = op.r_norm_max;
+    const bool several = segs > 1 || a.mma_per_seg;
+    if (several && op.one_segment) a.kb_per_seg = a.n_kb;
+    if (several && !op.one_segment && op.q_norms) {
+        a.q_norms = op.q_norms;
+        a.r_norms = op.r_norms;
         a.norm_limit = op.f4 ? mm_f4_norm_limit(op.limbs, dim) : (double)kMmMaxSum * (double)kMmMaxSum;
     }
     if (shape) {

@@ -8,6 +8,11 @@ namespace hdc {
 // How a search's operands reach the tensor cores.  F16: queries and references as fp16 integers (|v| <= 2048),
 // row-major.  F4: +1/0/-1 queries and references split into balanced base-8 digits (-4 .. 4), both as packed e2m1
 // in the tile order of mm_pack_*; the digits' weights are the MMA's power-of-two scales.
+// Largest squared norms of a set of rows: of whole rows, and of any 64 dims of a K block.
+struct alignas(16) MmNorms {
+    unsigned long long row, block;
+};
+
 struct MmOperands {
     bool f4 = false;
     const void* a = nullptr;    // F16: [nq][lda] fp16; F4: mm_pack_queries' tiles
@@ -16,10 +21,10 @@ struct MmOperands {
     int limbs = 1;              // F4: base-8 digits
     int64_t sum_per_dim = 1;    // no partial sum over n dims exceeds n times this
     // Whether a whole dot stays within 2^24 (one segment): known to the host, or decided on the device from the largest
-    // squared norms of the rows as they are (not the caller's, which only the scores use), both pointers set.
+    // squared norms of the rows as they are (not the caller's, which only the scores use), both pointers set (F16).
     bool one_segment = false;
-    const unsigned long long* q_norm_max = nullptr;
-    const unsigned long long* r_norm_max = nullptr;
+    const MmNorms* q_norms = nullptr;
+    const MmNorms* r_norms = nullptr;
     const int64_t* qn = nullptr;
     const float* rr = nullptr;  // references: 1 / sqrt(norm2) in fp32; sqrt(norm2); its reciprocal
     const double* rs = nullptr;
@@ -37,20 +42,18 @@ int mm_f4_limbs(int64_t max_abs);
 int64_t mm_f4_sum_per_dim(int64_t max_abs);
 size_t mm_f4_query_bytes(int64_t nq, int dim);
 size_t mm_f4_ref_bytes(int64_t nr, int dim, int limbs);
-// Whether the accumulators can be emptied often enough (at least once a K block).
+// Whether the accumulators can be emptied often enough (after every MMA at most; digits: every K block).
 bool mm_sums_fit(bool f4, int64_t sum_per_dim);
 
 int mm_pack_queries(const void* d_q, bool is_f16, int64_t nq, int dim, void* out, cudaStream_t stream);
 // references from int16 rows, or (limbs16 != null) from a database's fp16 limbs
 int mm_pack_refs(const int16_t* d_r, const __half* limbs16, int L16, int bits, int64_t r_pad, int64_t nr, int dim,
                  int limbs, void* out, cudaStream_t stream);
-// int16 rows -> fp16 rows of ld elements, zero past dim; *norm_max = max(*norm_max, the largest squared norm)
-int mm_rows_f16(const int16_t* d_v, int64_t n, int dim, int64_t ld, __half* out, unsigned long long* norm_max,
+// int16 rows -> fp16 rows of ld elements, zero past dim; *norms = max(*norms, theirs)
+int mm_rows_f16(const int16_t* d_v, int64_t n, int dim, int64_t ld, __half* out, MmNorms* norms,
                 cudaStream_t stream);
-// *norm_max = max(*norm_max, the largest squared norm of fp16 integer rows of dim elements, dim % 8 == 0), and
-// norm_max[1] = other
-int mm_norm_max(const __half* d_v, int64_t n, int dim, unsigned long long other, unsigned long long* norm_max,
-                cudaStream_t stream);
+// norms[0] = max(norms[0], those of fp16 integer rows of dim elements, dim % 8 == 0), and norms[1] = other
+int mm_norm_max(const __half* d_v, int64_t n, int dim, MmNorms other, MmNorms* norms, cudaStream_t stream);
 // F4: the largest |q|^2 |r|^2 at which one segment is exact
 double mm_f4_norm_limit(int limbs, int dim);
 // the values of a database's limbs as one fp16 row each
@@ -63,7 +66,7 @@ int mm_norm_tables(const int64_t* d_n2, int64_t n, float* rr, double* rs, double
 
 // Workspace of a search's lists for nq queries against nr references (a launch of nr or fewer); its first
 // kMmWorkWords 64-bit words are the caller's.
-constexpr int kMmWorkWords = 2;
+constexpr int kMmWorkWords = 4;
 size_t mm_list_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int dim, int k, bool f4, int limbs);
 // Clears the words and the thresholds of nq queries: before the first launch of a call.
 int mm_begin(void* work, int64_t nq, cudaStream_t stream);

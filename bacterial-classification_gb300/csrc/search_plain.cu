@@ -422,7 +422,7 @@ static PlainMm plain_mm_shape(const hdc_context* ctx, int64_t nq, int64_t nr, in
     p.nrc = std::min<int64_t>(nr, std::max<int64_t>(1, (int64_t)(kMmChunkBytes / r_of(ru))) * ru);
     p.q_bytes = mm_round(q_of(p.nqc));
     p.r_bytes = mm_round(r_of(p.nrc));
-    p.t_bytes = mm_round(sizeof(unsigned long long) + (size_t)p.nrc * (2 * sizeof(double) + sizeof(float)));
+    p.t_bytes = mm_round(sizeof(MmNorms) + (size_t)p.nrc * (2 * sizeof(double) + sizeof(float)));
     p.l_bytes = mm_list_bytes(ctx, p.nqc, p.nrc, dim, k, f4, limbs);
     if (nq > p.nqc) p.l_bytes = std::max(p.l_bytes, mm_list_bytes(ctx, (nq - 1) % p.nqc + 1, p.nrc, dim, k, f4, limbs));
     return p;
@@ -450,8 +450,8 @@ static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, co
     uint8_t* w = static_cast<uint8_t*>(d_work);
     uint8_t* wq = w;
     uint8_t* wr = wq + p.q_bytes;
-    unsigned long long* r_norm_max = reinterpret_cast<unsigned long long*>(wr + p.r_bytes);
-    double* rs = reinterpret_cast<double*>(r_norm_max + 1);
+    MmNorms* r_norms = reinterpret_cast<MmNorms*>(wr + p.r_bytes);
+    double* rs = reinterpret_cast<double*>(r_norms + 1);
     double* ri = rs + p.nrc;
     float* rr = reinterpret_cast<float*>(ri + p.nrc);
     void* lists = wr + p.r_bytes + p.t_bytes;
@@ -462,10 +462,10 @@ static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, co
     op.rs = rs;
     op.ri = ri;
     if (!op.f4) {
-        op.q_norm_max = static_cast<unsigned long long*>(lists);
-        op.r_norm_max = r_norm_max;
+        op.q_norms = static_cast<MmNorms*>(lists);
+        op.r_norms = r_norms;
     }
-    const cudaError_t e = cudaMemsetAsync(r_norm_max, 0, sizeof(unsigned long long), stream);
+    const cudaError_t e = cudaMemsetAsync(r_norms, 0, sizeof(MmNorms), stream);
     int st = e == cudaSuccess ? HDC_OK : cuda_fail(e, "search: clear the largest norm");
     for (int64_t q0 = 0; q0 < nq && st == HDC_OK; q0 += p.nqc) {
         const int64_t n = std::min(p.nqc, nq - q0);
@@ -474,12 +474,12 @@ static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, co
         if (st == HDC_OK)
             st = op.f4 ? mm_pack_queries(d_q + q0 * dim, false, n, dim, wq, stream)
                        : mm_rows_f16(d_q + q0 * dim, n, dim, op.lda, reinterpret_cast<__half*>(wq),
-                                     static_cast<unsigned long long*>(lists), stream);
+                                     static_cast<MmNorms*>(lists), stream);
         for (int64_t r0 = 0; r0 < nr && st == HDC_OK; r0 += p.nrc) {
             const int64_t m = std::min(p.nrc, nr - r0);
             if (q0 == 0 || p.nrc < nr) {  // one chunk stays converted for every batch
                 st = op.f4 ? mm_pack_refs(d_r + r0 * dim, nullptr, 1, 0, 0, m, dim, op.limbs, wr, stream)
-                           : mm_rows_f16(d_r + r0 * dim, m, dim, op.ldb, reinterpret_cast<__half*>(wr), r_norm_max, stream);
+                           : mm_rows_f16(d_r + r0 * dim, m, dim, op.ldb, reinterpret_cast<__half*>(wr), r_norms, stream);
                 if (st == HDC_OK) st = mm_norm_tables(d_rn + r0, m, rr, rs, ri, stream);
             }
             if (st == HDC_OK)

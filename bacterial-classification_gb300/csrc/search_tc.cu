@@ -906,27 +906,39 @@ int refdb_forms(hdc_refdb* db, cudaStream_t stream) {
     if (db->limb_bits == 11) {
         const int digits = mm_f4_limbs(db->value_max);
         const size_t bytes = digits ? mm_f4_ref_bytes(db->nr, db->dim, digits) : 0;
-        if (!digits || bytes / 64 > 0x7fffffff) return HDC_OK;  // TMA coordinates are 32-bit
-        if (cudaMalloc(&db->d_digits, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            db->d_digits = nullptr;
-            return HDC_OK;
+        if (digits && bytes / 64 <= 0x7fffffff) {  // TMA coordinates are 32-bit
+            if (cudaMalloc(&db->d_digits, bytes) == cudaSuccess) {
+                db->digits = digits;
+                st = mm_pack_refs(nullptr, db->d_limbs, db->L, db->limb_bits, db->r_pad, db->nr, db->dim, digits,
+                                  db->d_digits, stream);
+            } else {
+                cudaGetLastError();
+                db->d_digits = nullptr;
+            }
         }
-        db->digits = digits;
-        st = mm_pack_refs(nullptr, db->d_limbs, db->L, db->limb_bits, db->r_pad, db->nr, db->dim, digits, db->d_digits,
-                          stream);
     } else if (db->L > 1 && db->value_max <= 2048) {
-        if (cudaMalloc(&db->d_rows16, (size_t)db->r_pad * db->dim * sizeof(__half)) != cudaSuccess) {
+        if (cudaMalloc(&db->d_rows16, (size_t)db->r_pad * db->dim * sizeof(__half)) == cudaSuccess) {
+            st = mm_rows_from_limbs(db->d_limbs, db->L, db->limb_bits, db->r_pad, db->dim, db->d_rows16, stream);
+        } else {
             cudaGetLastError();
             db->d_rows16 = nullptr;
-            return HDC_OK;
         }
-        st = mm_rows_from_limbs(db->d_limbs, db->L, db->limb_bits, db->r_pad, db->dim, db->d_rows16, stream);
+    }
+    MmNorms* d_norms = nullptr;
+    if (st == HDC_OK && db->d_rows16) {
+        e = cudaMalloc(&d_norms, 2 * sizeof(MmNorms));
+        if (e == cudaSuccess) e = cudaMemsetAsync(d_norms, 0, 2 * sizeof(MmNorms), stream);
+        st = e == cudaSuccess ? mm_norm_max(db->d_rows16, db->nr, db->dim, {}, d_norms, stream)
+                              : cuda_fail(e, "refdb: allocation");
+        if (st == HDC_OK)
+            e = cudaMemcpyAsync(&db->block2_max, &d_norms->block, sizeof(int64_t), cudaMemcpyDeviceToHost, stream);
+        if (st == HDC_OK && e != cudaSuccess) st = cuda_fail(e, "refdb: largest norm of a K block");
     }
     if (st == HDC_OK) {
         e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) st = cuda_fail(e, "refdb: search forms");
     }
+    cudaFree(d_norms);
     return st;
 }
 
@@ -1088,7 +1100,7 @@ static bool tc_auto_schedule(const hdc_context* ctx) {
 }
 
 // The operand form for queries of magnitude up to maxq, or none: +1/0/-1 queries on the base-8 digits, others on the
-// fp16 rows while a K block's sums stay within 2^24 and a dot within int32.
+// fp16 rows while an MMA's sums stay within 2^24 and a dot within int32.
 static bool mm_form(const hdc_context* ctx, const hdc_refdb* db, int64_t nq, int32_t maxq, MmOperands& op) {
     if (!tc_auto_schedule(ctx)) return false;
     const bool f4 = maxq <= 1 && db->d_digits;
@@ -1361,10 +1373,11 @@ int launch_search_tc(hdc_context* ctx, const hdc_refdb* db, const __half* d_q, c
         op.qn = d_qn;
         if (st == HDC_OK) st = mm_begin(lists, nq, stream);
         if (st == HDC_OK && !op.f4) {
-            unsigned long long* words = static_cast<unsigned long long*>(lists);
-            st = mm_norm_max(d_q, nq, ctx->dim, (unsigned long long)db->norm2_max, words, stream);
-            op.q_norm_max = words;
-            op.r_norm_max = words + 1;
+            MmNorms* norms = static_cast<MmNorms*>(lists);
+            st = mm_norm_max(d_q, nq, ctx->dim, {(unsigned long long)db->norm2_max, (unsigned long long)db->block2_max}, norms,
+                             stream);
+            op.q_norms = norms;
+            op.r_norms = norms + 1;
         }
         if (st == HDC_OK)
             st = mm_search(ctx, op, nq, db->nr, 0, db->nr, ctx->dim, k, mode, lists, true, ctx->tc_last_shape, stream);

@@ -40,7 +40,11 @@ def _values(g, n, dim, vmax, dtype=np.int16):
     (2500, 300, 600, 5, 1, 2048, 125),    # a segment a K block
     (2500, 300, 600, 12, 2, 500, 500),    # a segment a K block, both large
     (1024, 140, 300, 5, 0, 2048, 128),    # the largest product that a K block's sums allow
-    (1024, 140, 300, 5, 0, 2048, 129),    # one above: CUDA cores
+    (1024, 140, 300, 5, 0, 2048, 129),    # one above: a segment two MMAs
+    (1024, 140, 300, 5, 0, 2048, 256),    # the largest product of those
+    (1100, 300, 700, 5, 1, 2048, 257),    # one above: a segment an MMA
+    (1000, 40, 300, 9, 0, 1023, 1025),    # the largest product accepted
+    (1030, 300, 600, 7, 2, 300, 300),     # several K blocks a segment by their norms, where the products allow two
     (1024, 140, 300, 5, 0, 1, 12000),     # +1/0/-1 queries on digits
     (300, 129, 225, 10, 2, 1, 18724),     # five digits at their largest
     (777, 17, 113, 20, 1, 1, 2341),       # five digits, the least that needs them
