@@ -607,6 +607,8 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
                             open = n < k || n > k + kSlack;
                         }
                     }
+                    // (a zero norm's COS estimate is 0 but its score -1: no k columns are known to reach an estimate below)
+                    if (a.mode == HDC_SCORE_COS && lo <= 0.0f) lo = -1.0f;
                     if (n_pass > k + kSlack) thr = fmaxf(thr, mm_filter_below(lo, a.mode));
                 }
                 if (__any_sync(0xffffffffu, n_pass != 0)) {

@@ -110,3 +110,23 @@ def test_plain_reference_chunks_equal_the_cuda_core_kernel(hdc, cuda):
     assert full > 64 << 20 and ctx.status() == 0
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("nq,nr", [(3, 64), (140, 20000)])
+def test_plain_zero_norm_references_among_negative_scores(hdc, orc, cuda, nq, nr, mode):
+    """A zero-norm reference scores -1 in every mode but DOT, below any negative cosine: many of them in a tile may not
+    raise the threshold that the others are filtered by."""
+    import torch
+    g = np.random.default_rng(nr)
+    dim = 72
+    q = g.integers(1, 60, (nq, dim)).astype(np.int16)
+    r = -g.integers(0, 60, (nr, dim)).astype(np.int16)
+    r[g.random(nr) < 0.7] = 0
+    r[nr // 2:, ::2] = 0
+    ctx = hdc.Context(dim, 8, 150, 10)
+    tq, tr = torch.from_numpy(q).to(cuda), torch.from_numpy(r).to(cuda)
+    got = ctx.search_plain(tq, ctx.norms(tq), 60, tr, ctx.norms(tr), 60, 5, mode)
+    torch.cuda.synchronize()
+    assert ctx.status() == 0
+    _check(got, orc, q, r, 5, mode)
