@@ -765,6 +765,319 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
     if constexpr (PAIR) tc::cluster_sync();  // no CTA leaves while its peer may still write into it
 }
 
+// ---------------------------------------------------------------- small problems: the K loop split over CTAs
+// A problem with fewer tiles than SMs leaves most of them idle, and its time is one tile's K loop (157 K blocks of 330
+// cycles at D = 10,000, bound by the issuer's waits and commits) plus lists, thresholds and a merge made for thousands of
+// tiles.  Here the CTAs of a tile share its K blocks, each stores the whole dots of its part (at most 5 MB in all), and
+// one CTA a query adds the parts up and selects.  48 x 2,000 at D = 10,000: 80 -> 40 us with
+// its conversion; 190 x 567 at D = 1,024, top-32: 200 -> 36.
+constexpr int kDotThreads = 192;   // producer, MMA issuer, four drain warps
+constexpr int kSplitRefs = 12288;  // a query's dots and keys in shared memory
+constexpr int kMinSplitBlocks = 4; // K blocks that a CTA is worth starting for
+
+struct DotsArgs {
+    int64_t nq;
+    int n_kb, kb_per_seg, limbs, stages, n_rtiles, splits, ldd, withhold;
+    int32_t* parts;  // [splits][nq][ldd]
+    int* status;
+    long long wait_cycles;
+};
+
+template <bool F4>
+__global__ void __launch_bounds__(kDotThreads, 1)
+    mm_dots_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const DotsArgs a) {
+    using T = MmTile<F4, 1>;
+    constexpr int BN = T::N;
+    constexpr uint32_t IDESC = F4 ? tc::idesc_f4_f32(kMmQueryTile, BN) : tc::idesc_f16_f32(kMmQueryTile, BN);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* ring = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
+    __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], accf_bar[2], acce_bar[2];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ volatile int err_s;
+    const int stages = a.stages, stage_bytes = mm_stage_bytes(T::A_BYTES, T::B_BYTES, a.limbs);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        err_s = 0;
+        for (int s = 0; s < stages; ++s) {
+            tc::mbar_init(&full_bar[s], 1);
+            tc::mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&accf_bar[b], 1);
+            tc::mbar_init(&acce_bar[b], 4);
+        }
+        tc::fence_mbar_init();
+        tc::prefetch_tmap(&tmA);
+        tc::prefetch_tmap(&tmB);
+    }
+    if (warp == 1) {
+        tc::tmem_alloc(&tmem_base_s, 512);
+        tc::tmem_relinquish();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = tmem_base_s;
+    if constexpr (F4) {  // the digits' block scales, as in mm_search_kernel
+        if (warp < 4) {
+            uint32_t v[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0x01010101u * (uint32_t)(127 + 3 * (i / 8));
+            tc::tmem_st32(tmem + ((uint32_t)(warp * 32) << 16) + kScaleCol, v);
+            tc::tmem_st_wait();
+        }
+        tc::fence_before();
+        __syncthreads();
+        tc::fence_after();
+    }
+    // this CTA's tile and K blocks
+    const int split = (int)(blockIdx.x % a.splits), tile = (int)(blockIdx.x / a.splits);
+    const int rt = tile % a.n_rtiles, qt = tile / a.n_rtiles;
+    const int kb0 = (int)((int64_t)split * a.n_kb / a.splits), kb1 = (int)((int64_t)(split + 1) * a.n_kb / a.splits);
+    if (warp == 0) {
+        if (tc::elect_one()) {
+            int stage = 0, issued = 0;
+            uint32_t phase = 0;
+            for (int kb = kb0; !a.withhold && kb < kb1; ++kb) {
+                if (!tc::mbar_wait(&empty_bar[stage], phase ^ 1, &err_s, 1, a.wait_cycles)) break;
+                uint8_t* st = ring + (size_t)stage * stage_bytes;
+                tc::mbar_arrive_expect_tx(&full_bar[stage], stage_bytes);
+                if constexpr (F4) {
+                    tc::tma_load_2d(st, &tmA, &full_bar[stage], 0, (qt * a.n_kb + kb) * kMmQueryTile);
+                    const int y = (((rt >> 1) * a.n_kb + kb) * 2 + (rt & 1)) * a.limbs * kMmF4Half;
+                    for (int l = 0; l < a.limbs; ++l)
+                        tc::tma_load_2d(st + T::A_BYTES + l * T::B_BYTES, &tmB, &full_bar[stage], 0, y + l * kMmF4Half);
+                } else {
+                    tc::tma_load_2d(st, &tmA, &full_bar[stage], kb * 64, qt * kMmQueryTile);
+                    tc::tma_load_2d(st + T::A_BYTES, &tmB, &full_bar[stage], kb * 64, rt * BN);
+                }
+                ++issued;
+                if (++stage == stages) {
+                    stage = 0;
+                    phase ^= 1;
+                }
+            }
+            // the last loads land before the CTA leaves (bounded)
+            for (int i = 0; i < min(issued, stages); ++i) {
+                if (--stage < 0) {
+                    stage = stages - 1;
+                    phase ^= 1;
+                }
+                const long long c0 = clock64();
+                while (!tc::mbar_try_wait(tc::smem_u32(&full_bar[stage]), phase) && clock64() - c0 < tc::kWaitCycles) {
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (tc::elect_one()) {
+            int stage = 0, acc = 0;
+            uint32_t phase = 0, acc_phase = 0;
+            bool ok = true;
+            for (int k0 = kb0; ok && k0 < kb1; k0 += a.kb_per_seg) {
+                if (!(ok = tc::mbar_wait(&acce_bar[acc], acc_phase ^ 1, &err_s, 2, a.wait_cycles))) break;
+                tc::fence_after();
+                const uint32_t d0 = tmem + (uint32_t)(acc * BN);
+                for (int kb = k0; kb < min(k0 + a.kb_per_seg, kb1); ++kb) {
+                    if (!(ok = tc::mbar_wait(&full_bar[stage], phase, &err_s, 3, a.wait_cycles))) break;
+                    tc::fence_after();
+                    const uint32_t sa = tc::smem_u32(ring + (size_t)stage * stage_bytes);
+                    const uint64_t adesc = tc::kmajor_desc(sa, T::SBO, T::LAYOUT);
+                    const uint64_t bdesc = tc::kmajor_desc(sa + (uint32_t)T::A_BYTES, T::SBO, T::LAYOUT);
+                    if constexpr (F4) {
+                        for (int l = 0; l < a.limbs; ++l) {
+                            const uint32_t sfa = tmem + kScaleCol + (l == 4 ? 8u : 0u);
+                            const uint32_t sfb = tmem + kScaleCol + 8u * (uint32_t)(l == 4 ? 3 : l);
+                            const uint64_t bl = bdesc + (uint64_t)(l * (T::B_BYTES >> 4));
+#pragma unroll
+                            for (int kk = 0; kk < 2; ++kk)
+                                tc::mma_f4(d0, adesc + 2 * kk, bl + 2 * kk, IDESC, sfa, sfb, (kb - k0) | l | kk ? 1u : 0u);
+                        }
+                    } else {
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            tc::mma_f16(d0, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (kb - k0) | kk ? 1u : 0u);
+                    }
+                    tc::mma_commit(&empty_bar[stage]);
+                    if (++stage == stages) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                }
+                if (!ok) break;
+                tc::mma_commit(&accf_bar[acc]);
+                if (++acc == 2) {
+                    acc = 0;
+                    acc_phase ^= 1;
+                }
+            }
+        }
+    } else {
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        const int64_t gq = (int64_t)qt * kMmQueryTile + row;
+        int32_t sum[BN];
+#pragma unroll
+        for (int c = 0; c < BN; ++c) sum[c] = 0;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        for (int k0 = kb0; k0 < kb1; k0 += a.kb_per_seg) {
+            if (!(ok = tc::mbar_wait(&accf_bar[acc], acc_phase, &err_s, 4, a.wait_cycles))) break;
+            tc::fence_after();
+            const uint32_t d0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
+#pragma unroll
+            for (int i = 0; i < BN / 16; ++i) {
+                uint32_t v[16];
+                tc::tmem_ld16(d0 + 16u * i, v);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 16; ++c) sum[16 * i + c] += __float2int_rn(__uint_as_float(v[c]));
+            }
+            tc::fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&acce_bar[acc]);
+            if (++acc == 2) {
+                acc = 0;
+                acc_phase ^= 1;
+            }
+        }
+        if (ok && gq < a.nq) {
+            int4* out = reinterpret_cast<int4*>(a.parts + ((int64_t)split * a.nq + gq) * a.ldd + (int64_t)rt * BN);
+#pragma unroll
+            for (int i = 0; i < BN / 4; ++i) out[i] = make_int4(sum[4 * i], sum[4 * i + 1], sum[4 * i + 2], sum[4 * i + 3]);
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc::fence_after();
+        tc::tmem_dealloc(tmem, 512);
+    }
+    if (threadIdx.x == 0 && err_s) atomicCAS(a.status, 0, 100 + err_s);
+}
+
+// One CTA a query: its dots from the parts, a threshold that at least k of them are known to reach (by bisection of the
+// threads' best estimates), exact scores of those that an estimate lets through, and their order by counting.  Bound by
+// the latency of that chain for a few queries, and by the FP64 pipe (two lanes a cycle) for thousands.
+template <int NT>
+__global__ void __launch_bounds__(NT) mm_select_kernel(
+    const int32_t* __restrict__ parts, int splits, int64_t nq, int nr, int ldd, const int64_t* __restrict__ qn,
+    const float* __restrict__ rr, const double* __restrict__ rs, const double* __restrict__ ri, int k, int mode,
+    float* __restrict__ out_s, int32_t* __restrict__ out_i, double* __restrict__ out_c, int64_t* __restrict__ out_d) {
+    extern __shared__ uint64_t keys[];  // [nr], then the dots
+    int32_t* dots = reinterpret_cast<int32_t*>(keys + nr);
+    __shared__ uint64_t warp_best[2][NT / 32];
+    __shared__ uint32_t warp_ord[2][NT / 32];
+    __shared__ double root_s[2];
+    __shared__ int n_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t q = blockIdx.x, n2 = qn[q];
+    if (tid == NT - 1) {  // (with the fewest references)
+        n_s = 0;
+        root_s[0] = __dsqrt_rn((double)n2);
+        root_s[1] = n2 ? __drcp_rn(root_s[0]) : 0.0;
+    }
+    const float rq = n2 ? __frsqrt_rn(__ll2float_rn(n2)) : 0.0f;
+    // a reference's estimate; under COS a zero norm scores -1, where the product would be 0
+    auto estimate = [&](int32_t dot, float f) {
+        return mode == HDC_SCORE_COS && (f == 0.0f || rq == 0.0f) ? -1.0f : approx_score((float)dot, rq, f, mode);
+    };
+    float best = -INFINITY;
+    for (int j = 4 * tid; j < nr; j += 4 * NT) {  // (ldd is a multiple of 16, and the parts are written that far)
+        const int32_t* from = parts + q * ldd + j;
+        const int64_t step = nq * ldd;
+        int4 d = make_int4(0, 0, 0, 0);
+#pragma unroll 8
+        for (int s = 0; s < splits; ++s) {
+            const int4 x = __ldcg(reinterpret_cast<const int4*>(from + s * step));
+            d.x += x.x;
+            d.y += x.y;
+            d.z += x.z;
+            d.w += x.w;
+        }
+        const int32_t v[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (j + u < nr) {
+                dots[j + u] = v[u];
+                best = fmaxf(best, estimate(v[u], __ldg(rr + j + u)));
+            }
+    }
+    const uint32_t mine_ord = ord_float(best), none = ord_float(-INFINITY);
+    const uint32_t top_ord = __reduce_max_sync(0xffffffffu, mine_ord);
+    const uint32_t low_ord = __reduce_min_sync(0xffffffffu, mine_ord == none ? 0xffffffffu : mine_ord);
+    if (lane == 0) {
+        warp_ord[0][warp] = low_ord;
+        warp_ord[1][warp] = top_ord;
+    }
+    __syncthreads();
+    float thr = -INFINITY;
+    if (min(NT, (nr + 3) / 4) >= k) {  // as many threads have a best
+        uint32_t a = warp_ord[0][0], b = warp_ord[1][0];
+#pragma unroll
+        for (int w = 1; w < NT / 32; ++w) {
+            a = min(a, warp_ord[0][w]);
+            b = max(b, warp_ord[1][w]);
+        }
+        float lo = unord_float(a), hi = unord_float(b);  // all of them reach lo
+        for (int it = 0; it < 12; ++it) {
+            const float mid = 0.5f * (lo + hi);
+            const int n = __syncthreads_count(best >= mid);
+            if (n >= k)
+                lo = mid;
+            else
+                hi = mid;
+            if (n >= k && n <= k + kSlack) break;
+        }
+        thr = mm_filter_below(lo, mode);
+    }
+    const double sq = root_s[0], iq = root_s[1];
+    auto exact_key = [&](int j) {
+        return make_key(exact_score_recip(dots[j], sq, __ldg(rs + j), iq, __ldg(ri + j), mode), (uint32_t)j);
+    };
+    auto put = [&](int at, uint64_t key) {
+        const uint32_t j = key_idx(key);
+        out_s[q * k + at] = key_score(key);
+        out_i[q * k + at] = (int32_t)j;
+        if (out_d) out_d[q * k + at] = dots[j];
+        if (out_c) {  // exact_cos with the roots at hand
+            const double sr = __ldg(rs + j);
+            out_c[q * k + at] = sq == 0.0 || sr == 0.0 ? 0.0 : __ddiv_rn((double)dots[j], __dmul_rn(sq, sr));
+        }
+    };
+    for (int j = tid; j < nr; j += NT)
+        if (estimate(dots[j], __ldg(rr + j)) >= thr) keys[atomicAdd(&n_s, 1)] = (uint64_t)j;
+    __syncthreads();
+    const int n = n_s;  // at least k
+    if (n <= NT) {
+        const uint64_t mine = tid < n ? exact_key((int)keys[tid]) : 0;
+        __syncthreads();
+        if (tid < n) keys[tid] = mine;
+        __syncthreads();
+        if (tid < n) {
+            int at = 0;
+            for (int i = 0; i < n; ++i) at += keys[i] > mine;
+            if (at < k) put(at, mine);
+        }
+        return;
+    }
+    // more of them (scores tied by the hundred): the largest key below the last one, k times
+    for (int i = tid; i < n; i += NT) keys[i] = exact_key((int)keys[i]);
+    uint64_t last = ~0ull;
+    for (int at = 0; at < k; ++at) {
+        uint64_t top = 0;
+        for (int i = tid; i < n; i += NT) {  // (the keys that this thread wrote)
+            const uint64_t x = keys[i];
+            top = x < last && x > top ? x : top;
+        }
+        for (int o = 16; o; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        if (lane == 0) warp_best[at & 1][warp] = top;
+        __syncthreads();
+        for (int w = 0; w < NT / 32; ++w) top = max(top, warp_best[at & 1][w]);
+        last = top;
+        if (tid == 0) put(at, top);
+    }
+}
+
 // ---------------------------------------------------------------- merge
 constexpr int kMergeWarps = 4;
 constexpr int kMergeHeads = 5;  // lists a lane follows: 160 lists in all
@@ -926,6 +1239,13 @@ __global__ void pack_refs_kernel(const int16_t* __restrict__ r16, const __half* 
     }
 }
 
+__device__ __forceinline__ void norm_tables_one(int64_t v, int64_t i, float* rr, double* rs, double* ri) {
+    const double s = __dsqrt_rn((double)v);
+    rr[i] = rsqrt_norm(v);
+    rs[i] = s;
+    ri[i] = v ? __drcp_rn(s) : 0.0;
+}
+
 // Eight threads' sums of squares of 8 dims each, as the K block's (the lanes of `group` take part).
 template <typename T>
 __device__ __forceinline__ T kblock_norm(T s, uint32_t group) {
@@ -990,6 +1310,33 @@ __global__ void __launch_bounds__(kRowThreads) rows_f16_kernel(const int16_t* __
     block_norm_max(s, most, norms);
 }
 
+// The rows of both operands of a small problem in one launch: queries, then references with their norms' tables.
+template <bool VEC>
+__global__ void __launch_bounds__(kRowThreads) rows2_f16_kernel(const int16_t* __restrict__ q, int64_t nq,
+                                                                const int16_t* __restrict__ r, int dim, int64_t ld,
+                                                                __half* __restrict__ out_q, __half* __restrict__ out_r,
+                                                                const int64_t* __restrict__ rn, float* __restrict__ rr,
+                                                                double* __restrict__ rs, double* __restrict__ ri) {
+    const bool ref = (int64_t)blockIdx.x >= nq;
+    const int64_t row = ref ? (int64_t)blockIdx.x - nq : (int64_t)blockIdx.x;
+    const int16_t* v = (ref ? r : q) + row * dim;
+    __half* out = (ref ? out_r : out_q) + row * ld;
+    if (ref && threadIdx.x == 0) norm_tables_one(rn[row], row, rr, rs, ri);
+    for (int d0 = threadIdx.x * 8; d0 < ld; d0 += kRowThreads * 8) {
+        int16_t x[8];
+        if (VEC && d0 + 8 <= dim) {
+            *reinterpret_cast<uint4*>(x) = __ldg(reinterpret_cast<const uint4*>(v + d0));
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) x[u] = d0 + u < dim ? v[d0 + u] : (int16_t)0;
+        }
+        __half h[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) h[u] = __short2half_rn(x[u]);
+        *reinterpret_cast<uint4*>(out + d0) = *reinterpret_cast<const uint4*>(h);
+    }
+}
+
 // the largest squared norms of fp16 integer rows (dim % 8 == 0, 16-byte aligned)
 __global__ void __launch_bounds__(kRowThreads) norm_max_kernel(const __half* __restrict__ v, int dim, MmNorms other,
                                                                MmNorms* __restrict__ norms) {
@@ -1052,11 +1399,7 @@ __global__ void norm_tables_kernel(const int64_t* __restrict__ n2, int64_t n, fl
                                    double* __restrict__ rs, double* __restrict__ ri) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t v = n2[i];
-    const double s = __dsqrt_rn((double)v);
-    rr[i] = rsqrt_norm(v);
-    rs[i] = s;
-    ri[i] = v ? __drcp_rn(s) : 0.0;
+    norm_tables_one(n2[i], i, rr, rs, ri);
 }
 
 // ---------------------------------------------------------------- plan
@@ -1325,6 +1668,90 @@ int mm_norm_tables(const int64_t* d_n2, int64_t n, float* rr, double* rs, double
     return check_launch([&] {
         norm_tables_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(d_n2, n, rr, rs, ri);
     }, "mm search: norm tables");
+}
+
+MmSplit mm_split_plan(const hdc_context* ctx, int64_t nq, int64_t nr, int dim, int k, bool f4, int64_t sum_per_dim) {
+    MmSplit p;
+    const int n = f4 ? MmTile<true, 1>::N : MmTile<false, 1>::N, n_kb = n_kblocks(dim, f4);
+    const int64_t qt = (nq + kMmQueryTile - 1) / kMmQueryTile, rt = (nr + n - 1) / n;
+    if (k < 1 || k > kMaxKMm || nr > kSplitRefs || qt * rt > ctx->num_sms) return p;
+    if (sum_per_dim * (f4 ? kMmF4Dims : 64) > kMmMaxSum) return p;
+    p.n_qtiles = (int)qt;
+    p.n_rtiles = (int)rt;
+    p.splits = (int)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms / (qt * rt), n_kb / kMinSplitBlocks));
+    p.ldd = (int)rt * n;
+    return p;
+}
+
+size_t mm_split_bytes(const MmSplit& p, int64_t nq) { return (size_t)p.splits * nq * p.ldd * sizeof(int32_t); }
+
+template <bool F4>
+static int launch_dots(hdc_context* ctx, const MmOperands& op, const MmSplit& p, DotsArgs a, int64_t nr, int dim,
+                       cudaStream_t stream) {
+    using T = MmTile<F4, 1>;
+    CUtensorMap tmA, tmB;
+    const int64_t a_rows = F4 ? (int64_t)p.n_qtiles * a.n_kb * kMmQueryTile : a.nq;
+    const int64_t b_tiles = (nr + 2 * kMmF4Half - 1) / (2 * kMmF4Half);
+    const int64_t b_rows = F4 ? b_tiles * a.n_kb * 2 * a.limbs * kMmF4Half : nr;
+    if (!make_map(&tmA, F4, op.a, a_rows, dim, op.lda, kMmQueryTile) ||
+        !make_map(&tmB, F4, op.b, b_rows, dim, op.ldb, T::ROWS))
+        return fail(HDC_ERR_CUDA, "mm search: cuTensorMapEncodeTiled failed");
+    const int stage = mm_stage_bytes(T::A_BYTES, T::B_BYTES, a.limbs);
+    a.stages = (int)std::min<size_t>(kMaxStages, (kMaxDynSmemMm - 1024) / stage);
+    const cudaError_t e = cudaFuncSetAttribute(mm_dots_kernel<F4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kMaxDynSmemMm);
+    if (e != cudaSuccess) return cuda_fail(e, "mm search: cudaFuncSetAttribute");
+    return check_launch([&] {
+        mm_dots_kernel<F4><<<(unsigned)(p.n_qtiles * p.n_rtiles * p.splits), kDotThreads, 1024 + (size_t)a.stages * stage,
+                             stream>>>(tmA, tmB, a);
+    }, "mm search: split launch");
+}
+
+int mm_split_search(hdc_context* ctx, const MmOperands& op, const MmSplit& p, int64_t nq, int64_t nr, int dim, int k,
+                    int mode, void* parts, float* d_score, int32_t* d_idx, double* d_cos,
+                    int64_t* d_dot, int32_t shape[5], cudaStream_t stream) {
+    DotsArgs a{};
+    a.nq = nq;
+    a.n_kb = n_kblocks(dim, op.f4);
+    const int64_t most = std::max<int64_t>(1, kMmMaxSum / (op.sum_per_dim * (op.f4 ? kMmF4Dims : 64)));
+    a.kb_per_seg = (int)std::min<int64_t>(a.n_kb, most);
+    a.limbs = op.f4 ? op.limbs : 1;
+    a.n_rtiles = p.n_rtiles;
+    a.splits = p.splits;
+    a.ldd = p.ldd;
+    a.withhold = ctx->test_withhold_loads == 1;
+    a.parts = static_cast<int32_t*>(parts);
+    a.status = ctx->d_status;
+    a.wait_cycles = ctx->wait_cycles > 0 ? ctx->wait_cycles : tc::kWaitCycles;
+    const int st = op.f4 ? launch_dots<true>(ctx, op, p, a, nr, dim, stream) : launch_dots<false>(ctx, op, p, a, nr, dim, stream);
+    if (st != HDC_OK) return st;
+    if (shape) {
+        shape[0] = 1;
+        shape[1] = p.n_qtiles;
+        shape[2] = p.n_rtiles;
+        shape[3] = 0;
+    }
+    const size_t smem = (size_t)nr * (sizeof(uint64_t) + sizeof(int32_t));
+    auto kern = nr <= 512 ? mm_select_kernel<128> : mm_select_kernel<256>;  // four references a thread, if there are as many
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               kSplitRefs * (int)(sizeof(uint64_t) + sizeof(int32_t)));
+    if (e != cudaSuccess) return cuda_fail(e, "mm search: cudaFuncSetAttribute");
+    return check_launch([&] {
+        kern<<<(unsigned)nq, nr <= 512 ? 128 : 256, smem, stream>>>(a.parts, p.splits, nq, (int)nr, p.ldd, op.qn, op.rr, op.rs,
+                                                                   op.ri, k, mode, d_score, d_idx, d_cos, d_dot);
+    }, "mm search: select launch");
+}
+
+int mm_rows2_f16(const int16_t* d_q, int64_t nq, const int16_t* d_r, int64_t nr, int dim, int64_t ld, __half* out_q,
+                 __half* out_r, const int64_t* d_rn, float* rr, double* rs, double* ri, cudaStream_t stream) {
+    return check_launch([&] {
+        if (dim % 8 == 0 && aligned16(d_q) && aligned16(d_r))
+            rows2_f16_kernel<true><<<(unsigned)(nq + nr), kRowThreads, 0, stream>>>(d_q, nq, d_r, dim, ld, out_q, out_r, d_rn,
+                                                                                    rr, rs, ri);
+        else
+            rows2_f16_kernel<false><<<(unsigned)(nq + nr), kRowThreads, 0, stream>>>(d_q, nq, d_r, dim, ld, out_q, out_r,
+                                                                                     d_rn, rr, rs, ri);
+    }, "mm search: fp16 rows");
 }
 
 size_t mm_list_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int dim, int k, bool f4, int limbs) {

@@ -64,6 +64,20 @@ int mm_limbs_max(const __half* limbs16, int L16, int bits, int64_t rows, int dim
 // rr, rs, ri of MmOperands from squared norms
 int mm_norm_tables(const int64_t* d_n2, int64_t n, float* rr, double* rs, double* ri, cudaStream_t stream);
 
+// A problem of at most one tile a SM: the K loop of a tile split over CTAs, then a selection per query.  splits 0: not
+// one (too large, or products whose K block does not fit an accumulator).
+struct MmSplit {
+    int splits = 0, n_qtiles = 0, n_rtiles = 0, ldd = 0;
+};
+MmSplit mm_split_plan(const hdc_context* ctx, int64_t nq, int64_t nr, int dim, int k, bool f4, int64_t sum_per_dim);
+size_t mm_split_bytes(const MmSplit& p, int64_t nq);
+int mm_split_search(hdc_context* ctx, const MmOperands& op, const MmSplit& p, int64_t nq, int64_t nr, int dim, int k,
+                    int mode, void* parts, float* d_score, int32_t* d_idx, double* d_cos,
+                    int64_t* d_dot, int32_t shape[5], cudaStream_t stream);
+// mm_rows_f16 of both operands without their norms, and mm_norm_tables of the references
+int mm_rows2_f16(const int16_t* d_q, int64_t nq, const int16_t* d_r, int64_t nr, int dim, int64_t ld, __half* out_q,
+                 __half* out_r, const int64_t* d_rn, float* rr, double* rs, double* ri, cudaStream_t stream);
+
 // Workspace of a search's lists for nq queries against nr references (a launch of nr or fewer); its first
 // kMmWorkWords 64-bit words are the caller's.
 constexpr int kMmWorkWords = 4;

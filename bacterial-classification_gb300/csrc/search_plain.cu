@@ -492,11 +492,26 @@ static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, co
     return st;
 }
 
+// A small problem (mm_split_plan) on fp16 rows: both operands' rows, the references' norm tables, the parts.
+struct PlainSplit {
+    size_t r_at = 0, t_at = 0, p_at = 0, total = 0;
+};
+static PlainSplit plain_split_shape(const hdc_context* ctx, int64_t nq, int64_t nr, const MmSplit& p) {
+    PlainSplit s;
+    s.r_at = mm_round((size_t)nq * mm_ld(ctx->dim) * 2);
+    s.t_at = s.r_at + mm_round((size_t)nr * mm_ld(ctx->dim) * 2);
+    s.p_at = s.t_at + mm_round((size_t)nr * (2 * sizeof(double) + sizeof(float)));
+    s.total = s.p_at + mm_split_bytes(p, nq);
+    return s;
+}
+
 size_t plain_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k) {
     const int kk = std::max(1, (int)std::min<int64_t>(k, nr));
     const size_t cuda_cores = plain_min_workspace_bytes(ctx, nq, nr, k);
     if (kk > kMaxK || nr > 0x7fffffffLL) return cuda_cores;
-    return std::max(cuda_cores, std::max(plain_mm_shape(ctx, nq, nr, kk, false, 1).total(),
+    const MmSplit p = mm_split_plan(ctx, nq, nr, ctx->dim, kk, false, 1);
+    const size_t split = p.splits ? plain_split_shape(ctx, nq, nr, p).total : 0;
+    return std::max(std::max(cuda_cores, split), std::max(plain_mm_shape(ctx, nq, nr, kk, false, 1).total(),
                                          plain_mm_shape(ctx, nq, nr, kk, true, kMmPlainDigits).total()));
 }
 
@@ -541,6 +556,26 @@ int launch_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_q
     // A workspace below the tensor cores' share (plain_min_workspace_bytes is enough) takes the CUDA-core kernel.
     MmOperands op;
     if (plain_mm_form(ctx, maxq, maxr, op)) {
+        const bool aligned = d_work && (reinterpret_cast<uintptr_t>(d_work) & 255) == 0;
+        const MmSplit sp = op.f4 ? MmSplit() : mm_split_plan(ctx, nq, nr, ctx->dim, k, false, op.sum_per_dim);
+        const PlainSplit s = sp.splits ? plain_split_shape(ctx, nq, nr, sp) : PlainSplit();
+        if (aligned && sp.splits && work_bytes >= s.total) {
+            uint8_t* w = static_cast<uint8_t*>(d_work);
+            double* rs = reinterpret_cast<double*>(w + s.t_at);
+            float* rr = reinterpret_cast<float*>(rs + 2 * nr);
+            op.a = w;
+            op.b = w + s.r_at;
+            op.lda = op.ldb = mm_ld(ctx->dim);
+            op.qn = d_qn;
+            op.rr = rr;
+            op.rs = rs;
+            op.ri = rs + nr;
+            const int st = mm_rows2_f16(d_q, nq, d_r, nr, ctx->dim, op.lda, reinterpret_cast<__half*>(w),
+                                        reinterpret_cast<__half*>(w + s.r_at), d_rn, rr, rs, rs + nr, stream);
+            if (st != HDC_OK) return st;
+            return mm_split_search(ctx, op, sp, nq, nr, ctx->dim, k, mode, w + s.p_at, d_score, d_idx, d_cos, d_dot,
+                                   nullptr, stream);
+        }
         const PlainMm p = plain_mm_shape(ctx, nq, nr, k, op.f4, op.limbs);
         if (d_work && (reinterpret_cast<uintptr_t>(d_work) & 255) == 0 && work_bytes >= p.total())
             return launch_plain_mm(ctx, op, p, d_q, d_qn, nq, d_r, d_rn, nr, k, mode, d_score, d_idx, d_cos, d_dot, d_work,

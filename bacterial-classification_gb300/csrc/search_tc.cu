@@ -1124,6 +1124,11 @@ static size_t mm_workspace(const hdc_context* ctx, const hdc_refdb* db, int64_t 
            mm_list_bytes(ctx, nq, db->nr, db->dim, k, op.f4, op.limbs);
 }
 
+// And of a small problem's: the packed queries, then the parts of its dots.
+static size_t mm_split_workspace(const hdc_refdb* db, int64_t nq, const MmOperands& op, const MmSplit& p) {
+    return (op.f4 ? mm_f4_query_bytes(nq, db->dim) : 0) + mm_split_bytes(p, nq);
+}
+
 static size_t limb_workspace_bytes(const hdc_context* ctx, int64_t nq, const hdc_refdb* db, int k);
 
 size_t tc_workspace_bytes(const hdc_context* ctx, int64_t nq, const hdc_refdb* db, int k) {
@@ -1131,7 +1136,10 @@ size_t tc_workspace_bytes(const hdc_context* ctx, int64_t nq, const hdc_refdb* d
     size_t need = limb_workspace_bytes(ctx, nq, db, k);
     for (int32_t maxq = 1; maxq <= 2; ++maxq) {  // the two operand forms
         MmOperands op;
-        if (k <= kMaxKTC && mm_form(ctx, db, nq, maxq, op)) need = std::max(need, mm_workspace(ctx, db, nq, k, op));
+        if (k > kMaxKTC || !mm_form(ctx, db, nq, maxq, op)) continue;
+        need = std::max(need, mm_workspace(ctx, db, nq, k, op));
+        const MmSplit p = mm_split_plan(ctx, nq, db->nr, db->dim, k, op.f4, op.sum_per_dim);
+        if (p.splits) need = std::max(need, mm_split_workspace(db, nq, op, p));
     }
     return need;
 }
@@ -1359,7 +1367,24 @@ int launch_search_tc(hdc_context* ctx, const hdc_refdb* db, const __half* d_q, c
     }
     if ((reinterpret_cast<uintptr_t>(d_q) & 15) != 0) return fail(HDC_ERR_INVALID, "tc search: queries not 16B aligned");
     MmOperands op;
-    if (mm_form(ctx, db, nq, maxq, op) && d_work && aligned256(d_work) && work_bytes >= mm_workspace(ctx, db, nq, k, op)) {
+    const bool mm = mm_form(ctx, db, nq, maxq, op) && d_work && aligned256(d_work);
+    const MmSplit split = mm ? mm_split_plan(ctx, nq, db->nr, ctx->dim, k, op.f4, op.sum_per_dim) : MmSplit();
+    if (split.splits && work_bytes >= mm_split_workspace(db, nq, op, split)) {
+        op.a = d_q;
+        op.lda = ctx->dim;
+        op.qn = d_qn;
+        uint8_t* parts = static_cast<uint8_t*>(d_work);
+        if (op.f4) {
+            const int st = mm_pack_queries(d_q, true, nq, ctx->dim, d_work, stream);
+            if (st != HDC_OK) return st;
+            op.a = d_work;
+            parts += mm_f4_query_bytes(nq, ctx->dim);
+        }
+        ctx->tc_last_shape[4] = op.f4 ? 3 : 2;  // packing, dots, selection
+        return mm_split_search(ctx, op, split, nq, db->nr, ctx->dim, k, mode, parts, d_score, d_idx, d_cos,
+                               d_dot, ctx->tc_last_shape, stream);
+    }
+    if (mm && work_bytes >= mm_workspace(ctx, db, nq, k, op)) {
         void* lists = d_work;
         int st = HDC_OK;
         if (op.f4) {

@@ -44,6 +44,10 @@ def _values(g, n, dim, vmax, dtype=np.int16):
     (1024, 140, 300, 5, 0, 2048, 256),    # the largest product of those
     (1100, 300, 700, 5, 1, 2048, 257),    # one above: a segment an MMA
     (1000, 40, 300, 9, 0, 1023, 1025),    # the largest product accepted
+    (520, 7, 3000, 32, 0, 143, 250),      # a zero query: every score tied, more than are scored at once
+    (72, 140, 9700, 5, 1, 143, 250),      # a tile an SM
+    (70, 129, 20001, 12, 0, 143, 250),    # more tiles than SMs, ragged
+    (4100, 2, 12288, 3, 2, 60, 60),       # the most references of a selection, one K block past whole splits
     (1030, 300, 600, 7, 2, 300, 300),     # several K blocks a segment by their norms, where the products allow two
     (1024, 140, 300, 5, 0, 1, 12000),     # +1/0/-1 queries on digits
     (300, 129, 225, 10, 2, 1, 18724),     # five digits at their largest
