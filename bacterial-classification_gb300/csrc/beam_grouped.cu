@@ -619,7 +619,7 @@ __global__ void output_kernel(const GArgs a, int32_t* __restrict__ path, float* 
 // beam slot) whose beam row is node P are scored against P's children (a childless P
 // against itself) as one dense [entries] x [children] product.  A work item is up to 128
 // entries x 32 children of one parent.  Producer warps, in groups of four taking every G-th K
-// block (TcLayout: three groups, two in the one-launch kernel that streams its leaf level too), write the
+// block (TcLayout: two or three groups), write the
 // entries' +1/-1 signs (from the packed bits) as fp16 straight into TMEM with tcgen05.st (the
 // A operand: lane = entry, two signs a column), and the children's int32
 // prototype rows, split into three balanced base-2048 fp16 limbs, into 128-byte-swizzled
@@ -652,8 +652,8 @@ constexpr int kTcMaxStages = 6;
 // g, g + G, ...): warps 0 .. 4G-1 produce, 4G .. 4G+3 run the epilogue, lane 0 of warp 4G+4
 // issues the MMAs.  A warp's registers come from its SM sub-partition's quarter of the file,
 // so 17 warps (G = 3: five on one sub-partition) get 96 registers a thread, 13 warps (G = 2)
-// 128: only the one-launch kernel with the streamed leaf level in it, whose scoring needs the
-// registers, takes two.
+// 128: the one-launch kernel takes two with the streamed leaf level in it, whose scoring needs the
+// registers, and for small batches (one_wide).
 //
 // What bounds a level is the producers' sequence per K block, mostly half-rate integer
 // instructions (64 dims: two a sign column, three a value and limb pair).  The K order within 32
@@ -675,8 +675,6 @@ struct TcLayout {
     static_assert(kTcACol + 32 * kStages <= kTcTmemCols, "the A stages fit the TMEM allocation");
 };
 using TcLevel = TcLayout<3>;  // descent_tc_kernel: 544 threads
-template <bool LEAF>
-using TcOne = TcLayout<LEAF ? 2 : 3>;  // descent_one_kernel: 416 threads with the streamed leaf level in it
 
 struct TcItems {
     int32_t* ent_read;    // [entries] grouped by parent
@@ -1284,7 +1282,7 @@ constexpr int kCodeGridBarrier = 20;  // status 100 + this: a grid barrier gave 
 // Dynamic shared memory of the one-launch kernel: the tensor-core levels use the first TcLayout::kSmem
 // bytes; the streamed leaf level uses all of it (row slots + the consumers' bit buffers).
 constexpr size_t kOneSmem = 225 * 1024;
-static_assert(kOneSmem >= TcOne<true>::kSmem && kOneSmem >= TcOne<false>::kSmem, "the one-launch kernel also runs the tensor-core levels");
+static_assert(kOneSmem >= TcLayout<2>::kSmem && kOneSmem >= TcLayout<3>::kSmem, "the one-launch kernel also runs the tensor-core levels");
 constexpr int kMaxPhaseTs = 64;       // phase timestamps kept of a launch (hdc_beam_phase_times)
 
 struct OneArgs {
@@ -1770,11 +1768,12 @@ __global__ void __launch_bounds__(kScoreThreads, ROWS16 ? kScoreBlocks16 : kLeaf
     select_reads<16>(a, l.L, w, a.nq, nw, [&](int64_t r) { output_one(a, r, l.path, l.path_score, l.depth); });
 }
 
-// LEAF: the last level too (streamed); without it, the registers of that phase free, three producer groups fit.
-template <bool LEAF>
-__global__ void __launch_bounds__(TcOne<LEAF>::kThreads, 1)
+// LEAF: the last level too (streamed).  G: the tensor-core levels' producer groups (two with LEAF, whose scoring needs
+// the registers).
+template <bool LEAF, int G>
+__global__ void __launch_bounds__(TcLayout<G>::kThreads, 1)
     descent_one_kernel(const GArgs a, const TcItems t, const OneArgs o) {
-    using Lay = TcOne<LEAF>;
+    using Lay = TcLayout<G>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ TcShared sm;
     __shared__ int32_t sh[32];
@@ -1793,15 +1792,15 @@ __global__ void __launch_bounds__(TcOne<LEAF>::kThreads, 1)
         __syncthreads();
     }
     TcRun run;
-    const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    const int n_cta = gridDim.x, b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
     // this CTA's reads [r0, r1) and nodes [n0, n1)
-    const int64_t rc = (a.nq + G - 1) / G, r0 = min(a.nq, (int64_t)b * rc), r1 = min(a.nq, r0 + rc);
-    const int64_t ncn = (a.n_nodes + G - 1) / G, n0 = min(a.n_nodes, (int64_t)b * ncn), n1 = min(a.n_nodes, n0 + ncn);
+    const int64_t rc = (a.nq + n_cta - 1) / n_cta, r0 = min(a.nq, (int64_t)b * rc), r1 = min(a.nq, r0 + rc);
+    const int64_t ncn = (a.n_nodes + n_cta - 1) / n_cta, n0 = min(a.n_nodes, (int64_t)b * ncn), n1 = min(a.n_nodes, n0 + ncn);
     const bool last_reads = r0 < r1 && r1 == a.nq, last_nodes = n0 < n1 && n1 == a.n_nodes;
-    const int64_t gtid = (int64_t)b * nt + tid, gstride = (int64_t)G * nt;
+    const int64_t gtid = (int64_t)b * nt + tid, gstride = (int64_t)n_cta * nt;
     int32_t* blk0 = o.blk;
-    int32_t* blk1 = o.blk + G;
-    int32_t* blk2 = o.blk + 2 * G;
+    int32_t* blk1 = o.blk + n_cta;
+    int32_t* blk2 = o.blk + 2 * n_cta;
     const bool rows16 = a.n32 < a.n_nodes;
 
     for (int64_t r = r0 + tid; r < r1; r += nt) {
@@ -1915,7 +1914,7 @@ __global__ void __launch_bounds__(TcOne<LEAF>::kThreads, 1)
             __syncthreads();
         }
         // (16 lanes a read where the producer groups leave no registers for 8 keys a lane)
-        select_reads<LEAF ? kSelLanes : 16>(a, L, r0 + (tid >> 5), r1, nt >> 5, [](int64_t) {});
+        select_reads<G == 2 ? kSelLanes : 16>(a, L, r0 + (tid >> 5), r1, nt >> 5, [](int64_t) {});
         __syncthreads();
     }
     if (ok && !apart_done)
@@ -1935,10 +1934,15 @@ struct OneLaunch {
     const void* kernel;
     int threads;
 };
-OneLaunch one_launch(bool leaf) {
-    if (leaf) return {(const void*)descent_one_kernel<true>, TcOne<true>::kThreads};
-    return {(const void*)descent_one_kernel<false>, TcOne<false>::kThreads};
+OneLaunch one_launch(bool leaf, bool wide) {
+    if (leaf) return {(const void*)descent_one_kernel<true, 2>, TcLayout<2>::kThreads};
+    if (wide) return {(const void*)descent_one_kernel<false, 3>, TcLayout<3>::kThreads};
+    return {(const void*)descent_one_kernel<false, 2>, TcLayout<2>::kThreads};
 }
+// Three producer groups take 13 % off the tensor-core levels (20,000 reads, beam 5, D = 16,384: 2.06 -> 1.79 ms), but
+// their 96 registers a thread cost every other phase about half a microsecond (102 reads, beam 8, D = 1,024: 406 us a call
+// with two groups, 414 with three): the two meet near 0.2 ms of scoring.
+bool one_wide(int64_t nq, int beam, int dim) { return nq * beam * dim >= (int64_t)1 << 28; }
 
 // The one-launch descent needs every CTA (one per SM) resident at once; checked once per
 // context, with the kernel's shared memory set.
@@ -1947,12 +1951,12 @@ bool one_launch_fits(hdc_context* ctx) {
     if (ctx->beam_one_fit < 0) {
         int per_sm = 0;
         cudaError_t e = cudaSuccess;
-        for (const bool leaf : {false, true}) {
-            const OneLaunch l = one_launch(leaf);
+        for (int form = 0; form < 3; ++form) {
+            const OneLaunch l = one_launch(form == 0, form == 1);
             int n = 0;
             if (e == cudaSuccess) e = cudaFuncSetAttribute(l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOneSmem);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, l.kernel, l.threads, kOneSmem);
-            per_sm = leaf ? std::min(per_sm, n) : n;
+            per_sm = form ? std::min(per_sm, n) : n;
         }
         int coop = 0;
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
@@ -2110,7 +2114,7 @@ int launch_beam_grouped(hdc_context* ctx, const int8_t* d_q, const uint32_t* d_q
         o.wait_cycles = a.wait_cycles;
         o.late_cta = ctx->test_withhold_loads == 2 ? 1 : 0;
         const bool with_leaf = ctx->beam_one == 1;  // automatic: the last level in a launch of its own
-        const OneLaunch launch = one_launch(with_leaf);
+        const OneLaunch launch = one_launch(with_leaf, one_wide(nq, beam, ctx->dim));
         e = cudaMemsetAsync(one_state, 0, 4 * sizeof(uint32_t), stream);
         void* args[] = {(void*)&a, (void*)&t, (void*)&o};
         if (e == cudaSuccess)
