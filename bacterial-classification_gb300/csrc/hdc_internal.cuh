@@ -128,7 +128,7 @@ int tc_default_kblock();
 int tc_default_pair_mma();
 // Build the forms of the single-accumulator search from the limbs (synchronizes the stream); a form that does not fit
 // in memory is left out.
-int refdb_forms(hdc_refdb* db, cudaStream_t stream);
+int refdb_forms(const hdc_context* ctx, hdc_refdb* db, cudaStream_t stream);
 // Fill db->d_sqrt (allocated here) from db->d_norm2.
 int refdb_sqrt_table(hdc_refdb* db, cudaStream_t stream);
 int tc_default_tile_n();

@@ -863,7 +863,7 @@ int refdb_create(hdc_context* ctx, const void* d_ref, int elem_bytes, int64_t nr
         if (e != cudaSuccess) st = cuda_fail(e, "refdb: build");
     }
     cudaFree(d_lmax);
-    if (st == HDC_OK) st = refdb_forms(db, stream);
+    if (st == HDC_OK) st = refdb_forms(ctx, db, stream);
     if (st != HDC_OK) {
         refdb_destroy(db);
         return st;
@@ -883,10 +883,12 @@ void refdb_destroy(hdc_refdb* db) {
     delete db;
 }
 
-int refdb_forms(hdc_refdb* db, cudaStream_t stream) {
-    int64_t* d_max = nullptr;  // the largest value (int32) and the largest squared norm
-    cudaError_t e = cudaMalloc(&d_max, 2 * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, 2 * sizeof(int64_t), stream);
+int refdb_forms(const hdc_context* ctx, hdc_refdb* db, cudaStream_t stream) {
+    // the largest value (int32), the largest squared norm, then the fp16 rows' norms
+    constexpr size_t kMeasured = 2 * sizeof(int64_t) + 2 * sizeof(MmNorms);
+    int64_t* d_max = nullptr;
+    cudaError_t e = scratch_alloc(ctx, reinterpret_cast<void**>(&d_max), kMeasured, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, kMeasured, stream);
     int st = e == cudaSuccess ? mm_limbs_max(db->d_limbs, db->L, db->limb_bits, db->r_pad, db->dim,
                                              reinterpret_cast<int32_t*>(d_max), stream)
                               : cuda_fail(e, "refdb: allocation");
@@ -899,8 +901,10 @@ int refdb_forms(hdc_refdb* db, cudaStream_t stream) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) st = cuda_fail(e, "refdb: largest value");
     }
-    cudaFree(d_max);
-    if (st != HDC_OK) return st;
+    if (st != HDC_OK) {
+        if (d_max) cudaFreeAsync(d_max, stream);
+        return st;
+    }
     if (db->L == 1) db->d_rows16 = db->d_limbs;
     // base-2048 limbs are a database for +1/-1 queries, smaller bases one for counts
     if (db->limb_bits == 11) {
@@ -924,21 +928,18 @@ int refdb_forms(hdc_refdb* db, cudaStream_t stream) {
             db->d_rows16 = nullptr;
         }
     }
-    MmNorms* d_norms = nullptr;
     if (st == HDC_OK && db->d_rows16) {
-        e = cudaMalloc(&d_norms, 2 * sizeof(MmNorms));
-        if (e == cudaSuccess) e = cudaMemsetAsync(d_norms, 0, 2 * sizeof(MmNorms), stream);
-        st = e == cudaSuccess ? mm_norm_max(db->d_rows16, db->nr, db->dim, {}, d_norms, stream)
-                              : cuda_fail(e, "refdb: allocation");
+        MmNorms* d_norms = reinterpret_cast<MmNorms*>(d_max + 2);
+        st = mm_norm_max(db->d_rows16, db->nr, db->dim, {}, d_norms, stream);
         if (st == HDC_OK)
             e = cudaMemcpyAsync(&db->block2_max, &d_norms->block, sizeof(int64_t), cudaMemcpyDeviceToHost, stream);
         if (st == HDC_OK && e != cudaSuccess) st = cuda_fail(e, "refdb: largest norm of a K block");
     }
+    cudaFreeAsync(d_max, stream);
     if (st == HDC_OK) {
         e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) st = cuda_fail(e, "refdb: search forms");
     }
-    cudaFree(d_norms);
     return st;
 }
 
