@@ -282,7 +282,10 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
         if (e != cudaSuccess) return cuda_fail(e, "identify: shared memory attribute");
     }
     // Batches of reads grouped by parent on the tensor cores, each followed by the per-read kernel for what does not
-    // fit there (it exits at once otherwise).
+    // fit there (it exits at once otherwise).  A few reads with one beam row each, a CTA a read, wait as long for their
+    // own gathers as for the grouped form's five launches a level: 17 reads, D = 1,024, 233 us against 251; 30, D = 2,048,
+    // 291 against 299 (10 reads with three rows each: 865 against 293).
+    const bool few = nq <= ctx->num_sms && beam == 1 && ctx->dim <= 2048;
     for (int64_t r0 = 0; r0 < nq; r0 += kIdBatch) {
         const int64_t n = std::min(kIdBatch, nq - r0);
         IdentifyArgs a{d_q + r0 * ctx->dim, d_qn + r0, d_rows, d_rn, d_node_rows, d_child_ptr, d_child_idx, d_roots, n_roots,
@@ -290,7 +293,7 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
                        d_depth + r0, d_stop_level ? d_stop_level + r0 : nullptr, nullptr};
         int32_t* flag = nullptr;
         void* ws = nullptr;
-        int st = launch_identify_grouped(ctx, a, n, &flag, &ws, stream);
+        const int st = few ? HDC_OK : launch_identify_grouped(ctx, a, n, &flag, &ws, stream);
         if (st != HDC_OK) return st;
         a.only_if = flag;
         identify_kernel<<<(unsigned)n, 32 * kIdWarps, smem, stream>>>(a);
