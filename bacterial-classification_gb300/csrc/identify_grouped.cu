@@ -4,7 +4,7 @@
 // from L2 (315 GB for 4,096 reads over a 2,000-leaf tree, 38 ms).  Here a level is scored for the whole batch: the
 // entries (read, beam row) that stand at the same parent share one dense product
 //     [up to 128 reads] x [up to 192 similarity rows of the parent's children],
-// so a row leaves DRAM about once a level and the dots run on tcgen05 (the same batch: 2.08 ms, of which the leaf level's
+// so a row leaves DRAM about once a level and the dots run on tcgen05 (the same batch: 1.98 ms, of which the leaf level's
 // 4.4 GB of rows take 1.0).
 //
 // A level is five kernels: entries are put into a hash table by parent (the call does not know the number of nodes),

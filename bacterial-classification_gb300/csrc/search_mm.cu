@@ -29,7 +29,10 @@
 // Pairs (CL = 2): one cta_group::2 MMA over two query tiles, each CTA staging half of the reference tile's rows.
 // Single CTAs (CL = 1) with narrow reference tiles serve batches too small to give every pair a tile.
 //
-// What bounds it: the tensor pipe for large batches; the reference bytes for a few queries.
+// Problems of at most a tile a SM go to mm_dots_kernel and mm_select_kernel below.
+//
+// What bounds it: the tensor pipe for large batches (10,000 x 50,000 count-valued reads, D = 8,192: 514 cycles a K block of
+// 512); the reference bytes for a few queries.
 #include <cuda.h>
 #include <cuda_fp16.h>
 

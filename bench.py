@@ -75,13 +75,24 @@ CONFIGS = {
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of the
-# dominant kernel, from single-pass ncu captures of the full-size workloads, per
-# unit of work, so a run's `traffic` is that per-unit figure times its own units:
-#   tc_search_kernel, c3 (38,912 reads x 200,000 refs = 304 x 1,564 tile pairs; the
-#     288 leading query tiles in clusters of 4 + the other 16 in pairs): 1.01427e12 B
+# dominant kernel, from single-pass ncu captures of the full-size workloads, reported
+# for calls of the captured size:
+#   mm_search_kernel, c3 (38,912 reads x 200,000 refs, four digits): 1.1690e11 B
 #   grouped descent, c5 (one call's 5 descent_tc_kernel launches + the leaf-level score_kernel,
 #     38,912 reads): 3.64798e10 B with every row int32, 2.03567e10 B with int16 leaf rows
-TRAFFIC_PER_TILE_PAIR_TC = (975.445256e9 + 0.170780e9 + 38.640838e9 + 0.012020e9) / (304 * 1564)
+TRAFFIC_SEARCH = {(38912, 200000): 116.88e9 + 22.80e6}  # (reads, references) -> bytes
+# block-scaled e2m1 MMAs (256 x 224 x 64, CTA pairs) on resident operands: the rate of the digits' search
+FP4_TFLOPS = 9160.0
+
+
+def base8_digits(max_abs):
+    """Balanced base-8 digits (-4 .. 4) that hold |v| <= max_abs."""
+    n, cover = 1, 4
+    while max_abs > cover:
+        n, cover = n + 1, cover * 8 + 4
+    return n
+
+
 # (reads per call, int16 rows) -> bytes (mostly the database, once)
 TRAFFIC_DESCENT = {(38912, False): 36.409726e9 + 70.093e6, (38912, True): 2.035667e10}
 
@@ -214,10 +225,11 @@ class Form:
     """One GPU form of the hot path for a fixed batch size: encode the batch of
     reads, then top-k search against the resident database.
       plain: int16 queries (counts, or +1/-1 when the workload is bipolar),
-             exact search on CUDA cores (hdc_search_plain)
+             exact search (hdc_search_plain: rows converted and searched on the tensor
+             cores where the values allow it, else on CUDA cores)
       tc:    fp16 queries (+1/-1, or counts when the workload is not bipolar), exact
-             search on tcgen05 tensor cores (hdc_search_tc against an fp16-limb
-             database whose limbs are sized for the largest query magnitude)"""
+             search on tcgen05 tensor cores (hdc_search_tc against a database of base-8
+             digits or fp16 rows, with fp16 limbs behind them for other schedules)"""
 
     def __init__(self, H, ctx, cfg, name, refs, rn, maxr, B, dev, db=None):
         import torch
@@ -249,7 +261,8 @@ class Form:
                     torch.empty((B, K), dtype=torch.int32, device=dev),
                     torch.empty((B, K), dtype=torch.float64, device=dev),
                     torch.empty((B, K), dtype=torch.int64, device=dev))
-        self.launches = 3 if cfg["bipolar"] else 4  # encode, [norms], search, merge
+        # encode, [norms], then (plain, one chunk of references) two conversions, norm tables, search, merge
+        self.launches = 6 if cfg["bipolar"] else 7
         # the reference's NORM scale by default; --score-mode dot/cos for kernel studies
         self.mode = {"norm": H.SCORE_NORM, "cos": H.SCORE_COS, "dot": H.SCORE_DOT}[cfg.get("score_mode", "norm")]
 
@@ -260,7 +273,7 @@ class Form:
         if ev is not None:
             ev[0].record(stream)
         if self.name == "tc":
-            ctx.search_tc(self.db, self.q, qn, 1, self.K, self.mode, work=self.work, out=self.out)
+            ctx.search_tc(self.db, self.q, qn, self.maxq, self.K, self.mode, work=self.work, out=self.out)
             # encode, [norms], then the search kernels and merges the library reports (one or two parts)
             self.launches = (1 if self.cfg["bipolar"] else 2) + ctx.tc_last_shape()[4]
         else:
@@ -351,7 +364,7 @@ def run_pipeline(args, cfg, H, ctx, tree, refs, rn, maxr, dev, db=None):
     bat = [(torch.from_numpy(pool[0].off).to(dev), torch.from_numpy(pool[0].len).to(dev))]
     _, search_ms = time_form(form, bat, d_buf, 2, 3)
     return dict(ms=ms, e2e_ms=e2e_ms, search_ms=search_ms, clocks=clk.summary(), launches=per_step * args.steps,
-                refs=refs.shape[0], limbs=db.limbs, h2d=max_bytes + B * 16, d2h=B * K * 8, tree=tree,
+                refs=refs.shape[0], limbs=db.limbs, maxr=maxr, h2d=max_bytes + B * 16, d2h=B * K * 8, tree=tree,
                 tuned=tuned, mean_len=float(np.mean(pool[0].len)), top1_accuracy=acc,
                 refs_host=refs.cpu().numpy() if not args.no_cpu_baseline else None, reads=pool[0],
                 gpu_first=(first_s[:1024], first_idx[:1024], None, None))
@@ -382,7 +395,7 @@ def run_ours(args, cfg):
     clk = ClockSampler(dev.index)
     ms, search_ms = time_form(form, batches, d_buf, args.steps, args.warmup, clk)
     res = dict(ms=ms, search_ms=search_ms, clocks=clk.summary(), launches=form.launches * args.steps,
-               refs=refs.shape[0], limbs=form.db.limbs if form.db is not None else 0)
+               refs=refs.shape[0], limbs=form.db.limbs if form.db is not None else 0, maxr=maxr)
     # the source leaf of every read is known: how often is it the top hit
     form.run(d_buf, *batches[0])
     torch.cuda.synchronize()
@@ -879,7 +892,8 @@ def batching_line(args, b, refs_host, pk):
     the oracle's parity sample on the first reads of its batch."""
     cfg = b["cfg"]
     B = args.batch
-    flops = 2.0 * cfg["dim"] * b["refs"] * b["limbs"] * B
+    digits = base8_digits(b["maxr"])
+    flops = 2.0 * cfg["dim"] * b["refs"] * digits * B
     achieved = flops / (b["search_ms"] / 1e3) / 1e12
     out = {"workload": "c4 reads on this database: log-normal lengths (median %d bp, sigma %.1f, %d-%d bp), %d%% "
                        "with %d%% sub:ins:del 3:1:1, top-%d, CUDA-graph encode -> search -> top-k" % (
@@ -888,8 +902,8 @@ def batching_line(args, b, refs_host, pk):
            "value": B / (b["ms"] / 1e3), "unit": "reads/s", "batch_reads": B, "ms_per_step": b["ms"],
            "e2e": {"value": B / (b["e2e_ms"] / 1e3), "unit": "reads/s", "h2d_bytes_per_step": b["h2d"],
                    "d2h_bytes_per_step": b["d2h"]},
-           "search_roofline": {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"],
-                               "unit": "TFLOP/s", "frac": achieved / pk["bf16_tflops"]},
+           "search_roofline": {"bound": "tensor", "achieved": achieved, "peak": FP4_TFLOPS, "unit": "TFLOP/s",
+                               "frac": achieved / FP4_TFLOPS, "digits": digits},
            "autotuned_schedule": b["tuned"], "mean_read_len": b["mean_len"], "top1_accuracy": b["top1_accuracy"],
            "gpu_launches": b["launches"], "clocks": b["clocks"]}
     if refs_host is not None:
@@ -1311,36 +1325,36 @@ def main():
     value = B / (r["ms"] / 1e3)
     dim, nr = cfg["dim"], r["refs"]
     if args.form in ("tc", "pipe"):
-        # tensor work per read: one fp16 MMA pass per limb, 2*D*R*limbs flops
-        flops = 2.0 * dim * nr * r["limbs"] * B
+        # tensor work per read: 2*D*R, times the digits for +1/-1 reads (one e2m1 MMA step each)
+        digits = base8_digits(r["maxr"]) if cfg["bipolar"] else 0
+        flops = 2.0 * dim * nr * max(1, digits) * B
         achieved = flops / (r["search_ms"] / 1e3) / 1e12
-        tile_pairs = ((B + 127) // 128) * (((nr + 255) // 256) * 2)
-        roof = {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
-                "frac": achieved / pk["bf16_tflops"], "traffic": TRAFFIC_PER_TILE_PAIR_TC * tile_pairs,
-                "traffic_source": "ncu DRAM bytes of the two search launches of a full-size c3 call, per "
-                                  "128x128 tile pair, times this call's %d pairs (query tiles re-read for every "
-                                  "reference tile, half of them through L2)" % tile_pairs,
-                "peak_source": "%s dense bf16/fp16 burst (MEASURED_PEAKS.json)" % src,
-                "kernel": "tc_search_kernel (clusters of 4 + pair remainder) + merge, %d fp16 limbs; "
-                          "algorithmic 2*D*R*limbs per read" % r["limbs"]}
-        dtype = "fp16 integer limbs, fp32 accumulators (exact int64 dots), FP64 scores"
+        peak = FP4_TFLOPS if digits else pk["bf16_tflops"]
+        roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                "frac": achieved / peak, "traffic": TRAFFIC_SEARCH.get((B, nr)),
+                "traffic_source": "ncu DRAM bytes of the search kernel of one call of this size",
+                "algorithmic_tflops": 2.0 * dim * nr * B / (r["search_ms"] / 1e3) / 1e12,
+                "peak_source": "block-scaled e2m1 MMAs on resident operands, measured" if digits else
+                               "%s dense bf16/fp16 burst (MEASURED_PEAKS.json)" % src,
+                "kernel": "mm_search_kernel + packing + merge; algorithmic 2*D*R per read" +
+                          (" for each of %d base-8 digits" % digits if digits else " on fp16 rows")}
+        dtype = ("e2m1 digits, block-scaled" if digits else "fp16 integers") + \
+            ", fp32 accumulators (exact integer dots), FP64 scores"
     else:
         flops = 2.0 * dim * nr * B
         achieved = flops / (r["search_ms"] / 1e3) / 1e12
-        sm_mhz = r["clocks"].get("sm_mhz") or pk.get("sm_max_mhz", 2070.0)
-        fp32_peak = 152 * 128 * 2 * sm_mhz * 1e6 / 1e12
-        roof = {"bound": "fp32-pipe", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
-                "frac": achieved / fp32_peak, "traffic": None,
-                "peak_source": "152 SMs x 128 FFMA x 2 x median SM clock",
-                "kernel": "plain_kernel + merge on CUDA cores; algorithmic 2*D*R per read"}
-        dtype = "int16 (exact integer dots on the fp32 pipe), FP64 scores"
+        roof = {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
+                "frac": achieved / pk["bf16_tflops"], "traffic": None,
+                "peak_source": "%s dense bf16/fp16 burst (MEASURED_PEAKS.json)" % src,
+                "kernel": "conversion of both operands + mm_search_kernel + merge; algorithmic 2*D*R per read"}
+        dtype = "int16 rows as fp16 integers, fp32 accumulators (exact integer dots), FP64 scores"
     line = {
         "metric": metric, "value": value, "unit": "reads/s", "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": r["ms"], "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": dtype, "data": "synthetic (seeded 6-rank tree, see bench.py)",
         "config": {"workload": workload, "form": args.form, "batch_reads": B,
                    "l2": "inputs larger than L2: %.0f MB reference database streamed every step" %
-                         (nr * dim * 2 * max(1, r["limbs"]) / 1e6)},
+                         (nr * dim * (base8_digits(r["maxr"]) / 2 if args.form != "plain" and cfg["bipolar"] else 2) / 1e6)},
         "e2e": {"value": B / (r["e2e_ms"] / 1e3), "unit": "reads/s", "h2d_bytes_per_step": r["h2d"],
                 "d2h_bytes_per_step": r["d2h"]},
         "roofline": roof, "clocks": r["clocks"], "gpu_launches": r["launches"],
