@@ -292,6 +292,12 @@ int hdc_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnor
                                     static_cast<cudaStream_t>(stream));
 }
 
+int hdc_search_plain_last_form(const hdc_context* ctx, int32_t form[2]) {
+    if (!ctx || !form) return fail(HDC_ERR_INVALID, "search form: null argument");
+    for (int i = 0; i < 2; ++i) form[i] = ctx->plain_last_form[i];
+    return HDC_OK;
+}
+
 int hdc_context_status(hdc_context* ctx, int* status) {
     if (!ctx || !status) return fail(HDC_ERR_INVALID, "status: null argument");
     cudaError_t e = cudaMemcpy(status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost);

@@ -443,6 +443,11 @@ static bool plain_mm_form(const hdc_context* ctx, int32_t maxq, int32_t maxr, Mm
     return mm_sums_fit(op.f4, op.sum_per_dim) && op.sum_per_dim * ctx->dim <= 0x7fffffff;
 }
 
+static void plain_ran(hdc_context* ctx, int form, int kernels) {
+    ctx->plain_last_form[0] = form;
+    ctx->plain_last_form[1] = kernels;
+}
+
 static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, const int16_t* d_q, const int64_t* d_qn,
                            int64_t nq, const int16_t* d_r, const int64_t* d_rn, int64_t nr, int k, int mode, float* d_score,
                            int32_t* d_idx, double* d_cos, int64_t* d_dot, void* d_work, cudaStream_t stream) {
@@ -467,6 +472,7 @@ static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, co
     }
     const cudaError_t e = cudaMemsetAsync(r_norms, 0, sizeof(MmNorms), stream);
     int st = e == cudaSuccess ? HDC_OK : cuda_fail(e, "search: clear the largest norm");
+    int kernels = 0;
     for (int64_t q0 = 0; q0 < nq && st == HDC_OK; q0 += p.nqc) {
         const int64_t n = std::min(p.nqc, nq - q0);
         op.qn = d_qn + q0;
@@ -481,14 +487,18 @@ static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, co
                 st = op.f4 ? mm_pack_refs(d_r + r0 * dim, nullptr, 1, 0, 0, m, dim, op.limbs, wr, stream)
                            : mm_rows_f16(d_r + r0 * dim, m, dim, op.ldb, reinterpret_cast<__half*>(wr), r_norms, stream);
                 if (st == HDC_OK) st = mm_norm_tables(d_rn + r0, m, rr, rs, ri, stream);
+                kernels += 2;
             }
             if (st == HDC_OK)
                 st = mm_search(ctx, op, n, m, r0, p.nrc, dim, k, mode, lists, r0 == 0, nullptr, stream);
+            ++kernels;
         }
         if (st == HDC_OK)
             st = mm_finish(ctx, n, p.nrc, nr, dim, k, op.f4, op.limbs, d_qn + q0, d_rn, lists, d_score + q0 * k,
                            d_idx + q0 * k, d_cos ? d_cos + q0 * k : nullptr, d_dot ? d_dot + q0 * k : nullptr, stream);
+        kernels += 2;  // the queries' conversion, the merge
     }
+    plain_ran(ctx, op.f4 ? HDC_PLAIN_DIGITS : HDC_PLAIN_F16, kernels);
     return st;
 }
 
@@ -573,11 +583,12 @@ int launch_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_q
             const int st = mm_rows2_f16(d_q, nq, d_r, nr, ctx->dim, op.lda, reinterpret_cast<__half*>(w),
                                         reinterpret_cast<__half*>(w + s.r_at), d_rn, rr, rs, rs + nr, stream);
             if (st != HDC_OK) return st;
+            plain_ran(ctx, HDC_PLAIN_SPLIT, 3);
             return mm_split_search(ctx, op, sp, nq, nr, ctx->dim, k, mode, w + s.p_at, d_score, d_idx, d_cos, d_dot,
                                    nullptr, stream);
         }
         const PlainMm p = plain_mm_shape(ctx, nq, nr, k, op.f4, op.limbs);
-        if (d_work && (reinterpret_cast<uintptr_t>(d_work) & 255) == 0 && work_bytes >= p.total())
+        if (aligned && work_bytes >= p.total())
             return launch_plain_mm(ctx, op, p, d_q, d_qn, nq, d_r, d_rn, nr, k, mode, d_score, d_idx, d_cos, d_dot, d_work,
                                    stream);
     }
@@ -612,6 +623,7 @@ int launch_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_q
         st = tq == 4 ? (vec ? launch_plain_t<4, false, true>(a, nq, stream) : launch_plain_t<4, false, false>(a, nq, stream))
                      : (vec ? launch_plain_t<8, false, true>(a, nq, stream) : launch_plain_t<8, false, false>(a, nq, stream));
     if (st != HDC_OK) return st;
+    plain_ran(ctx, HDC_PLAIN_CUDA_CORES, 2);
     return launch_merge(a.ws_key, a.ws_dot, a.n_splits, nq, k, d_qn, d_rn, nr, d_score, d_idx, d_cos, d_dot, stream);
 }
 

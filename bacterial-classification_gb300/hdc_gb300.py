@@ -18,6 +18,7 @@ SCORE_NORM, SCORE_COS, SCORE_DOT = 0, 1, 2
 TC_PREFETCH, TC_CLUSTER, TC_SHARE, BEAM_GROUPED, TC_SCATTER, TC_KBLOCK, TC_PAIR_MMA, TC_LANES = 1, 2, 3, 4, 5, 6, 7, 8
 OUT_I16, OUT_I32, OUT_BIPOLAR_BF16, OUT_BIPOLAR_I16, OUT_BIPOLAR_F16, OUT_BIPOLAR_I8, OUT_F16 = 0, 1, 2, 3, 4, 5, 6
 WAIT_LIMIT, TEST_WITHHOLD_LOADS, BEAM_ONE_LAUNCH, GREEDY_FORM = 9, 10, 11, 12
+PLAIN_CUDA_CORES, PLAIN_SPLIT, PLAIN_F16, PLAIN_DIGITS = 0, 1, 2, 3  # how a plain search ran
 OUT_SIGN_BITS = 7  # sign bits, int32 [n][dim / 32] (bit b of word w: element 32 w + b >= 0)
 
 # (name, restype, argtypes) of every exported entry point
@@ -43,6 +44,7 @@ SIGNATURES = [
     ("hdc_search_workspace_bytes", SZ, [P, I64, I64, I32]),
     ("hdc_search_plain", I32, [P, P, P, I64, ctypes.c_int32, P, P, I64, ctypes.c_int32, I32, I32, P, P, P, P, P,
                                SZ, P]),
+    ("hdc_search_plain_last_form", I32, [P, P]),
     ("hdc_bundle", I32, [P, P, I32, P, P, I64, P, P]),
     ("hdc_beam_search", I32, [P, P, P, I64, P, P, I64, P, P, P, I32, I32, I32, ctypes.c_double, I32, P, P, P, P]),
     ("hdc_beam_search_split", I32, [P, P, P, I64, P, I64, P, P, I64, P, P, P, I32, I32, I32, I32, ctypes.c_double,
@@ -213,6 +215,12 @@ class Context:
         check(lib().hdc_search_plain(self.h, ptr(q), ptr(qn), nq, int(maxq), ptr(r), ptr(rn), nr, int(maxr), k, mode,
                                      ptr(s), ptr(i), ptr(c), ptr(d), ptr(work), work.numel(), stream_ptr(stream)))
         return out
+
+    def plain_last_form(self):
+        """(PLAIN_*, kernels launched) of the last plain search."""
+        out = (ctypes.c_int32 * 2)()
+        check(lib().hdc_search_plain_last_form(self.h, ctypes.addressof(out)))
+        return tuple(out)
 
     def status(self):
         st = ctypes.c_int(0)

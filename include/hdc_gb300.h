@@ -180,6 +180,15 @@ int hdc_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnor
                      int32_t max_abs_r, int k, int score_mode, float* d_score, int32_t* d_idx,
                      double* d_cos, int64_t* d_dot, void* d_work, size_t work_bytes, void* stream);
 
+/* How the last hdc_search_plain (or hdc_search_plain_noalloc) on this context
+ * ran (diagnostic): form[0] = one of HDC_PLAIN_*, -1 before the first, form[1] =
+ * the kernels that it launched. */
+#define HDC_PLAIN_CUDA_CORES 0
+#define HDC_PLAIN_SPLIT 1  /* tensor cores, at most a tile an SM: fp16 rows, the K loop split over CTAs */
+#define HDC_PLAIN_F16 2    /* tensor cores: fp16 rows */
+#define HDC_PLAIN_DIGITS 3 /* tensor cores: +1/0/-1 queries against base-8 digits */
+int hdc_search_plain_last_form(const hdc_context* ctx, int32_t form[2]);
+
 /* Read and clear the device status word of the context (synchronizes the
  * device): 0, 100 + the code of a bounded device-side wait that gave up in
  * a tensor-core search or descent (which then returned partial results), or
