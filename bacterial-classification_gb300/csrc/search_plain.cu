@@ -401,6 +401,7 @@ int launch_norms(hdc_context* ctx, const void* d_hv, int elem_bytes, int64_t n, 
 // queries in batches of as much, so the workspace stays bounded.
 constexpr size_t kMmChunkBytes = (size_t)1 << 30;
 constexpr int kMmPlainDigits = 5;  // the most digits of a reference here: 2.5 bytes a value
+constexpr int32_t kMmPlainRows16 = 2048;  // the largest value of an fp16 row
 
 static size_t mm_round(size_t x) { return (x + 255) / 256 * 256; }
 static int64_t mm_ld(int dim) { return ((int64_t)dim + 63) / 64 * 64; }
@@ -431,11 +432,11 @@ static PlainMm plain_mm_shape(const hdc_context* ctx, int64_t nq, int64_t nr, in
 // The operand form for |q| <= maxq and |r| <= maxr, or false: the CUDA-core kernel.
 static bool plain_mm_form(const hdc_context* ctx, int32_t maxq, int32_t maxr, MmOperands& op) {
     const int digits = mm_f4_limbs(maxr);
-    if (maxq <= 1 && maxr > 2048 && digits) {
+    if (maxq <= 1 && maxr > kMmPlainRows16 && digits) {
         op.f4 = true;
         op.limbs = digits;
         op.sum_per_dim = mm_f4_sum_per_dim(maxr);
-    } else if (maxq <= 2048 && maxr <= 2048) {
+    } else if (maxq <= kMmPlainRows16 && maxr <= kMmPlainRows16) {
         op.sum_per_dim = (int64_t)std::max(maxq, 1) * std::max(maxr, 1);
     } else {
         return false;
@@ -520,9 +521,12 @@ size_t plain_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int
     const size_t cuda_cores = plain_min_workspace_bytes(ctx, nq, nr, k);
     if (kk > kMaxK || nr > 0x7fffffffLL) return cuda_cores;
     const MmSplit p = mm_split_plan(ctx, nq, nr, ctx->dim, kk, false, 1);
-    const size_t split = p.splits ? plain_split_shape(ctx, nq, nr, p).total : 0;
-    return std::max(std::max(cuda_cores, split), std::max(plain_mm_shape(ctx, nq, nr, kk, false, 1).total(),
-                                         plain_mm_shape(ctx, nq, nr, kk, true, kMmPlainDigits).total()));
+    size_t need = std::max(cuda_cores, p.splits ? plain_split_shape(ctx, nq, nr, p).total : 0);
+    need = std::max(need, plain_mm_shape(ctx, nq, nr, kk, false, 1).total());
+    // every number of digits: with fewer, a chunk holds more rows, whose norm tables may come to more bytes
+    for (int digits = mm_f4_limbs(kMmPlainRows16 + 1); digits <= kMmPlainDigits; ++digits)
+        need = std::max(need, plain_mm_shape(ctx, nq, nr, kk, true, digits).total());
+    return need;
 }
 
 size_t plain_min_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k) {

@@ -63,3 +63,20 @@ def test_plain_form_and_results(hdc, cuda, dim, nq, nr, k, maxq, maxr, work, off
     assert ctx.plain_last_form()[0] == CUDA
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dim,nq,nr,k,maxr,form", [
+    (10240, 8, 100000, 5, 2340, DIGITS),   # four digits, more references than a chunk of either form holds
+    (10240, 8, 100000, 5, 2341, DIGITS),   # five
+    (10240, 8, 100000, 5, 2048, F16),
+    (10240, 300, 70000, 32, 2340, DIGITS),
+])
+def test_the_workspace_asked_for_holds_every_form(hdc, cuda, dim, nq, nr, k, maxr, form):
+    """hdc_search_workspace_bytes does not know the values; with all of it a search runs on the tensor cores."""
+    import torch
+    ctx = hdc.Context(dim, 8, 150, 10)
+    r = torch.zeros((nr, dim), dtype=torch.int16, device=cuda)
+    r[::7, ::3] = maxr
+    q = torch.ones((nq, dim), dtype=torch.int16, device=cuda)
+    _search(hdc, ctx, q, 1, r, maxr, k)
+    assert ctx.plain_last_form()[0] == form and ctx.status() == 0
