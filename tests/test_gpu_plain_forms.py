@@ -21,9 +21,10 @@ def _search(hdc, ctx, q, maxq, r, maxr, k, mode=0, work_bytes=None, offset=0):
            (torch.float32, torch.int32, torch.float64, torch.int64)]
     n = ctx.workspace_bytes(nq, r.shape[0], k) if work_bytes is None else work_bytes
     work = torch.empty(n + offset, dtype=torch.uint8, device=q.device)[offset:]
+    qn, rn = ctx.norms(q), ctx.norms(r)
     p = hdc.ptr
-    hdc.check(hdc.lib().hdc_search_plain(ctx.h, p(q), p(ctx.norms(q)), nq, maxq, p(r), p(ctx.norms(r)), r.shape[0], maxr, k,
-                                         mode, *(p(x) for x in out), p(work), n, hdc.stream_ptr()))
+    hdc.check(hdc.lib().hdc_search_plain(ctx.h, p(q), p(qn), nq, maxq, p(r), p(rn), r.shape[0], maxr, k, mode,
+                                         *(p(x) for x in out), p(work), n, hdc.stream_ptr()))
     torch.cuda.synchronize()
     return out
 
@@ -80,3 +81,51 @@ def test_the_workspace_asked_for_holds_every_form(hdc, cuda, dim, nq, nr, k, max
     q = torch.ones((nq, dim), dtype=torch.int16, device=cuda)
     _search(hdc, ctx, q, 1, r, maxr, k)
     assert ctx.plain_last_form()[0] == form and ctx.status() == 0
+
+
+def _same_as_cuda_cores(hdc, ctx, got, q, maxq, r, maxr, k, rows):
+    """The results of the given query rows against those of a search of these rows alone on CUDA cores."""
+    import torch
+    want = _search(hdc, ctx, q[rows].contiguous(), maxq, r, maxr, k, 0, None, 16)
+    assert ctx.plain_last_form()[0] == CUDA
+    for a, b in zip(got, want):
+        assert torch.equal(a[rows], b)
+
+
+def test_plain_digits_go_on_from_chunk_to_chunk(hdc, cuda):
+    """+1/0/-1 queries against more references than one chunk of digits holds (1 GiB: 65,536 rows of 8,192 in four digits
+    and 52,416 in five): answers on both sides of the border, ties across it to the lower index."""
+    import torch
+    dim, nq, nr, k = 8192, 140, 70000, 9
+    q = _rows(torch, cuda, 3, nq, dim, 1)
+    for maxr, border in ((2340, 65536 // 224 * 224), (2341, 52416)):
+        r = _rows(torch, cuda, maxr, nr, dim, maxr)
+        r[border - 3:border + 3] = q[:6] * 100
+        r[border + 20] = r[border - 2]
+        r[nr - 1] = r[5]
+        ctx = hdc.Context(dim, 8, 150, 10)
+        got = _search(hdc, ctx, q, 1, r, maxr, k)
+        form, kernels = ctx.plain_last_form()
+        assert form == DIGITS and kernels == 8 and ctx.status() == 0  # two chunks
+        _same_as_cuda_cores(hdc, ctx, got, q, 1, r, maxr, k, torch.arange(nq, device=cuda))
+
+
+@pytest.mark.parametrize("maxq,maxr,nr,kernels", [
+    (60, 90, 300, 8),        # fp16 rows: two batches of queries, one chunk of references
+    (60, 90, 33000, 16),     # and two chunks, converted again for the second batch
+    (1, 2340, 400, 8),       # digits
+])
+def test_plain_query_batches(hdc, cuda, maxq, maxr, nr, kernels):
+    """More converted queries than a batch holds (1 GiB: 32,768 rows of 16,384 in fp16, 131,072 in e2m1), with a short last
+    batch of another plan: rows on both sides of the border and at the ends."""
+    import torch
+    dim, k = 16384, 7
+    batch = 32768 if maxq > 1 else 131072
+    nq = batch + 77
+    ctx = hdc.Context(dim, 8, 150, 10)
+    q, r = _rows(torch, cuda, 5, nq, dim, maxq), _rows(torch, cuda, 6, nr, dim, maxr)
+    got = _search(hdc, ctx, q, maxq, r, maxr, k)
+    form, n = ctx.plain_last_form()
+    assert form == (DIGITS if maxq == 1 else F16) and n == kernels and ctx.status() == 0
+    rows = torch.cat([torch.arange(a, b, device=cuda) for a, b in ((0, 40), (batch - 50, batch + 77))])
+    _same_as_cuda_cores(hdc, ctx, got, q, maxq, r, maxr, k, rows)
