@@ -277,6 +277,11 @@ size_t hdc_search_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr
     return hdc::plain_workspace_bytes(ctx, nq, nr, k);
 }
 
+size_t hdc_search_workspace_min_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k) {
+    if (!ctx || nq <= 0 || nr <= 0 || k <= 0) return 0;
+    return hdc::plain_min_workspace_bytes(ctx, nq, nr, k);
+}
+
 int hdc_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, int64_t nq, int32_t max_abs_q,
                      const int16_t* d_r, const int64_t* d_rnorm2, int64_t nr, int32_t max_abs_r, int k,
                      int score_mode, float* d_score, int32_t* d_idx, double* d_cos, int64_t* d_dot, void* d_work,
@@ -567,7 +572,9 @@ int hdc_device_alloc(size_t bytes, void** out) {
     *out = nullptr;
     if (bytes == 0) return HDC_OK;
     cudaError_t e = cudaMalloc(out, bytes);
-    return e == cudaSuccess ? HDC_OK : hdc::cuda_fail(e, "alloc: cudaMalloc");
+    if (e == cudaSuccess) return HDC_OK;
+    cudaGetLastError();  // a caller may go on with less memory: the next launch does not report this
+    return hdc::cuda_fail(e, "alloc: cudaMalloc");
 }
 
 int hdc_device_free(void* p) {

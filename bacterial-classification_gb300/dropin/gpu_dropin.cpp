@@ -35,7 +35,10 @@ hdc_context* context() {
 // device buffer freed on scope exit
 struct DeviceBuffer {
     void* p = nullptr;
-    explicit DeviceBuffer(size_t bytes) { check(hdc_device_alloc(bytes, &p), "hdc_device_alloc"); }
+    // (of memory that is allocated already, or of its own)
+    explicit DeviceBuffer(size_t bytes, void* have = nullptr) : p(have) {
+        if (!p) check(hdc_device_alloc(bytes, &p), "hdc_device_alloc");
+    }
     ~DeviceBuffer() { hdc_device_free(p); }
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
@@ -121,8 +124,11 @@ std::unordered_map<HV_16*, std::vector<std::pair<float, HV_16*>>> cosine_search(
     int32_t maxabs[2];
     check(hdc_copy(maxabs, d_max.p, 8, 0, nullptr), "hdc_copy");
     check(hdc_stream_sync(nullptr), "hdc_stream_sync");
-    const size_t wb = hdc_search_workspace_bytes(ctx, nq, nr, k);
-    DeviceBuffer d_w(wb);
+    // where the rows leave no room for the tensor cores' operands, the CUDA-core kernel's few megabytes
+    size_t wb = hdc_search_workspace_bytes(ctx, nq, nr, k);
+    void* full = nullptr;
+    if (hdc_device_alloc(wb, &full) != HDC_OK) wb = hdc_search_workspace_min_bytes(ctx, nq, nr, k);
+    DeviceBuffer d_w(wb, full);
     check(hdc_search_plain(ctx, d_q.as<int16_t>(), d_qn.as<int64_t>(), nq, maxabs[0], d_r.as<int16_t>(),
                            d_rn.as<int64_t>(), nr, maxabs[1], k, mode, d_s.as<float>(), d_i.as<int32_t>(), nullptr,
                            nullptr, d_w.p, wb, nullptr),

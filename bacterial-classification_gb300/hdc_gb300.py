@@ -42,6 +42,7 @@ SIGNATURES = [
     ("hdc_encode_windows", I32, [P, P, P, P, I64, I64, P, P]),
     ("hdc_norms", I32, [P, P, I32, I64, P, P, P]),
     ("hdc_search_workspace_bytes", SZ, [P, I64, I64, I32]),
+    ("hdc_search_workspace_min_bytes", SZ, [P, I64, I64, I32]),
     ("hdc_search_plain", I32, [P, P, P, I64, ctypes.c_int32, P, P, I64, ctypes.c_int32, I32, I32, P, P, P, P, P,
                                SZ, P]),
     ("hdc_search_plain_last_form", I32, [P, P]),
@@ -210,7 +211,12 @@ class Context:
                    torch.empty((nq, kk), dtype=torch.int64, device=dev))
         wb = self.workspace_bytes(nq, nr, k)
         if work is None or work.numel() < wb:
-            work = torch.empty(max(wb, 16), dtype=torch.uint8, device=dev)
+            try:
+                work = torch.empty(max(wb, 16), dtype=torch.uint8, device=dev)
+            except torch.cuda.OutOfMemoryError:  # the CUDA-core kernel needs some megabytes only
+                wb = lib().hdc_search_workspace_min_bytes(self.h, nq, nr, k)
+                if work is None or work.numel() < wb:
+                    work = torch.empty(max(wb, 16), dtype=torch.uint8, device=dev)
         s, i, c, d = out
         check(lib().hdc_search_plain(self.h, ptr(q), ptr(qn), nq, int(maxq), ptr(r), ptr(rn), nr, int(maxr), k, mode,
                                      ptr(s), ptr(i), ptr(c), ptr(d), ptr(work), work.numel(), stream_ptr(stream)))

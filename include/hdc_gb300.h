@@ -157,9 +157,11 @@ int hdc_norms_f16(hdc_context* ctx, const void* d_hv, int64_t n, int64_t* d_norm
 
 /* Workspace of the plain search for nq queries and top-k (at most 2 GiB beyond
  * its partial lists): with all of it the search runs on the tensor cores where
- * the values allow; a smaller one that holds the partial lists of the CUDA-core
- * kernel is accepted too, and takes that kernel. */
+ * the values allow; a smaller one, down to hdc_search_workspace_min_bytes (the
+ * partial lists of the CUDA-core kernel, some megabytes), is accepted too and
+ * takes that kernel: for callers whose rows leave no room for more. */
 size_t hdc_search_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k);
+size_t hdc_search_workspace_min_bytes(const hdc_context* ctx, int64_t nq, int64_t nr, int k);
 
 /* Plain form: exact integer cosine top-k of int16 queries against int16
  * references, the drop-in for launch_cosine_topk
@@ -171,8 +173,8 @@ size_t hdc_search_workspace_bytes(const hdc_context* ctx, int64_t nq, int64_t nr
  * optional), d_dot (int64 exact dot; optional).  max_abs_q / max_abs_r bound
  * |element| of queries / references (from hdc_norms); products must satisfy
  * max_abs_q * max_abs_r <= 2^20 (else HDC_ERR_RANGE).  d_qnorm2 / d_rnorm2 come from hdc_norms.
- * d_work must hold hdc_search_workspace_bytes(nq, nr, k) bytes (256-byte
- * aligned).  Rows of |v| <= 2048 (and +1/0/-1 queries against |r| <= 18724) are
+ * d_work should hold hdc_search_workspace_bytes(nq, nr, k) bytes, 256-byte
+ * aligned; it must hold hdc_search_workspace_min_bytes.  Rows of |v| <= 2048 (and +1/0/-1 queries against |r| <= 18724) are
  * converted in the workspace and searched on the tensor cores, exactly; larger
  * values take CUDA cores. */
 int hdc_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, int64_t nq,

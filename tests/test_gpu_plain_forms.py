@@ -129,3 +129,27 @@ def test_plain_query_batches(hdc, cuda, maxq, maxr, nr, kernels):
     assert form == (DIGITS if maxq == 1 else F16) and n == kernels and ctx.status() == 0
     rows = torch.cat([torch.arange(a, b, device=cuda) for a, b in ((0, 40), (batch - 50, batch + 77))])
     _same_as_cuda_cores(hdc, ctx, got, q, maxq, r, maxr, k, rows)
+
+
+def test_plain_without_room_for_the_full_workspace(hdc, cuda):
+    """The binding goes on with the least workspace when the full one cannot be allocated, and a failed allocation
+    through the library leaves nothing behind for the next launch."""
+    import ctypes
+    import torch
+    ctx = hdc.Context(256, 8, 150, 10)
+    q, r = _rows(torch, cuda, 7, 40, 256, 60), _rows(torch, cuda, 8, 500, 256, 90)
+    qn, rn = ctx.norms(q), ctx.norms(r)
+    want = ctx.search_plain(q, qn, 60, r, rn, 90, 5)
+    assert ctx.plain_last_form()[0] == SPLIT
+    p = ctypes.c_void_p()
+    assert hdc.lib().hdc_device_alloc(1 << 50, ctypes.byref(p)) == 4 and not p.value
+    assert torch.equal(ctx.norms(q), qn)
+    ctx.workspace_bytes = lambda nq, nr, k: 1 << 50
+    got = ctx.search_plain(q, qn, 60, r, rn, 90, 5)
+    torch.cuda.synchronize()
+    assert ctx.plain_last_form()[0] == CUDA
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    small = torch.empty(1 << 16, dtype=torch.uint8, device=cuda)
+    ctx.search_plain(q, qn, 60, r, rn, 90, 5, work=small)
+    assert ctx.plain_last_form()[0] == CUDA
