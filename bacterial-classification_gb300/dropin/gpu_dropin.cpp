@@ -129,6 +129,9 @@ std::unordered_map<HV_16*, std::vector<std::pair<float, HV_16*>>> cosine_search(
     void* full = nullptr;
     if (hdc_device_alloc(wb, &full) != HDC_OK) wb = hdc_search_workspace_min_bytes(ctx, nq, nr, k);
     DeviceBuffer d_w(wb, full);
+    // one search at a time: the status word is the context's (the default stream runs them one after the other anyway)
+    static std::mutex one;
+    std::unique_lock<std::mutex> lock(one);
     check(hdc_search_plain(ctx, d_q.as<int16_t>(), d_qn.as<int64_t>(), nq, maxabs[0], d_r.as<int16_t>(),
                            d_rn.as<int64_t>(), nr, maxabs[1], k, mode, d_s.as<float>(), d_i.as<int32_t>(), nullptr,
                            nullptr, d_w.p, wb, nullptr),
@@ -138,6 +141,10 @@ std::unordered_map<HV_16*, std::vector<std::pair<float, HV_16*>>> cosine_search(
     check(hdc_copy(hs.data(), d_s.p, hs.size() * 4, 0, nullptr), "hdc_copy");
     check(hdc_copy(hi.data(), d_i.p, hi.size() * 4, 0, nullptr), "hdc_copy");
     check(hdc_stream_sync(nullptr), "hdc_stream_sync");
+    int gave_up = 0;  // a search on the tensor cores whose waits ran out leaves partial results
+    check(hdc_context_status(ctx, &gave_up), "hdc_context_status");
+    lock.unlock();
+    if (gave_up) throw std::runtime_error("hdc_search_plain: device status " + std::to_string(gave_up));
     result.reserve((size_t)nq);
     for (int64_t i = 0; i < nq; ++i) {
         std::vector<std::pair<float, HV_16*>> m((size_t)k);

@@ -193,7 +193,8 @@ int hdc_search_plain_last_form(const hdc_context* ctx, int32_t form[2]);
 
 /* Read and clear the device status word of the context (synchronizes the
  * device): 0, 100 + the code of a bounded device-side wait that gave up in
- * a tensor-core search or descent (which then returned partial results), or
+ * a search on the tensor cores (hdc_search_tc, hdc_search_plain, pipeline) or a
+ * descent (which then returned partial results), or
  * 200 when hdc_beam_search_split was given a max_children below the tree's. */
 int hdc_context_status(hdc_context* ctx, int* status);
 
@@ -340,7 +341,7 @@ int hdc_search_tc_last_shape(const hdc_context* ctx, int32_t shape[5]);
                               tensor-core kernel has more producer warps than the cooperative
                               CTA can hold (3 % faster at D = 16,384); -1 automatic (2 where
                               the cooperative CTAs fit, else 0); results are identical */
-#define HDC_WAIT_LIMIT 9   /* tensor-core search and grouped descent: their bounded device-side
+#define HDC_WAIT_LIMIT 9   /* searches on the tensor cores, identify and grouped descent: their bounded device-side
                               waits (pipeline mbarriers, grid barriers) give up after value x
                               1,000 SM cycles, 1 .. 4,000,000 (0: the default, 4,000,000,
                               about 2 s at 2 GHz); a wait that gives up makes the call return

@@ -21,3 +21,8 @@ def test_a_full_card_searches_with_the_least_workspace(stub):
     assert stub(2 << 30) == ["work %d" % (1 << 30), "found 1"]
     assert stub(1 << 20) == ["work 4096", "found 1"]
     assert stub(1 << 10) == ["threw hdc_device_alloc: stub"]
+
+
+def test_a_search_that_gave_up_is_an_error(stub):
+    """The tensor-core search reports a bounded wait that ran out in the status word only, with partial results."""
+    assert stub(2 << 30, 103)[-1].startswith("threw ") and "103" in stub(2 << 30, 103)[-1]
