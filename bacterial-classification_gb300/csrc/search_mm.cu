@@ -1144,6 +1144,7 @@ __global__ void __launch_bounds__(32 * kMergeWarps) mm_merge_kernel(
 
 // ---------------------------------------------------------------- operand preparation
 constexpr int kRowThreads = 128;
+constexpr int kCodeQueryBound = 201;  // status: a query value beyond the +1/0/-1 that the caller declared
 
 // e2m1 code of an integer digit of magnitude <= 4
 __device__ __forceinline__ uint32_t e2m1(int d) {
@@ -1165,10 +1166,11 @@ template <>
 __device__ __forceinline__ int as_int<__half>(__half x) { return __half2int_rn(x); }
 
 // Queries of values -1, 0, 1 as e2m1 tiles [query tile][K block][128 rows][64 bytes]; a thread makes 16 bytes (32
-// dims of one row).  Bound by the bytes of the 16-bit rows.
+// dims of one row).  Bound by the bytes of the 16-bit rows.  A value that the caller's bound does not allow is reported:
+// its code would be another number's.
 template <typename Q, bool VEC>
 __global__ void pack_queries_kernel(const Q* __restrict__ q, int64_t nq, int dim, int n_kb, int64_t n_chunks,
-                                    uint8_t* __restrict__ out) {
+                                    uint8_t* __restrict__ out, int* __restrict__ status) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_chunks) return;
     const int64_t per_row = (int64_t)n_kb * 4;
@@ -1178,6 +1180,7 @@ __global__ void pack_queries_kernel(const Q* __restrict__ q, int64_t nq, int dim
     uint32_t w[4] = {0, 0, 0, 0};
     if (row < nq) {
         const Q* src = q + row * dim + d0;
+        bool beyond = false;
         Q x[32];
         if (VEC && d0 + 32 <= dim) {
 #pragma unroll
@@ -1187,7 +1190,12 @@ __global__ void pack_queries_kernel(const Q* __restrict__ q, int64_t nq, int dim
             for (int u = 0; u < 32; ++u) x[u] = d0 + u < dim ? src[u] : Q(0);
         }
 #pragma unroll
-        for (int u = 0; u < 32; ++u) w[u >> 3] |= e2m1(as_int<Q>(x[u])) << (4 * (u & 7));
+        for (int u = 0; u < 32; ++u) {
+            const int v = as_int<Q>(x[u]);
+            beyond |= (uint32_t)(v + 1) > 2u;
+            w[u >> 3] |= e2m1(v) << (4 * (u & 7));
+        }
+        if (beyond) atomicCAS(status, 0, kCodeQueryBound);
     }
     const int64_t tile = ((row / kMmQueryTile) * n_kb + kb) * kMmQueryTile;
     *reinterpret_cast<uint4*>(out + f4_chunk(tile, (int)(row % kMmQueryTile), c)) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -1588,7 +1596,7 @@ size_t mm_f4_ref_bytes(int64_t nr, int dim, int limbs) {
 
 bool mm_sums_fit(bool f4, int64_t sum_per_dim) { return sum_per_dim * (f4 ? kMmF4Dims : 16) <= kMmMaxSum; }
 
-int mm_pack_queries(const void* d_q, bool is_f16, int64_t nq, int dim, void* out, cudaStream_t stream) {
+int mm_pack_queries(const void* d_q, bool is_f16, int64_t nq, int dim, void* out, int* status, cudaStream_t stream) {
     const int n_kb = n_kblocks(dim, true);
     const int64_t chunks = (nq + kMmQueryTile - 1) / kMmQueryTile * kMmQueryTile * n_kb * 4;
     const unsigned grid = (unsigned)((chunks + 255) / 256);
@@ -1598,15 +1606,15 @@ int mm_pack_queries(const void* d_q, bool is_f16, int64_t nq, int dim, void* out
         if (is_f16) {
             const __half* q = static_cast<const __half*>(d_q);
             if (vec)
-                pack_queries_kernel<__half, true><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o);
+                pack_queries_kernel<__half, true><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o, status);
             else
-                pack_queries_kernel<__half, false><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o);
+                pack_queries_kernel<__half, false><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o, status);
         } else {
             const int16_t* q = static_cast<const int16_t*>(d_q);
             if (vec)
-                pack_queries_kernel<int16_t, true><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o);
+                pack_queries_kernel<int16_t, true><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o, status);
             else
-                pack_queries_kernel<int16_t, false><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o);
+                pack_queries_kernel<int16_t, false><<<grid, 256, 0, stream>>>(q, nq, dim, n_kb, chunks, o, status);
         }
     }, "mm search: pack queries");
 }

@@ -45,7 +45,8 @@ size_t mm_f4_ref_bytes(int64_t nr, int dim, int limbs);
 // Whether the accumulators can be emptied often enough (after every MMA at most; digits: every K block).
 bool mm_sums_fit(bool f4, int64_t sum_per_dim);
 
-int mm_pack_queries(const void* d_q, bool is_f16, int64_t nq, int dim, void* out, cudaStream_t stream);
+// (a value other than -1, 0, 1 raises *status)
+int mm_pack_queries(const void* d_q, bool is_f16, int64_t nq, int dim, void* out, int* status, cudaStream_t stream);
 // references from int16 rows, or (limbs16 != null) from a database's fp16 limbs
 int mm_pack_refs(const int16_t* d_r, const __half* limbs16, int L16, int bits, int64_t r_pad, int64_t nr, int dim,
                  int limbs, void* out, cudaStream_t stream);

@@ -479,7 +479,7 @@ static int launch_plain_mm(hdc_context* ctx, MmOperands op, const PlainMm& p, co
         op.qn = d_qn + q0;
         st = mm_begin(lists, n, stream);
         if (st == HDC_OK)
-            st = op.f4 ? mm_pack_queries(d_q + q0 * dim, false, n, dim, wq, stream)
+            st = op.f4 ? mm_pack_queries(d_q + q0 * dim, false, n, dim, wq, ctx->d_status, stream)
                        : mm_rows_f16(d_q + q0 * dim, n, dim, op.lda, reinterpret_cast<__half*>(wq),
                                      static_cast<MmNorms*>(lists), stream);
         for (int64_t r0 = 0; r0 < nr && st == HDC_OK; r0 += p.nrc) {

@@ -1376,7 +1376,7 @@ int launch_search_tc(hdc_context* ctx, const hdc_refdb* db, const __half* d_q, c
         op.qn = d_qn;
         uint8_t* parts = static_cast<uint8_t*>(d_work);
         if (op.f4) {
-            const int st = mm_pack_queries(d_q, true, nq, ctx->dim, d_work, stream);
+            const int st = mm_pack_queries(d_q, true, nq, ctx->dim, d_work, ctx->d_status, stream);
             if (st != HDC_OK) return st;
             op.a = d_work;
             parts += mm_f4_query_bytes(nq, ctx->dim);
@@ -1389,7 +1389,7 @@ int launch_search_tc(hdc_context* ctx, const hdc_refdb* db, const __half* d_q, c
         void* lists = d_work;
         int st = HDC_OK;
         if (op.f4) {
-            st = mm_pack_queries(d_q, true, nq, ctx->dim, d_work, stream);
+            st = mm_pack_queries(d_q, true, nq, ctx->dim, d_work, ctx->d_status, stream);
             op.a = d_work;
             lists = static_cast<uint8_t*>(d_work) + mm_f4_query_bytes(nq, ctx->dim);
         } else {

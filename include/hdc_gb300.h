@@ -195,7 +195,9 @@ int hdc_search_plain_last_form(const hdc_context* ctx, int32_t form[2]);
  * device): 0, 100 + the code of a bounded device-side wait that gave up in
  * a search on the tensor cores (hdc_search_tc, hdc_search_plain, pipeline) or a
  * descent (which then returned partial results), or
- * 200 when hdc_beam_search_split was given a max_children below the tree's. */
+ * 200 when hdc_beam_search_split was given a max_children below the tree's, or
+ * 201 when a search declared for +1/0/-1 queries (max_abs_q = 1) met a larger
+ * value, whose results are then meaningless. */
 int hdc_context_status(hdc_context* ctx, int* status);
 
 /* Precision form, reference side: build a tensor-core database from int16

@@ -153,3 +153,28 @@ def test_plain_without_room_for_the_full_workspace(hdc, cuda):
     small = torch.empty(1 << 16, dtype=torch.uint8, device=cuda)
     ctx.search_plain(q, qn, 60, r, rn, 90, 5, work=small)
     assert ctx.plain_last_form()[0] == CUDA
+
+
+@pytest.mark.parametrize("kind", ["plain", "tc"])
+@pytest.mark.parametrize("at,value", [(0, 2), (39 * 256 + 255, -2), (7 * 256 + 31, 9), (20 * 256 + 64, -2048)])
+def test_queries_beyond_their_declared_bound_are_reported(hdc, cuda, kind, at, value):
+    """A search on digits declared for +1/0/-1 queries packs e2m1 codes: a larger value raises status 201."""
+    import torch
+    ctx = hdc.Context(256, 8, 150, 10)
+    q, r = _rows(torch, cuda, 9, 40, 256, 1), _rows(torch, cuda, 10, 300, 256, 3000)
+
+    def run():
+        if kind == "plain":
+            ctx.search_plain(q, ctx.norms(q), 1, r, ctx.norms(r), 3000, 5)
+            assert ctx.plain_last_form()[0] == DIGITS
+        else:
+            h = q.half()
+            ctx.search_tc(db, h, ctx.norms(h), 1, 5)
+        torch.cuda.synchronize()
+        return ctx.status()
+    db = ctx.refdb(r, 3000) if kind == "tc" else None
+    assert run() == 0
+    q.view(-1)[at] = value
+    assert run() == 201
+    q.view(-1)[at] = 1
+    assert run() == 0
