@@ -407,6 +407,10 @@ int hdc_context_option(hdc_context* ctx, int option, int value) {
             if (value != 0 && value != 32 && value != 64) return fail(HDC_ERR_INVALID, "option: K block must be 0, 32 or 64");
             ctx->tc_kblock = value;
             return HDC_OK;
+        case HDC_TC_FORMS:
+            if (value < -1 || value > 0) return fail(HDC_ERR_INVALID, "option: database search forms must be -1 or 0");
+            ctx->tc_forms = value == 0 ? 0 : 1;
+            return HDC_OK;
         case HDC_BEAM_GROUPED:
             if (value < -1 || value > 2) return fail(HDC_ERR_INVALID, "option: beam grouping must be -1, 0, 1 or 2");
             ctx->beam_grouped = value;

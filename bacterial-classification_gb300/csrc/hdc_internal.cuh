@@ -37,6 +37,7 @@ struct hdc_context {
     int tc_pair_mma = -1;           // tensor-core search: CTA pairs as one M = 256 MMA (-1: automatic)
     int tc_kblock = 0;              // tensor-core search: dims per K block, 32 or 64 (0: automatic)
     int tc_scatter = -1;            // tensor-core search: 1 scattered reference-tile order, 0 index order (-1: auto)
+    int tc_forms = 1;               // tensor-core databases made on it get their search forms (0: the limbs alone)
     int beam_grouped = -1;          // descent: 1 grouped by candidate node, 2 + tensor-core levels, 0 warp per read
     void* noalloc_scratch = nullptr;  // device address of hdc_search_plain_noalloc's fixed scratch (first call)
     int greedy_form = -1;             // propagate-children selection: 1 scored (dim % 8 == 0), 0 sequential, -1 automatic
@@ -62,8 +63,8 @@ struct hdc_refdb {
     int32_t limb_max[4] = {0, 0, 0, 0};
     int limb_bits = 11;         // limbs are balanced base-2^limb_bits digits (the top one within the cap)
     int32_t max_abs = 0;
-    // The same references for the single-accumulator search, beside the limbs where the values allow it and memory
-    // is left (null otherwise: the limbs serve): base-8 digit tiles for +1/-1 queries, or one fp16 row each for
+    // The same references for the single-accumulator search, beside the limbs where the values allow it and enough
+    // memory is left (null otherwise: the limbs serve): base-8 digit tiles for +1/-1 queries, or one fp16 row each for
     // count-valued queries.
     void* d_digits = nullptr;
     int digits = 0;
@@ -127,8 +128,8 @@ int tc_default_share();
 int tc_default_scatter();
 int tc_default_kblock();
 int tc_default_pair_mma();
-// Build the forms of the single-accumulator search from the limbs (synchronizes the stream); a form that does not fit
-// in memory is left out.
+// Build the forms of the single-accumulator search from the limbs (synchronizes the stream); a form that would not leave
+// the caller enough memory is left out.
 int refdb_forms(const hdc_context* ctx, hdc_refdb* db, cudaStream_t stream);
 // Fill db->d_sqrt (allocated here) from db->d_norm2.
 int refdb_sqrt_table(hdc_refdb* db, cudaStream_t stream);

@@ -883,6 +883,21 @@ void refdb_destroy(hdc_refdb* db) {
     delete db;
 }
 
+// Memory of a search form, or null: the forms are an extra that the limbs can do without, so they leave the caller at least
+// a quarter of the device's memory (a database of +1/-1 queries takes half of its limbs' bytes again in digits, and what
+// the caller allocates afterwards fitted beside the limbs alone).
+static void* form_alloc(const hdc_context* ctx, size_t bytes) {
+    size_t free_bytes = 0, total = 0;
+    void* p = nullptr;
+    if (!ctx->tc_forms) return nullptr;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || bytes > free_bytes || free_bytes - bytes < total / 4 ||
+        cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
 int refdb_forms(const hdc_context* ctx, hdc_refdb* db, cudaStream_t stream) {
     // the largest value (int32), the largest squared norm, then the fp16 rows' norms
     constexpr size_t kMeasured = 2 * sizeof(int64_t) + 2 * sizeof(MmNorms);
@@ -911,22 +926,17 @@ int refdb_forms(const hdc_context* ctx, hdc_refdb* db, cudaStream_t stream) {
         const int digits = mm_f4_limbs(db->value_max);
         const size_t bytes = digits ? mm_f4_ref_bytes(db->nr, db->dim, digits) : 0;
         if (digits && bytes / 64 <= 0x7fffffff) {  // TMA coordinates are 32-bit
-            if (cudaMalloc(&db->d_digits, bytes) == cudaSuccess) {
+            db->d_digits = form_alloc(ctx, bytes);
+            if (db->d_digits) {
                 db->digits = digits;
                 st = mm_pack_refs(nullptr, db->d_limbs, db->L, db->limb_bits, db->r_pad, db->nr, db->dim, digits,
                                   db->d_digits, stream);
-            } else {
-                cudaGetLastError();
-                db->d_digits = nullptr;
             }
         }
     } else if (db->L > 1 && db->value_max <= 2048) {
-        if (cudaMalloc(&db->d_rows16, (size_t)db->r_pad * db->dim * sizeof(__half)) == cudaSuccess) {
+        db->d_rows16 = static_cast<__half*>(form_alloc(ctx, (size_t)db->r_pad * db->dim * sizeof(__half)));
+        if (db->d_rows16)
             st = mm_rows_from_limbs(db->d_limbs, db->L, db->limb_bits, db->r_pad, db->dim, db->d_rows16, stream);
-        } else {
-            cudaGetLastError();
-            db->d_rows16 = nullptr;
-        }
     }
     if (st == HDC_OK && db->d_rows16) {
         MmNorms* d_norms = reinterpret_cast<MmNorms*>(d_max + 2);

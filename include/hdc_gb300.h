@@ -204,7 +204,13 @@ int hdc_context_status(hdc_context* ctx, int* status);
  * (elem_bytes 2) or int32 (4) reference hypervectors [nr][dim] with
  * max |v| <= max_abs.  Each value is split into balanced base-2048 fp16
  * limbs (1 limb for |v| <= 2048, 2 for |v| <= 2048*2048+1023, ...), and the
- * exact squared norms are kept.  Synchronizes the stream.  dim must be a
+ * exact squared norms are kept: 2 bytes a value and limb.  Beside the limbs,
+ * where the values allow it and a quarter of the device's memory stays free,
+ * the database holds them in the form that hdc_search_tc runs fastest on:
+ * base-8 digits, half a byte a value and digit (4 up to |v| = 2340, 5 up to
+ * 18,724), or for count-valued queries (hdc_refdb_create_ex) 2 bytes a value
+ * of |v| <= 2048.  Without that form the limbs serve, at less than half the
+ * speed (HDC_TC_FORMS 0 declines it and its memory).  Synchronizes the stream.  dim must be a
  * multiple of 8.  No reference counterpart (the reference re-uploads and
  * re-normalises the database on every cosine_search call, src/cosine.cu:
  * 512-533). */
@@ -329,6 +335,9 @@ int hdc_search_tc_last_shape(const hdc_context* ctx, int32_t shape[5]);
                               (cta_group::2), 1 on, 0 off, -1 automatic */
 #define HDC_TC_LANES 8     /* tensor-core search: at most this many reference lanes per query tile
                               (CTAs that split the references of one query tile); 0 automatic */
+#define HDC_TC_FORMS 13    /* databases created or loaded on the context: -1 (automatic) with the search
+                              forms beside their limbs where these leave a quarter of the device's
+                              memory free (see hdc_refdb_create), 0 without */
 #define HDC_BEAM_GROUPED 4 /* hdc_beam_search: 1 reads grouped by candidate node, 2 the same
                               with every level but the last scored on the tensor cores
                               (entries grouped by parent), 0 one warp per read, -1
