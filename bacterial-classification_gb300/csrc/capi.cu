@@ -131,8 +131,9 @@ int hdc_context_create(int dim, int kmer, int window, int step, hdc_context** ou
         if (excess > 0) w[c->words64 - 1] &= (~uint64_t(0)) >> excess;
     }
     e = cudaMalloc(&c->d_base32, sizeof(uint64_t) * 4 * (size_t)c->words64);
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(c->d_status, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_status, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(c->d_status, 0, 2 * sizeof(int));
+    c->d_id_form = c->d_status + 1;
     if (e != cudaSuccess) {
         cudaFree(c->d_base32);
         cudaFree(c->d_status);
@@ -301,6 +302,12 @@ int hdc_search_plain_last_form(const hdc_context* ctx, int32_t form[2]) {
     if (!ctx || !form) return fail(HDC_ERR_INVALID, "search form: null argument");
     for (int i = 0; i < 2; ++i) form[i] = ctx->plain_last_form[i];
     return HDC_OK;
+}
+
+int hdc_identify_last_form(const hdc_context* ctx, int* form) {
+    if (!ctx || !form) return fail(HDC_ERR_INVALID, "identify form: null argument");
+    const cudaError_t e = cudaMemcpy(form, ctx->d_id_form, sizeof(int), cudaMemcpyDeviceToHost);
+    return e == cudaSuccess ? HDC_OK : hdc::cuda_fail(e, "identify form: read");
 }
 
 int hdc_context_status(hdc_context* ctx, int* status) {

@@ -23,6 +23,7 @@ struct hdc_context {
     uint64_t* host_base = nullptr;  // [4][words64], A,C,G,T
     uint32_t* d_base32 = nullptr;   // [4][words32] on the device
     int* d_status = nullptr;        // device status word written by kernels that can give up
+    int* d_id_form = nullptr;       // how the last identify ran (hdc_identify_last_form), the word after it
     int tc_group = 0;               // tensor-core search: query tiles per group (0: automatic)
     int tc_policy = -1;             // tensor-core search: L2 policy (-1: automatic, see hdc_search_tc_tuning)
     int tc_tile_n = 0;              // tensor-core search: references per tile, 128 or 256 (0: automatic)

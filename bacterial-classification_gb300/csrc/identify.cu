@@ -95,7 +95,14 @@ __global__ void __launch_bounds__(32 * kIdWarps) identify_kernel(const IdentifyA
     __shared__ int n_beam_s, done_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r = blockIdx.x;
-    if (a.only_if && *a.only_if == 0) return;
+    int first = 0;  // level to start from
+    if (a.from.level) {
+        first = *a.from.level - 1;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.form = first + 1;
+        if (first < 0 || (first > 0 && a.from.done[r])) return;
+    } else if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.form = HDC_IDENTIFY_PER_READ;
+    }
     {
         const uint4* src = reinterpret_cast<const uint4*>(a.q + r * a.dim);
         uint4* dst = reinterpret_cast<uint4*>(qs);
@@ -108,12 +115,19 @@ __global__ void __launch_bounds__(32 * kIdWarps) identify_kernel(const IdentifyA
     int32_t out_path[kMaxLevels];
     float out_score[kMaxLevels];
     if (threadIdx.x == 0) {
-        n_beam_s = 0;
+        n_beam_s = first > 0 ? a.from.nbeam[r] : 0;
         done_s = 0;
+    }
+    if (first > 0 && threadIdx.x < kMaxBeam * kMaxLevels) {
+        const int b = threadIdx.x / kMaxLevels, l = threadIdx.x % kMaxLevels;
+        if (b < a.from.nbeam[r] && l < first) {
+            paths[b][l] = a.from.paths[(r * kMaxBeam + b) * kMaxLevels + l];
+            scores[b][l] = a.from.scores[(r * kMaxBeam + b) * kMaxLevels + l];
+        }
     }
     __syncthreads();
     int parity = 0;
-    for (int L = 0; L < a.levels; ++L) {
+    for (int L = first; L < a.levels; ++L) {
         n_top = 0;
         const int n_src = L == 0 ? 1 : n_beam_s;
         for (int b = 0; b < n_src; ++b) {
@@ -281,8 +295,8 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
         cudaError_t e = cudaFuncSetAttribute(identify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return cuda_fail(e, "identify: shared memory attribute");
     }
-    // Batches of reads grouped by parent on the tensor cores, each followed by the per-read kernel for what does not
-    // fit there (it exits at once otherwise).  A few reads with one beam row each, a CTA a read, wait as long for their
+    // Batches of reads grouped by parent on the tensor cores, each followed by the per-read kernel, which goes on from the
+    // level that does not fit there (and exits at once if all did).  A few reads with one beam row each, a CTA a read, wait as long for their
     // own gathers as for the grouped form's five launches a level: 17 reads, D = 1,024, 233 us against 251; 30, D = 2,048,
     // 291 against 299 (10 reads with three rows each: 865 against 293).
     const bool few = nq <= ctx->num_sms && beam == 1 && ctx->dim <= 2048;
@@ -290,12 +304,10 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
         const int64_t n = std::min(kIdBatch, nq - r0);
         IdentifyArgs a{d_q + r0 * ctx->dim, d_qn + r0, d_rows, d_rn, d_node_rows, d_child_ptr, d_child_idx, d_roots, n_roots,
                        ctx->dim, levels, beam, mode, threshold, d_path + r0 * levels, d_path_score + r0 * levels,
-                       d_depth + r0, d_stop_level ? d_stop_level + r0 : nullptr, nullptr};
-        int32_t* flag = nullptr;
+                       d_depth + r0, d_stop_level ? d_stop_level + r0 : nullptr, ctx->d_id_form, {}};
         void* ws = nullptr;
-        const int st = few ? HDC_OK : launch_identify_grouped(ctx, a, n, &flag, &ws, stream);
+        const int st = few ? HDC_OK : launch_identify_grouped(ctx, a, n, &a.from, &ws, stream);
         if (st != HDC_OK) return st;
-        a.only_if = flag;
         identify_kernel<<<(unsigned)n, 32 * kIdWarps, smem, stream>>>(a);
         cudaError_t e = cudaGetLastError();
         if (ws) cudaFreeAsync(ws, stream);

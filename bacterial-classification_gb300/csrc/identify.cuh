@@ -8,6 +8,15 @@ namespace hdc {
 constexpr int kIdBeam = 8;
 constexpr int kIdLevels = 8;
 
+// The beams that a grouped descent has reached.
+struct IdentifyState {
+    const int32_t* level;  // 0: it did every level; l + 1: level l and the ones after it are still to be done
+    const int32_t* done;   // [nq] reads that have stopped (their outputs are written)
+    const int32_t* nbeam;  // [nq]
+    const int32_t* paths;  // [nq][kIdBeam][kIdLevels] node and score of each beam row's levels so far
+    const float* scores;
+};
+
 struct IdentifyArgs {
     const int16_t* q;         // [nq][dim] whole-read hypervectors
     const int64_t* qn;        // [nq]
@@ -24,12 +33,13 @@ struct IdentifyArgs {
     float* path_score;        // [nq][levels]
     int32_t* depth;           // [nq]
     int32_t* stop_level;      // [nq] level of an early stop, -1 when all levels ran (may be null)
-    const int32_t* only_if;   // the per-read kernel runs only where this is null or points at a nonzero word
+    int32_t* form;            // how the batch ran (hdc_identify_last_form), written by the per-read kernel
+    IdentifyState from;       // of a grouped descent that the per-read kernel finishes
 };
 
-// The descent of nq reads grouped by parent.  *flag (in *workspace, which the caller frees on the stream) is nonzero
-// afterwards where the per-read kernel has to do the batch instead; null: it was not started.
-int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t nq, int32_t** flag, void** workspace,
+// The descent of nq reads grouped by parent; *from is its state (in *workspace, which the caller frees on the stream),
+// which says afterwards where the per-read kernel has to go on.  Its level null: it was not started.
+int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t nq, IdentifyState* from, void** workspace,
                             cudaStream_t stream);
 
 }  // namespace hdc

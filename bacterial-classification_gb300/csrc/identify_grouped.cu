@@ -13,8 +13,9 @@
 //
 // Exactness.  Rows and reads are int16; |v| <= 2048 is exact in fp16, and by Cauchy-Schwarz every partial sum of a dot is
 // at most |q| |r|, so with |q|^2 |r|^2 <= 2^48 the fp32 accumulator holds exact integers.  Whatever does not fit (a
-// larger value or norm, a level with more candidates than the workspace) raises a flag on the device, and the per-read
-// kernel, launched behind, then does the whole batch; it exits at once otherwise.
+// larger value or norm, a level with more candidates than the workspace, a wait that ran out) raises a flag on the device
+// with the level that it happened in, and the per-read kernel, launched behind, takes the reads on from the beams that the
+// level started with; it exits at once otherwise.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -74,9 +75,10 @@ struct Level {
     uint32_t* best;       // [max_pairs] orderable score of each candidate, 0: nothing yet
     int64_t max_pairs;
     int32_t* counters;    // entries, items, pairs, next item of the level
-    int32_t* flag;        // 1: leave the batch to the per-read kernel
+    int32_t* flag;        // l + 1: leave level l and the ones after it to the per-read kernel
     int* status;
     long long wait_cycles;
+    int withhold;         // test hook: no rows are copied
 };
 enum { kCntEntries, kCntItems, kCntPairs, kCounters };
 
@@ -103,12 +105,12 @@ __device__ __forceinline__ void add_items(const Level& v, int32_t slot, int32_t 
     }
     const int64_t chunks = (rows + kN - 1) / kN, n = chunks * ((m + kM - 1) / kM);
     if (n > v.max_items || rows > 0x7fffffff) {
-        *v.flag = 1;
+        *v.flag = v.L + 1;
         return;
     }
     const int32_t x = atomicAdd(v.counters + kCntItems, (int32_t)n);
     if (x + n > v.max_items) {
-        *v.flag = 1;
+        *v.flag = v.L + 1;
         return;
     }
     // the entry tiles of one row chunk side by side: they read the same rows at about the same time
@@ -153,7 +155,7 @@ __global__ void entries_kernel(const Level v) {
     if (lane == 0 && total) p0 = atomicAdd(v.counters + kCntPairs, total);
     p0 = __shfl_sync(0xffffffffu, p0, 0);
     if ((int64_t)p0 + total > v.max_pairs || p0 < 0) {
-        if (lane == 0) *v.flag = 1;
+        if (lane == 0) *v.flag = v.L + 1;
         return;  // the whole warp
     }
     if (!on) return;
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
     if (warp < kCopyWarps) {
         int stage = 0;
         uint32_t phase = 0;
-        bool ok = true;
+        bool ok = !v.withhold;
         int n = 0;  // items so far
         for (int it = blockIdx.x; ok && it < n_items; it += gridDim.x, ++n) {
             const int buf = n & 1;
@@ -392,7 +394,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
                 };
                 for (int i = 0; i < end_a; i += 4) four(i, end_a, n_ent);
                 for (int i = kTasksA; i < end_b; i += 4) four(i, end_b, kM + n_cols);
-                if (out) *v.flag = 1;
+                if (out) *v.flag = v.L + 1;
                 tc::fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&sm.full[stage]);
@@ -510,7 +512,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
                 double m[2] = {0, 0};
                 for (int w = 0; w < kM / 32; ++w)
                     for (int i = 0; i < 2; ++i) m[i] = fmax(m[i], (double)sm.norm_max[i][w]);
-                if (m[0] * m[1] > 281474976710656.0) *v.flag = 1;  // |q| |r| <= 2^24 for every pair of the item
+                if (m[0] * m[1] > 281474976710656.0) *v.flag = v.L + 1;  // |q| |r| <= 2^24 for every pair of the item
             }
             epi_sync();
             if (row == 0) t.seg[t.n_seg] = t.n_cols;
@@ -589,6 +591,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
         tc::tmem_dealloc(tmem, 512);
     }
     if (tid == 0 && sm.err) {
+        *v.flag = v.L + 1;
         atomicCAS(v.status, 0, 100 + sm.err);
     }
 }
@@ -720,15 +723,16 @@ T* carve(uint8_t*& cur, int64_t n) {
 
 }  // namespace
 
-int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t nq, int32_t** flag, void** workspace,
+int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t nq, IdentifyState* from, void** workspace,
                             cudaStream_t stream) {
-    *flag = nullptr;
+    *from = IdentifyState{};
     *workspace = nullptr;
     Level v{};
     v.a = args;
     v.nq = nq;
     v.status = ctx->d_status;
     v.wait_cycles = ctx->wait_cycles > 0 ? ctx->wait_cycles : tc::kWaitCycles;
+    v.withhold = ctx->test_withhold_loads == 1;
     const int64_t E = nq * args.beam;
     v.table = 1024;
     while (v.table < 2 * E) v.table *= 2;
@@ -784,7 +788,7 @@ int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t 
         *workspace = nullptr;
         return cuda_fail(e, "identify: grouped launch");
     }
-    *flag = v.flag;
+    *from = IdentifyState{v.flag, v.done, v.nbeam, v.paths, v.scores};
     return HDC_OK;
 }
 

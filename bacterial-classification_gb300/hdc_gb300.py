@@ -54,6 +54,7 @@ SIGNATURES = [
                                          ctypes.c_double, I32, P, P, P, P]),
     ("hdc_similarity", I32, [P, P, P, P, P, P, P, P, P, I64, I32, P, P, P]),
     ("hdc_identify", I32, [P, P, P, I64, P, P, P, P, P, P, I32, I32, I32, ctypes.c_double, I32, P, P, P, P, P]),
+    ("hdc_identify_last_form", I32, [P, ctypes.POINTER(ctypes.c_int)]),
     ("hdc_propagate_greedy", I32, [P, P, P, P, P, P, P, I64, ctypes.c_double, I32, P, P, P, P]),
     ("hdc_context_status", I32, [P, ctypes.POINTER(ctypes.c_int)]),
     ("hdc_search_plain_noalloc", I32, [P, P, P, I64, ctypes.c_int32, P, P, I64, ctypes.c_int32, I32, I32, P, P, P,
@@ -349,6 +350,12 @@ class Context:
                                  ptr(child_idx), ptr(roots), roots.numel(), levels, beam, threshold, mode, ptr(path),
                                  ptr(score), ptr(depth), ptr(stop), stream_ptr(stream)))
         return path, score, depth, stop
+
+    def identify_last_form(self):
+        """How the last identify ran: 0 grouped, l > 0 one CTA a read from level l - 1, -1 one CTA a read."""
+        form = ctypes.c_int(0)
+        check(lib().hdc_identify_last_form(self.h, ctypes.byref(form)))
+        return form.value
 
     def fasta_parse(self, d_bytes, max_records=None, stream=None):
         """Device FASTA ingest of raw file bytes (uint8 tensor): returns (sequence bytes, seq_off,

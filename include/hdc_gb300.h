@@ -355,8 +355,9 @@ int hdc_search_tc_last_shape(const hdc_context* ctx, int32_t shape[5]);
 #define HDC_WAIT_LIMIT 9   /* searches on the tensor cores, identify and grouped descent: their bounded device-side
                               waits (pipeline mbarriers, grid barriers) give up after value x
                               1,000 SM cycles, 1 .. 4,000,000 (0: the default, 4,000,000,
-                              about 2 s at 2 GHz); a wait that gives up makes the call return
-                              partial results and hdc_context_status report 100 + its code
+                              about 2 s at 2 GHz); a wait that gives up makes hdc_context_status
+                              report 100 + its code and the call return partial results
+                              (identify: all of them, one CTA a read from there on)
                               (120: a grid barrier of the cooperative descent) */
 #define HDC_GREEDY_FORM 12 /* hdc_propagate_greedy: 1 scores every pair a decision can need in
                               bulk (tiled kernels), then decides each parent's candidates in order
@@ -364,7 +365,7 @@ int hdc_search_tc_last_shape(const hdc_context* ctx, int32_t shape[5]);
                               dots as it goes; -1 automatic (1 when dim % 8 == 0); results are
                               identical */
 #define HDC_TEST_WITHHOLD_LOADS 10 /* for tests of the bounded waits only: 1 makes the
-                              tensor-core search's producer issue no operand loads, so the MMA
+                              tensor-core search's and identify's producers issue no operand loads, so the MMA
                               issuer's and the epilogue's waits run out (after HDC_WAIT_LIMIT)
                               with nothing in flight; 2 makes the cooperative descent's first
                               CTA reach its first grid barrier four limits late, so the other
@@ -466,6 +467,14 @@ int hdc_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, 
                  const int32_t* d_child_idx, const int32_t* d_roots, int n_roots, int levels, int beam,
                  double threshold, int score_mode, int32_t* d_path, float* d_path_score, int32_t* d_depth,
                  int32_t* d_stop_level, void* stream);
+
+/* How the last hdc_identify on this context ran, its last 65,536 reads where it
+ * took several passes (diagnostic; synchronizes the device): 0 grouped by
+ * parent on the tensor cores, l > 0 the same down to level l - 1, from which one
+ * CTA a read went on, HDC_IDENTIFY_PER_READ one CTA a read from the start (0
+ * before the first). */
+#define HDC_IDENTIFY_PER_READ (-1)
+int hdc_identify_last_form(const hdc_context* ctx, int* form);
 
 /* FASTA ingest on the device, with the reading of targets/identify.cpp:46-71:
  * lines end at '\n' only (a '\r' stays part of the line); a line starting with
