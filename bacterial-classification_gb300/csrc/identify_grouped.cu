@@ -737,7 +737,9 @@ int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t 
     v.table = 1024;
     while (v.table < 2 * E) v.table *= 2;
     v.max_items = 2 * E + 65536;
-    v.max_pairs = std::max<int64_t>(nq * args.n_roots, 32 * E) + 4096;
+    // 32 candidates an entry, and 256 up to 32 MB: beams of a few thousand reads over a genus of hundreds stay grouped
+    // (4,096 reads, five beam rows, 4 x 20 x 200 nodes of 20 rows, D = 1,024: 2.1 ms against 128 with the last level per read)
+    v.max_pairs = std::max<int64_t>(nq * args.n_roots, std::max<int64_t>(32 * E, std::min<int64_t>(256 * E, 8 << 20))) + 4096;
     if (v.max_pairs > 0x7fffffff - 65536) return HDC_OK;
     auto carve_all = [&](uint8_t* base) {
         uint8_t* cur = base;

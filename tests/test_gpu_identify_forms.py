@@ -76,9 +76,9 @@ def test_descent_goes_on_from_the_level_that_does_not_fit(hdc, orc, cuda, level,
     assert form == (0 if level is None else level + 1) and ctx.status() == 0
 
 
-@pytest.mark.parametrize("branches,beam,form", [([2, 2, 60], 3, 3), ([2, 60], 1, 2), ([70], 1, 0), ([2, 2, 30], 3, 0)])
+@pytest.mark.parametrize("branches,beam,form", [([2, 2, 300], 3, 3), ([2, 300], 1, 2), ([300], 1, 0), ([2, 2, 250], 3, 0)])
 def test_levels_with_more_candidates_than_the_workspace(hdc, orc, cuda, branches, beam, form):
-    """A pass reserves 32 candidates an entry (and one a read and root)."""
+    """A pass of a few reads reserves 256 candidates an entry (and one a read and root)."""
     g, tree, rows, q = _inputs(3, branches, 64, 300, lambda rank, node: 1)
     ctx = hdc.Context(64, 8, 150, 10)
     assert _check(hdc, orc, cuda, ctx, q, rows, tree, len(branches), beam, -2.0, 0) == form
