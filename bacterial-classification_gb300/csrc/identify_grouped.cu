@@ -46,6 +46,8 @@ constexpr int kRowStep = kGroupThreads / kPieces;            // rows between the
 constexpr int kTasksA = kM / kRowStep;                 // the first of them are the entries'
 static_assert(kCopyThreads == kGroupThreads && (kM + kN) % kRowStep == 0 && kM % kRowStep == 0, "whole chunks a thread");
 
+constexpr int kMaxChildren = 1 << 25;  // a warp's candidates sum to 2^30 at most
+
 struct Item {
     int32_t slot, e0, n, col0;  // parent's table slot (-1: the roots), first entry and entries, first row
 };
@@ -74,7 +76,7 @@ struct Level {
     int64_t max_items;
     uint32_t* best;       // [max_pairs] orderable score of each candidate, 0: nothing yet
     int64_t max_pairs;
-    int32_t* counters;    // entries, items, pairs, next item of the level
+    unsigned long long* counters;  // entries, items and pairs of the level (64 bits: what does not fit is still counted)
     int32_t* flag;        // l + 1: leave level l and the ones after it to the per-read kernel
     int* status;
     long long wait_cycles;
@@ -108,13 +110,13 @@ __device__ __forceinline__ void add_items(const Level& v, int32_t slot, int32_t 
         *v.flag = v.L + 1;
         return;
     }
-    const int32_t x = atomicAdd(v.counters + kCntItems, (int32_t)n);
+    const int64_t x = (int64_t)atomicAdd(v.counters + kCntItems, (unsigned long long)n);
     if (x + n > v.max_items) {
         *v.flag = v.L + 1;
         return;
     }
     // the entry tiles of one row chunk side by side: they read the same rows at about the same time
-    int32_t i = x;
+    int64_t i = x;
     for (int64_t c = 0; c < chunks; ++c)
         for (int32_t e = 0; e < m; e += kM) v.items[i++] = Item{slot, e, min(kM, m - e), (int32_t)(c * kN)};
 }
@@ -142,6 +144,10 @@ __global__ void entries_kernel(const Level v) {
     if (on) {
         if (v.L > 0) P = v.paths[at(r, b, v.L - 1)];
         nch = n_children(v.a, P);
+        if (nch > kMaxChildren) {
+            *v.flag = v.L + 1;
+            nch = 0;
+        }
     }
     // the candidates' places: one atomic a warp
     int32_t before = nch;
@@ -151,15 +157,15 @@ __global__ void entries_kernel(const Level v) {
     }
     const int32_t total = __shfl_sync(0xffffffffu, before, 31);
     before -= nch;
-    int32_t p0 = 0;
-    if (lane == 0 && total) p0 = atomicAdd(v.counters + kCntPairs, total);
+    long long p0 = 0;
+    if (lane == 0 && total) p0 = (long long)atomicAdd(v.counters + kCntPairs, (unsigned long long)total);
     p0 = __shfl_sync(0xffffffffu, p0, 0);
-    if ((int64_t)p0 + total > v.max_pairs || p0 < 0) {
+    if (p0 + total > v.max_pairs) {
         if (lane == 0) *v.flag = v.L + 1;
         return;  // the whole warp
     }
     if (!on) return;
-    v.ent_p0[e] = p0 + before;
+    v.ent_p0[e] = (int32_t)p0 + before;  // (below max_pairs < 2^31)
     for (int j = 0; j < nch; ++j) v.best[p0 + before + j] = 0;
     if (v.L == 0) {
         v.ent_slot[e] = -1;
@@ -191,7 +197,7 @@ __global__ void parents_kernel(const Level v) {
     if (h >= v.table) return;
     const int32_t m = v.tab_cnt[h];
     if (!m) return;
-    v.tab_off[h] = atomicAdd(v.counters + kCntEntries, m);
+    v.tab_off[h] = (int32_t)atomicAdd(v.counters + kCntEntries, (unsigned long long)m);
     add_items(v, (int32_t)h, v.tab_key[h], m);
 }
 
@@ -281,7 +287,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
     volatile int* err = &sm.err;
     if (tid == 0) {
         sm.err = 0;
-        sm.n_items = *v.flag ? 0 : v.counters[kCntItems];
+        sm.n_items = *v.flag ? 0 : (int)v.counters[kCntItems];
         for (int s = 0; s < kStagesId; ++s) {
             tc::mbar_init(&sm.raw[s], kCopyThreads);
             tc::mbar_init(&sm.full[s], kGroupWarps);
@@ -744,7 +750,7 @@ int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t 
     auto carve_all = [&](uint8_t* base) {
         uint8_t* cur = base;
         v.flag = carve<int32_t>(cur, 1);
-        v.counters = carve<int32_t>(cur, kCounters);
+        v.counters = carve<unsigned long long>(cur, kCounters);
         v.nbeam = carve<int32_t>(cur, nq);
         v.done = carve<int32_t>(cur, nq);
         v.tab_cnt = carve<int32_t>(cur, v.table);
