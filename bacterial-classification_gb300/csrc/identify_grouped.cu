@@ -50,6 +50,7 @@ constexpr int kMaxChildren = 1 << 25;  // a warp's candidates sum to 2^30 at mos
 
 struct Item {
     int32_t slot, e0, n, col0;  // parent's table slot (-1: the roots), first entry and entries, first row
+    int32_t kid, skip;          // the child that holds it, and that child's rows before it
 };
 
 struct Level {
@@ -98,27 +99,68 @@ __device__ __forceinline__ int32_t child(const IdentifyArgs& a, int32_t P, int j
     return c0 == a.child_ptr[P + 1] ? P : a.child_idx[c0 + j];
 }
 
+__device__ __forceinline__ int64_t child_rows(const IdentifyArgs& a, int32_t P, int j) {
+    const int32_t c = child(a, P, j);
+    return a.node_rows[c + 1] - a.node_rows[c];
+}
+
+// Places for the items of a parent of `rows` rows and m entries: the first, or -1 where they do not fit.
+__device__ __forceinline__ int64_t take_items(const Level& v, int64_t rows, int32_t m) {
+    const int64_t n = (rows + kN - 1) / kN * ((m + kM - 1) / kM);
+    if (n <= v.max_items && rows <= 0x7fffffff) {
+        const int64_t x = (int64_t)atomicAdd(v.counters + kCntItems, (unsigned long long)n);
+        if (x + n <= v.max_items) return x;
+    }
+    *v.flag = v.L + 1;
+    return -1;
+}
+
+// The items of the row chunks that start in child j, whose rows are s .. s + m_rows - 1 of its parent's; x is the parent's
+// first.  The entry tiles of one chunk stand side by side: they read the same rows at about the same time.
+__device__ __forceinline__ void put_items(const Level& v, int64_t x, int32_t slot, int32_t m, int j, int64_t s, int64_t m_rows) {
+    const int32_t tiles = (m + kM - 1) / kM;
+    for (int64_t c = (s + kN - 1) / kN; c * kN < s + m_rows; ++c)
+        for (int32_t t = 0; t < tiles; ++t)
+            v.items[x + c * tiles + t] = Item{slot, t * kM, min(kM, m - t * kM), (int32_t)(c * kN), j, (int32_t)(c * kN - s)};
+}
+
+// A parent of a few children, by one thread ...
+constexpr int kThreadChildren = 32;
 __device__ __forceinline__ void add_items(const Level& v, int32_t slot, int32_t P, int32_t m) {
     int64_t rows = 0;
     const int nch = n_children(v.a, P);
+    for (int j = 0; j < nch; ++j) rows += child_rows(v.a, P, j);
+    const int64_t x = take_items(v, rows, m);
+    if (x < 0) return;
+    int64_t s = 0;
     for (int j = 0; j < nch; ++j) {
-        const int32_t c = child(v.a, P, j);
-        rows += v.a.node_rows[c + 1] - v.a.node_rows[c];
+        const int64_t r = child_rows(v.a, P, j);
+        put_items(v, x, slot, m, j, s, r);
+        s += r;
     }
-    const int64_t chunks = (rows + kN - 1) / kN, n = chunks * ((m + kM - 1) / kM);
-    if (n > v.max_items || rows > 0x7fffffff) {
-        *v.flag = v.L + 1;
-        return;
+}
+
+// ... and of many, by a warp, 32 children at a time (a flat tree of 300,000 roots would keep one thread for seconds).
+__device__ __forceinline__ void add_items_wide(const Level& v, int32_t slot, int32_t P, int32_t m, int lane) {
+    int64_t rows = 0;
+    const int nch = n_children(v.a, P);
+    for (int j = lane; j < nch; j += 32) rows += child_rows(v.a, P, j);
+    for (int o = 16; o; o >>= 1) rows += __shfl_xor_sync(0xffffffffu, rows, o);
+    int64_t x = lane == 0 ? take_items(v, rows, m) : 0;
+    x = __shfl_sync(0xffffffffu, x, 0);
+    if (x < 0) return;
+    int64_t s = 0;
+    for (int j0 = 0; j0 < nch; j0 += 32) {
+        const int j = j0 + lane;
+        const int64_t r = j < nch ? child_rows(v.a, P, j) : 0;
+        int64_t upto = r;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += y;
+        }
+        put_items(v, x, slot, m, j, s + upto - r, r);
+        s += __shfl_sync(0xffffffffu, upto, 31);
     }
-    const int64_t x = (int64_t)atomicAdd(v.counters + kCntItems, (unsigned long long)n);
-    if (x + n > v.max_items) {
-        *v.flag = v.L + 1;
-        return;
-    }
-    // the entry tiles of one row chunk side by side: they read the same rows at about the same time
-    int64_t i = x;
-    for (int64_t c = 0; c < chunks; ++c)
-        for (int32_t e = 0; e < m; e += kM) v.items[i++] = Item{slot, e, min(kM, m - e), (int32_t)(c * kN)};
 }
 
 __global__ void read_norms_kernel(const Level v) {
@@ -189,16 +231,27 @@ __global__ void entries_kernel(const Level v) {
 // each parent's places in the entry list, and its items; level 0: the roots' (the entries are the reads in order)
 __global__ void parents_kernel(const Level v) {
     const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (*v.flag) return;
+    const int lane = threadIdx.x & 31;
+    if (__shfl_sync(0xffffffffu, lane == 0 ? *v.flag : 0, 0)) return;  // (it may rise meanwhile)
+    int32_t slot = -1, P = -1, m = 0;
     if (v.L == 0) {
-        if (h == 0) add_items(v, -1, -1, (int32_t)v.nq);
-        return;
+        if (h == 0) m = (int32_t)v.nq;
+    } else if (h < v.table) {
+        m = v.tab_cnt[h];
+        if (m) {
+            slot = (int32_t)h;
+            P = v.tab_key[h];
+            v.tab_off[h] = (int32_t)atomicAdd(v.counters + kCntEntries, (unsigned long long)m);
+        }
     }
-    if (h >= v.table) return;
-    const int32_t m = v.tab_cnt[h];
-    if (!m) return;
-    v.tab_off[h] = (int32_t)atomicAdd(v.counters + kCntEntries, (unsigned long long)m);
-    add_items(v, (int32_t)h, v.tab_key[h], m);
+    const bool wide = m && n_children(v.a, P) > kThreadChildren;
+    if (m && !wide) add_items(v, slot, P, m);
+    __syncwarp();
+    for (uint32_t w = __ballot_sync(0xffffffffu, wide); w; w &= w - 1) {
+        const int from = __ffs(w) - 1;
+        add_items_wide(v, __shfl_sync(0xffffffffu, slot, from), __shfl_sync(0xffffffffu, P, from),
+                       __shfl_sync(0xffffffffu, m, from), lane);
+    }
 }
 
 __global__ void scatter_kernel(const Level v) {
@@ -471,10 +524,10 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
             // ... and rows: the candidate that holds row item.col0 + c of the parent's
             const int nch = n_children(a, P);
             for (int c = row; c < kN; c += kM) {
-                int64_t left = (int64_t)item.col0 + c;
+                int64_t left = (int64_t)item.skip + c;
                 int32_t kid = -1;
                 int64_t j = 0;
-                for (int i = 0; i < nch; ++i) {
+                for (int i = item.kid; i < nch; ++i) {
                     const int32_t node = child(a, P, i);
                     const int64_t r0 = a.node_rows[node], m = a.node_rows[node + 1] - r0;
                     if (left < m) {

@@ -98,3 +98,24 @@ def test_a_wait_that_runs_out_leaves_the_results_right(hdc, orc, cuda):
     ctx.option(hdc.WAIT_LIMIT, 0)
     assert _check(hdc, orc, cuda, ctx, q, rows, tree, 3, 5, -2.0, 0) == 0
     assert ctx.status() == 0
+
+
+# children counted by a thread (to 32) and by a warp, with none, a few or many rows each (several children a row chunk, and
+# several chunks a child), at the roots and below; the last child empty
+@pytest.mark.parametrize("branches", [[32], [33], [1000], [2, 33], [3, 200], [40, 5], [70, 40]])
+def test_wide_parents(hdc, orc, cuda, branches):
+    per = lambda rank, node: 0 if node % 5 == 4 else 500 if node % 31 == 7 else node % 4
+    g, tree, rows, q = _inputs(len(branches) + branches[0], branches, 72, 200, per)
+    ctx = hdc.Context(72, 8, 150, 10)
+    reads = np.arange(0, 200, 1 if len(rows) < 3000 else 9)
+    assert _check(hdc, orc, cuda, ctx, q, rows, tree, len(branches), 3, -2.0, 0, reads) == 0
+    assert ctx.status() == 0
+
+
+def test_a_flat_tree_of_many_roots(hdc, orc, cuda):
+    """The time that an item's tables take does not grow with the number of roots: within short waits, 100,000 of them."""
+    g, tree, rows, q = _inputs(1, [100000], 64, 160, lambda rank, node: 1)
+    ctx = hdc.Context(64, 8, 150, 10)
+    ctx.option(hdc.WAIT_LIMIT, 3000)  # 3 million cycles, 1.5 ms
+    assert _check(hdc, orc, cuda, ctx, q, rows, tree, 1, 5, -2.0, 0, [0, 63, 159]) == 0
+    assert ctx.status() == 0
