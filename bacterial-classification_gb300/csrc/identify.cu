@@ -273,7 +273,7 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
         return fail(HDC_ERR_INVALID, "identify: dim must be a multiple of 8 and rows 16-byte aligned");
     const size_t smem = (size_t)ctx->dim * sizeof(int16_t);
     if (smem > 200 * 1024) return fail(HDC_ERR_INVALID, "identify: dim too large for a shared-memory query");
-    if (smem > 48 * 1024) {
+    if (smem > 46 * 1024) {  // with the kernel's own shared memory, more than the 48 KiB that a launch has by default
         cudaError_t e = cudaFuncSetAttribute(identify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return cuda_fail(e, "identify: shared memory attribute");
     }

@@ -119,3 +119,13 @@ def test_a_flat_tree_of_many_roots(hdc, orc, cuda):
     ctx.option(hdc.WAIT_LIMIT, 3000)  # 3 million cycles, 1.5 ms
     assert _check(hdc, orc, cuda, ctx, q, rows, tree, 1, 5, -2.0, 0, [0, 63, 159]) == 0
     assert ctx.status() == 0
+
+
+@pytest.mark.parametrize("dim", [23960, 24216, 24224, 24576, 24584, 102400])
+def test_reads_near_the_default_shared_memory(hdc, orc, cuda, dim):
+    """A read beside the kernel's own shared memory, around the 48 KiB that a launch may take without asking, and the most."""
+    g, tree, rows, q = _inputs(1, [3, 2], dim, 5, lambda rank, node: 2, 9)
+    rows[0, 0] = 2049  # not for the tensor cores
+    ctx = hdc.Context(dim, 8, 150, 10)
+    assert _check(hdc, orc, cuda, ctx, q, rows, tree, 2, 3, -2.0, 0) == 1
+    assert ctx.status() == 0
