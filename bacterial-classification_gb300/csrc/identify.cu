@@ -36,7 +36,8 @@ constexpr int kMaxBeam = kIdBeam;
 constexpr int kMaxLevels = kIdLevels;
 constexpr int kIdWarps = 8;
 constexpr int kSimWarps = 8;
-constexpr int64_t kIdBatch = 65536;  // reads of a grouped pass
+constexpr int64_t kIdBatch = 65536;  // reads of a grouped pass ...
+constexpr int64_t kIdRootPairs = 256 << 20;  // ... and its reads times roots: a pass keeps a word for each (1 GiB)
 
 // exact dot of an int16 row (global) with an int16 vector (shared or global),
 // one warp; dim % 8 == 0 and both 16-byte aligned.  NARROW: every partial sum
@@ -278,17 +279,22 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
         if (e != cudaSuccess) return cuda_fail(e, "identify: shared memory attribute");
     }
     // Batches of reads grouped by parent on the tensor cores, each followed by the per-read kernel, which goes on from the
-    // level that does not fit there (and exits at once if all did).  A few reads with one beam row each, a CTA a read, wait as long for their
-    // own gathers as for the grouped form's five launches a level: 17 reads, D = 1,024, 233 us against 251; 30, D = 2,048,
-    // 291 against 299 (10 reads with three rows each: 865 against 293).
+    // level that does not fit there (and exits at once if all did).  A few reads with one beam row each, a CTA a read, wait
+    // as long for their own gathers as for the grouped form's five launches a level: 17 reads, D = 1,024, 233 us against
+    // 251; 30, D = 2,048, 291 against 299 (10 reads with three rows each: 865 against 293).
     const bool few = nq <= ctx->num_sms && beam == 1 && ctx->dim <= 2048;
-    for (int64_t r0 = 0; r0 < nq; r0 += kIdBatch) {
-        const int64_t n = std::min(kIdBatch, nq - r0);
+    // passes of about as many reads each, in whole items of 128; too many roots even for one item of reads: none
+    const int64_t most = std::min(kIdBatch, kIdRootPairs / std::max(n_roots, 1) / 128 * 128);
+    const bool grouped = !few && most > 0;
+    const int64_t passes = (nq + (grouped ? most : kIdBatch) - 1) / (grouped ? most : kIdBatch);
+    const int64_t step = ((nq + passes - 1) / passes + 127) / 128 * 128;
+    for (int64_t r0 = 0; r0 < nq; r0 += step) {
+        const int64_t n = std::min(step, nq - r0);
         IdentifyArgs a{d_q + r0 * ctx->dim, d_qn + r0, d_rows, d_rn, d_node_rows, d_child_ptr, d_child_idx, d_roots, n_roots,
                        ctx->dim, levels, beam, mode, threshold, d_path + r0 * levels, d_path_score + r0 * levels,
                        d_depth + r0, d_stop_level ? d_stop_level + r0 : nullptr, ctx->d_id_form, {}};
         void* ws = nullptr;
-        const int st = few ? HDC_OK : launch_identify_grouped(ctx, a, n, &a.from, &ws, stream);
+        const int st = grouped ? launch_identify_grouped(ctx, a, n, &a.from, &ws, stream) : HDC_OK;
         if (st != HDC_OK) return st;
         identify_kernel<<<(unsigned)n, 32 * kIdWarps, smem, stream>>>(a);
         cudaError_t e = cudaGetLastError();

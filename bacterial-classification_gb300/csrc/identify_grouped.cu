@@ -140,25 +140,37 @@ __device__ __forceinline__ void add_items(const Level& v, int32_t slot, int32_t 
     }
 }
 
-// ... and of many, by a warp, 32 children at a time (a flat tree of 300,000 roots would keep one thread for seconds).
+// ... and of many, by a warp, 8 a lane at a time, whose look-ups overlap (a flat tree of 300,000 roots would keep one thread
+// for seconds).
+constexpr int kLaneChildren = 8;
 __device__ __forceinline__ void add_items_wide(const Level& v, int32_t slot, int32_t P, int32_t m, int lane) {
     int64_t rows = 0;
     const int nch = n_children(v.a, P);
+#pragma unroll 8
     for (int j = lane; j < nch; j += 32) rows += child_rows(v.a, P, j);
     for (int o = 16; o; o >>= 1) rows += __shfl_xor_sync(0xffffffffu, rows, o);
     int64_t x = lane == 0 ? take_items(v, rows, m) : 0;
     x = __shfl_sync(0xffffffffu, x, 0);
     if (x < 0) return;
     int64_t s = 0;
-    for (int j0 = 0; j0 < nch; j0 += 32) {
-        const int j = j0 + lane;
-        const int64_t r = j < nch ? child_rows(v.a, P, j) : 0;
-        int64_t upto = r;
+    for (int j0 = 0; j0 < nch; j0 += 32 * kLaneChildren) {
+        const int j = j0 + lane * kLaneChildren;
+        int64_t r[kLaneChildren], sum = 0;
+#pragma unroll
+        for (int u = 0; u < kLaneChildren; ++u) r[u] = j + u < nch ? child_rows(v.a, P, j + u) : 0;
+#pragma unroll
+        for (int u = 0; u < kLaneChildren; ++u) sum += r[u];
+        int64_t upto = sum;
         for (int o = 1; o < 32; o <<= 1) {
             const int64_t y = __shfl_up_sync(0xffffffffu, upto, o);
             if (lane >= o) upto += y;
         }
-        put_items(v, x, slot, m, j, s + upto - r, r);
+        int64_t at = s + upto - sum;
+#pragma unroll
+        for (int u = 0; u < kLaneChildren; ++u) {
+            put_items(v, x, slot, m, j + u, at, r[u]);
+            at += r[u];
+        }
         s += __shfl_sync(0xffffffffu, upto, 31);
     }
 }

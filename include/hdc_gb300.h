@@ -461,15 +461,20 @@ int hdc_similarity(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2
  * hdc_beam_search, plus d_stop_level [nq] (may be NULL): the level at which
  * the read stopped because its best score fell below the threshold, or -1
  * when it ran all levels.  levels <= 8; beam <= 8; dim % 8 == 0;
- * dim * 2 bytes <= 200 KiB. */
+ * dim * 2 bytes <= 200 KiB.  The squared norms must be those of the rows
+ * (hdc_norms): the exactness of a dot's partial sums is judged by them.
+ * Reads go in passes of up to 65,536, whose workspace (up to some 1.1 GB) comes
+ * from a pool that the device's contexts share and that keeps up to 512 MB until
+ * the last of them is destroyed; a pass without room for it runs one CTA a read,
+ * and so does a call with more than 2,097,152 roots. */
 int hdc_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, int64_t nq, const int16_t* d_rows,
                  const int64_t* d_row_norm2, const int64_t* d_node_rows, const int64_t* d_child_ptr,
                  const int32_t* d_child_idx, const int32_t* d_roots, int n_roots, int levels, int beam,
                  double threshold, int score_mode, int32_t* d_path, float* d_path_score, int32_t* d_depth,
                  int32_t* d_stop_level, void* stream);
 
-/* How the last hdc_identify on this context ran, its last 65,536 reads where it
- * took several passes (diagnostic; synchronizes the device): 0 grouped by
+/* How the last hdc_identify on this context ran, its last pass where it took
+ * several (diagnostic; synchronizes the device): 0 grouped by
  * parent on the tensor cores, l > 0 the same down to level l - 1, from which one
  * CTA a read went on, HDC_IDENTIFY_PER_READ one CTA a read from the start (0
  * before the first). */

@@ -33,7 +33,7 @@ def _check(hdc, orc, cuda, ctx, q, rows, tree, levels, beam, threshold, mode, re
     got = ctx.identify(tq, qn, tr, rn, t(node_rows), t(ptr), t(idx), torch.tensor(roots, dtype=torch.int32, device=cuda),
                        levels, beam, threshold, mode)
     path, score, depth, stop = (x.cpu().numpy() for x in got)
-    at = np.arange(len(q)) if reads is None else np.asarray(reads)
+    at = np.arange(len(q)) if reads is None else np.asarray(reads, np.int64)
     want = orc.identify(q[at], rows, node_rows, ptr, idx, roots, levels, beam, threshold, mode)
     for i, (wp, ws, wstop) in zip(at, want):
         assert depth[i] == len(wp), i
@@ -128,4 +128,16 @@ def test_reads_near_the_default_shared_memory(hdc, orc, cuda, dim):
     rows[0, 0] = 2049  # not for the tensor cores
     ctx = hdc.Context(dim, 8, 150, 10)
     assert _check(hdc, orc, cuda, ctx, q, rows, tree, 2, 3, -2.0, 0) == 1
+    assert ctx.status() == 0
+
+
+@pytest.mark.parametrize("roots,nq,reads,form", [
+    (70000, 4000, [0, 2047, 2048, 3999], 0),  # two passes of 2,048 and 1,952 reads (a pass keeps 256 Mi reads times roots)
+    (2097153, 160, [], -1),                   # more roots than that holds for 128 reads: one CTA a read
+])
+def test_passes_bounded_by_the_roots(hdc, orc, cuda, roots, nq, reads, form):
+    dim = 64 if reads else 8
+    g, tree, rows, q = _inputs(2, [roots], dim, nq, lambda rank, node: 1)
+    ctx = hdc.Context(dim, 8, 150, 10)
+    assert _check(hdc, orc, cuda, ctx, q, rows, tree, 1, 3, -2.0, 0, reads) == form
     assert ctx.status() == 0
