@@ -554,16 +554,26 @@ int hdc_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, 
                  const int32_t* d_child_idx, const int32_t* d_roots, int n_roots, int levels, int beam,
                  double threshold, int score_mode, int32_t* d_path, float* d_path_score, int32_t* d_depth,
                  int32_t* d_stop_level, void* stream) {
+    return hdc_identify_sized(ctx, d_q, d_qnorm2, nq, d_rows, d_row_norm2, 0, d_node_rows, 0, d_child_ptr, d_child_idx,
+                              d_roots, n_roots, levels, beam, threshold, score_mode, d_path, d_path_score, d_depth,
+                              d_stop_level, stream);
+}
+
+int hdc_identify_sized(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, int64_t nq, const int16_t* d_rows,
+                       const int64_t* d_row_norm2, int64_t n_rows, const int64_t* d_node_rows, int64_t n_nodes,
+                       const int64_t* d_child_ptr, const int32_t* d_child_idx, const int32_t* d_roots, int n_roots,
+                       int levels, int beam, double threshold, int score_mode, int32_t* d_path, float* d_path_score,
+                       int32_t* d_depth, int32_t* d_stop_level, void* stream) {
     if (!ctx) return fail(HDC_ERR_INVALID, "identify: null context");
-    if (nq < 0) return fail(HDC_ERR_INVALID, "identify: negative count");
+    if (nq < 0 || n_rows < 0 || n_nodes < 0) return fail(HDC_ERR_INVALID, "identify: negative count");
     if (nq == 0) return HDC_OK;
     if (!hdc::valid_score_mode(score_mode)) return fail(HDC_ERR_INVALID, "identify: bad score mode");
     if (!d_q || !d_qnorm2 || !d_rows || !d_row_norm2 || !d_node_rows || !d_child_ptr || !d_child_idx ||
         (n_roots > 0 && !d_roots) || !d_path || !d_path_score || !d_depth)
         return fail(HDC_ERR_INVALID, "identify: null pointer");
-    return hdc::launch_identify(ctx, d_q, d_qnorm2, nq, d_rows, d_row_norm2, d_node_rows, d_child_ptr, d_child_idx,
-                                d_roots, n_roots, levels, beam, threshold, score_mode, d_path, d_path_score, d_depth,
-                                d_stop_level, static_cast<cudaStream_t>(stream));
+    return hdc::launch_identify(ctx, d_q, d_qnorm2, nq, d_rows, d_row_norm2, n_rows, d_node_rows, n_nodes, d_child_ptr,
+                                d_child_idx, d_roots, n_roots, levels, beam, threshold, score_mode, d_path, d_path_score,
+                                d_depth, d_stop_level, static_cast<cudaStream_t>(stream));
 }
 
 int hdc_fasta_parse(hdc_context* ctx, const char* d_in, int64_t n, char* d_out, int64_t* d_seq_off,

@@ -151,9 +151,10 @@ int launch_beam_search(hdc_context* ctx, const int8_t* d_q, const uint32_t* d_qb
                        int levels, int beam, double threshold, int mode, int32_t* d_path, float* d_path_score,
                        int32_t* d_depth, cudaStream_t stream);
 
+// (n_nodes 0: the sizes are not known)
 int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, int64_t nq, const int16_t* d_rows,
-                    const int64_t* d_rn, const int64_t* d_node_rows, const int64_t* d_child_ptr,
-                    const int32_t* d_child_idx, const int32_t* d_roots, int n_roots, int levels, int beam,
+                    const int64_t* d_rn, int64_t n_rows, const int64_t* d_node_rows, int64_t n_nodes,
+                    const int64_t* d_child_ptr, const int32_t* d_child_idx, const int32_t* d_roots, int n_roots, int levels, int beam,
                     double threshold, int mode, int32_t* d_path, float* d_path_score, int32_t* d_depth,
                     int32_t* d_stop_level, cudaStream_t stream);
 

@@ -258,11 +258,42 @@ bool rows_ok(const hdc_context* ctx, const void* q, const void* rows) {
     return ctx->dim % 8 == 0 && !(reinterpret_cast<uintptr_t>(q) & 15) && !(reinterpret_cast<uintptr_t>(rows) & 15);
 }
 
+// Microseconds that one CTA a read and the grouped form take, for the choice between them: the one grows with the
+// candidates and rows that a read meets, the other is a handful of launches a level however few they are.  The tree's sizes
+// give its average branching and rows a node.  As measured on trees of 10 to 1,092 nodes of 1 to 150 rows: a candidate
+// takes 1.5 us and 2.5-3.8 for every 8 of its rows (a CTA's warps), D = 1,024-8,192, and beyond a CTA an SM the batch
+// some 1 / 700 longer with each read; a grouped level 40 us and 0.55 a K block of 64 dims.  8 reads over 14 nodes of 3 rows,
+// beam 1, D = 8,192: 59 us against 267; 152 reads, beam 5, D = 1,024: 66 against 167; 4,096: 388 against 190.
+struct IdTimes {
+    double per_read, grouped;
+};
+IdTimes id_times(const hdc_context* ctx, int64_t nq, int64_t n_nodes, int64_t n_rows, int n_roots, int levels, int beam) {
+    const double roots = std::max(n_roots, 1), dim = ctx->dim;
+    auto nodes_of = [&](double b) {
+        double sum = 0, rank = roots;
+        for (int l = 0; l < levels; ++l, rank *= b) sum += rank;
+        return sum;
+    };
+    double lo = 1, hi = (double)n_nodes;  // children a node, a childless one counted as its own
+    for (int i = 0; i < 50 && levels > 1; ++i) {
+        const double b = 0.5 * (lo + hi);
+        (nodes_of(b) <= (double)n_nodes ? lo : hi) = b;
+    }
+    double met = roots, rank = roots;
+    for (int l = 1; l < levels; ++l) {
+        rank *= lo;
+        met += std::min(rank, beam * lo);
+    }
+    const double eights = std::max<int64_t>(1, (n_rows + 8 * n_nodes - 1) / (8 * n_nodes));
+    const double crowd = 1 + (double)std::max<int64_t>(0, nq - ctx->num_sms) / 700;
+    return {(15 + met * (1.5 + eights * (2.5 + 1.6e-4 * dim))) * crowd, 20 + levels * (40 + 0.55 / 64 * dim)};
+}
+
 }  // namespace
 
 int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, int64_t nq, const int16_t* d_rows,
-                    const int64_t* d_rn, const int64_t* d_node_rows, const int64_t* d_child_ptr,
-                    const int32_t* d_child_idx, const int32_t* d_roots, int n_roots, int levels, int beam,
+                    const int64_t* d_rn, int64_t n_rows, const int64_t* d_node_rows, int64_t n_nodes,
+                    const int64_t* d_child_ptr, const int32_t* d_child_idx, const int32_t* d_roots, int n_roots, int levels, int beam,
                     double threshold, int mode, int32_t* d_path, float* d_path_score, int32_t* d_depth,
                     int32_t* d_stop_level, cudaStream_t stream) {
     if (nq == 0) return HDC_OK;
@@ -281,8 +312,15 @@ int launch_identify(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qn, i
     // Batches of reads grouped by parent on the tensor cores, each followed by the per-read kernel, which goes on from the
     // level that does not fit there (and exits at once if all did).  A few reads with one beam row each, a CTA a read, wait
     // as long for their own gathers as for the grouped form's five launches a level: 17 reads, D = 1,024, 233 us against
-    // 251; 30, D = 2,048, 291 against 299 (10 reads with three rows each: 865 against 293).
-    const bool few = nq <= ctx->num_sms && beam == 1 && ctx->dim <= 2048;
+    // 251; 30, D = 2,048, 291 against 299 (10 reads with three rows each: 865 against 293; without a tree's sizes there is no
+    // telling the many that lose from the many that gain: 12 candidates of 150 rows, D = 1,024, 605 against 224, 6 of 3
+    // rows 46 against 142).  With them the estimates decide, and in that corner the per-read one may be 2.5 times the
+    // other, as it takes every node to have the average's rows and most of them are leaves'.
+    bool few = nq <= ctx->num_sms && beam == 1 && ctx->dim <= 2048;
+    if (n_nodes > 0) {
+        const IdTimes t = id_times(ctx, nq, n_nodes, n_rows, n_roots, levels, beam);
+        few = t.per_read <= t.grouped * (few ? 2.5 : 1.0);
+    }
     // passes of about as many reads each, in whole items of 128; too many roots even for one item of reads: none
     const int64_t most = std::min(kIdBatch, kIdRootPairs / std::max(n_roots, 1) / 128 * 128);
     const bool grouped = !few && most > 0;

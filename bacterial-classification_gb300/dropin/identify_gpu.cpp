@@ -182,10 +182,10 @@ int main(int argc, char** argv) {
         upload(d_cp, child_ptr);
         upload(d_ci, child_idx);
         upload(d_roots, root_ids);
-        check(hdc_identify(ctx, d_q.as<int16_t>(), d_qn.as<int64_t>(), nq, d_rows.as<int16_t>(), d_rn.as<int64_t>(),
-                           d_nrows.as<int64_t>(), d_cp.as<int64_t>(), d_ci.as<int32_t>(), d_roots.as<int32_t>(),
-                           (int)root_ids.size(), kLevels, kBeam, kThreshold, HDC_SCORE_NORM, d_path.as<int32_t>(),
-                           d_ps.as<float>(), d_depth.as<int32_t>(), d_stop.as<int32_t>(), nullptr),
+        check(hdc_identify_sized(ctx, d_q.as<int16_t>(), d_qn.as<int64_t>(), nq, d_rows.as<int16_t>(), d_rn.as<int64_t>(),
+                                 nr, d_nrows.as<int64_t>(), (int64_t)nodes.size(), d_cp.as<int64_t>(), d_ci.as<int32_t>(),
+                                 d_roots.as<int32_t>(), (int)root_ids.size(), kLevels, kBeam, kThreshold, HDC_SCORE_NORM,
+                                 d_path.as<int32_t>(), d_ps.as<float>(), d_depth.as<int32_t>(), d_stop.as<int32_t>(), nullptr),
               "identify");
         check(hdc_copy(path.data(), d_path.p, path.size() * 4, 0, nullptr), "copy");
         check(hdc_copy(path_score.data(), d_ps.p, path.size() * 4, 0, nullptr), "copy");

@@ -54,6 +54,8 @@ SIGNATURES = [
                                          ctypes.c_double, I32, P, P, P, P]),
     ("hdc_similarity", I32, [P, P, P, P, P, P, P, P, P, I64, I32, P, P, P]),
     ("hdc_identify", I32, [P, P, P, I64, P, P, P, P, P, P, I32, I32, I32, ctypes.c_double, I32, P, P, P, P, P]),
+    ("hdc_identify_sized", I32, [P, P, P, I64, P, P, I64, P, I64, P, P, P, I32, I32, I32, ctypes.c_double, I32, P, P, P, P,
+                                 P]),
     ("hdc_identify_last_form", I32, [P, ctypes.POINTER(ctypes.c_int)]),
     ("hdc_propagate_greedy", I32, [P, P, P, P, P, P, P, I64, ctypes.c_double, I32, P, P, P, P]),
     ("hdc_context_status", I32, [P, ctypes.POINTER(ctypes.c_int)]),
@@ -346,9 +348,10 @@ class Context:
         score = torch.empty((nq, levels), dtype=torch.float32, device=q.device)
         depth = torch.empty(nq, dtype=torch.int32, device=q.device)
         stop = torch.empty(nq, dtype=torch.int32, device=q.device)
-        check(lib().hdc_identify(self.h, ptr(q), ptr(qn), nq, ptr(rows), ptr(rn), ptr(node_rows), ptr(child_ptr),
-                                 ptr(child_idx), ptr(roots), roots.numel(), levels, beam, threshold, mode, ptr(path),
-                                 ptr(score), ptr(depth), ptr(stop), stream_ptr(stream)))
+        check(lib().hdc_identify_sized(self.h, ptr(q), ptr(qn), nq, ptr(rows), ptr(rn), rows.shape[0], ptr(node_rows),
+                                       node_rows.numel() - 1, ptr(child_ptr), ptr(child_idx), ptr(roots), roots.numel(),
+                                       levels, beam, threshold, mode, ptr(path), ptr(score), ptr(depth), ptr(stop),
+                                       stream_ptr(stream)))
         return path, score, depth, stop
 
     def identify_last_form(self):

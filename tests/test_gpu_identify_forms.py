@@ -23,15 +23,24 @@ def _tree(branches, rows_of):
     return node_rows, np.array(ptr, np.int64), np.array(idx or [0], np.int32), list(range(branches[0])), base
 
 
-def _check(hdc, orc, cuda, ctx, q, rows, tree, levels, beam, threshold, mode, reads=None):
-    """Runs the descent and compares the reads (all of them by default) with the oracle; returns the form."""
+def _check(hdc, orc, cuda, ctx, q, rows, tree, levels, beam, threshold, mode, reads=None, sized=False):
+    """Runs the descent (without the tree's sizes: small trees run grouped too) and compares the reads (all of them by
+    default) with the oracle; returns the form."""
     import torch
     node_rows, ptr, idx, roots = tree[:4]
     t = lambda a: torch.from_numpy(a).to(cuda)
     tq, tr = t(q), t(rows)
     qn, rn = ctx.norms(tq), ctx.norms(tr)
-    got = ctx.identify(tq, qn, tr, rn, t(node_rows), t(ptr), t(idx), torch.tensor(roots, dtype=torch.int32, device=cuda),
-                       levels, beam, threshold, mode)
+    tables = [t(node_rows), t(ptr), t(idx), torch.tensor(roots, dtype=torch.int32, device=cuda)]
+    if sized:
+        got = ctx.identify(tq, qn, tr, rn, *tables, levels, beam, threshold, mode)
+    else:
+        i32 = dict(dtype=torch.int32, device=cuda)
+        got = (torch.empty((len(q), levels), **i32), torch.empty((len(q), levels), dtype=torch.float32, device=cuda),
+               torch.empty(len(q), **i32), torch.empty(len(q), **i32))
+        p = hdc.ptr
+        hdc.check(hdc.lib().hdc_identify(ctx.h, p(tq), p(qn), len(q), p(tr), p(rn), *(p(x) for x in tables), len(roots), levels,
+                                         beam, threshold, mode, *(p(x) for x in got), hdc.stream_ptr()))
     path, score, depth, stop = (x.cpu().numpy() for x in got)
     at = np.arange(len(q)) if reads is None else np.asarray(reads, np.int64)
     want = orc.identify(q[at], rows, node_rows, ptr, idx, roots, levels, beam, threshold, mode)
@@ -48,8 +57,9 @@ def _inputs(seed, branches, dim, nq, rows_of=lambda rank, node: 4 + node % 3, vm
     tree = _tree(branches, rows_of)
     rows = g.integers(-vmax, vmax + 1, (int(tree[0][-1]), dim)).astype(np.int16)
     q = g.integers(-vmax, vmax + 1, (nq, dim)).astype(np.int16)
-    near = g.integers(0, len(rows), nq)
-    q[::2] = np.clip(rows[near[::2]] // 2 + q[::2] // 2, -vmax, vmax)
+    near = g.integers(0, max(len(rows), 1), nq)
+    if len(rows):
+        q[::2] = np.clip(rows[near[::2]] // 2 + q[::2] // 2, -vmax, vmax)
     return g, tree, rows, q
 
 
@@ -140,4 +150,28 @@ def test_passes_bounded_by_the_roots(hdc, orc, cuda, roots, nq, reads, form):
     g, tree, rows, q = _inputs(2, [roots], dim, nq, lambda rank, node: 1)
     ctx = hdc.Context(dim, 8, 150, 10)
     assert _check(hdc, orc, cuda, ctx, q, rows, tree, 1, 3, -2.0, 0, reads) == form
+    assert ctx.status() == 0
+
+
+# few nodes of few rows, and the same with many reads; a few reads with one beam row over many rows; wide trees; a leaf root
+@pytest.mark.parametrize("branches,rows,dim,nq,beam,form", [
+    ([2, 2, 2], 3, 8192, 8, 1, -1),
+    ([2, 2, 2], 3, 1024, 152, 5, -1),
+    ([2, 2, 2], 3, 1024, 3000, 5, 0),
+    ([10], 1, 1024, 152, 5, -1),
+    ([10], 1, 1024, 3000, 5, 0),
+    ([1], 0, 64, 40, 1, -1),
+    ([3, 3, 3, 3], 150, 1024, 17, 1, 0),
+    ([3, 3, 3, 3, 3], 30, 1024, 17, 1, -1),
+    ([4, 4, 4], 20, 1024, 200, 5, 0),
+    ([5000], 1, 64, 20, 1, 0),
+])
+def test_the_sizes_of_a_tree_pick_the_form(hdc, orc, cuda, branches, rows, dim, nq, beam, form):
+    g, tree, r, q = _inputs(4, branches, dim, nq, lambda rank, node: rows, 60)
+    if not len(r):
+        r = np.zeros((1, dim), np.int16)
+    ctx = hdc.Context(dim, 8, 150, 10)
+    args = (hdc, orc, cuda, ctx, q, r, tree, len(branches), beam, -2.0, 0, np.arange(0, nq, max(1, nq // 20)))
+    assert _check(*args, sized=True) == form
+    _check(*args)
     assert ctx.status() == 0
