@@ -291,7 +291,7 @@ struct Tables {  // of one item
 };
 
 struct IdShared {
-    uint64_t raw[kStagesId], full[kStagesId], empty[kStagesId], accf[2], acce[2], tabf[2];
+    uint64_t raw[kStagesId], full[kStagesId], empty[kStagesId], accf[2], acce[2], tabf[2], drain;
     uint32_t tmem;
     int err;
     int n_items;  // read once a CTA: the flag may rise meanwhile, and the roles have to agree
@@ -363,6 +363,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
             tc::mbar_init(&sm.acce[b], 4);
             tc::mbar_init(&sm.tabf[b], kM / 32);
         }
+        tc::mbar_init(&sm.drain, 1);
         tc::fence_mbar_init();
     }
     if (warp == kMmaWarp) {
@@ -657,7 +658,9 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
     }
     tc::fence_before();
     __syncthreads();
+    if (warp == kMmaWarp && *err && tc::elect_one()) tc::mma_drain<false>(&sm.drain);
     if (warp == kMmaWarp) {
+        __syncwarp();
         tc::fence_after();
         tc::tmem_dealloc(tmem, 512);
     }

@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
-    __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], accf_bar[2], acce_bar[2];
+    __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], accf_bar[2], acce_bar[2], drain_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int err_s;
     __shared__ int seg_s[2];  // K blocks of a segment; MMAs of one, where less than a K block
@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
             tc::mbar_init(&accf_bar[b], 1);
             tc::mbar_init(&acce_bar[b], kDrainWarps * CL);  // each drain warp of the MMA's CTAs
         }
+        tc::mbar_init(&drain_bar, 1);
         tc::fence_mbar_init();
         tc::prefetch_tmap(&tmA);
         tc::prefetch_tmap(&tmB);
@@ -756,8 +757,10 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
 
     tc::fence_before();
     __syncthreads();
+    if (warp == 1 && crank == 0 && err_s && tc::elect_one()) tc::mma_drain<PAIR>(&drain_bar);
     if constexpr (PAIR) tc::cluster_sync();  // both CTAs are done with the pair's TMEM
     if (warp == 1) {
+        __syncwarp();
         tc::fence_after();
         if constexpr (PAIR)
             tc::tmem_dealloc_pair(tmem, 512);
@@ -794,7 +797,7 @@ __global__ void __launch_bounds__(kDotThreads, 1)
     constexpr uint32_t IDESC = F4 ? tc::idesc_f4_f32(kMmQueryTile, BN) : tc::idesc_f16_f32(kMmQueryTile, BN);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
-    __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], accf_bar[2], acce_bar[2];
+    __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], accf_bar[2], acce_bar[2], drain_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int err_s;
     const int stages = a.stages, stage_bytes = mm_stage_bytes(T::A_BYTES, T::B_BYTES, a.limbs);
@@ -809,6 +812,7 @@ __global__ void __launch_bounds__(kDotThreads, 1)
             tc::mbar_init(&accf_bar[b], 1);
             tc::mbar_init(&acce_bar[b], 4);
         }
+        tc::mbar_init(&drain_bar, 1);
         tc::fence_mbar_init();
         tc::prefetch_tmap(&tmA);
         tc::prefetch_tmap(&tmB);
@@ -951,7 +955,9 @@ __global__ void __launch_bounds__(kDotThreads, 1)
     }
     tc::fence_before();
     __syncthreads();
+    if (warp == 1 && err_s && tc::elect_one()) tc::mma_drain<false>(&drain_bar);
     if (warp == 1) {
+        __syncwarp();
         tc::fence_after();
         tc::tmem_dealloc(tmem, 512);
     }

@@ -359,6 +359,20 @@ __device__ __forceinline__ void mma_commit_pair_mc(uint64_t* bar, uint16_t cta_m
         : "memory");
 }
 
+// Wait (bounded) for every tcgen05.mma that this thread issued, on a barrier (count 1) kept for that: before a CTA some of
+// whose roles gave up, so that nobody waits for the accumulators any more, frees its tensor memory or leaves.  A pair's
+// issuer is its CTA 0.
+template <bool PAIR>
+__device__ __forceinline__ void mma_drain(uint64_t* bar) {
+    if constexpr (PAIR)
+        mma_commit_pair_mc(bar, 1);
+    else
+        mma_commit(bar);
+    const long long c0 = clock64();
+    while (!mbar_try_wait(smem_u32(bar), 0) && clock64() - c0 < kWaitCycles) {
+    }
+}
+
 // 32 consecutive 32-bit TMEM columns of this thread's lane.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
