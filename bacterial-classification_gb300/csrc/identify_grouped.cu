@@ -50,7 +50,7 @@ constexpr int kMaxChildren = 1 << 25;  // a warp's candidates sum to 2^30 at mos
 
 struct Item {
     int32_t slot, e0, n, col0;  // parent's table slot (-1: the roots), first entry and entries, first row
-    int32_t kid, skip;          // the child that holds it, and that child's rows before it
+    int32_t kid, skip;          // the child that its rows are counted from, and that child's first row to it
 };
 
 struct Level {
@@ -78,7 +78,8 @@ struct Level {
     uint32_t* best;       // [max_pairs] orderable score of each candidate, 0: nothing yet
     int64_t max_pairs;
     unsigned long long* counters;  // entries, items and pairs of the level (64 bits: what does not fit is still counted)
-    int32_t* flag;        // l + 1: leave level l and the ones after it to the per-read kernel
+    int32_t* flag;        // 1: leave this level and the ones after it to the per-read kernel ...
+    int32_t* from;        // ... which goes on from level *from - 1 (0: not at all), noted by the level's selection
     int* status;
     long long wait_cycles;
     int withhold;         // test hook: no rows are copied
@@ -111,12 +112,12 @@ __device__ __forceinline__ int64_t take_items(const Level& v, int64_t rows, int3
         const int64_t x = (int64_t)atomicAdd(v.counters + kCntItems, (unsigned long long)n);
         if (x + n <= v.max_items) return x;
     }
-    *v.flag = v.L + 1;
+    *v.flag = 1;
     return -1;
 }
 
-// The items of the row chunks that start in child j, whose rows are s .. s + m_rows - 1 of its parent's; x is the parent's
-// first.  The entry tiles of one chunk stand side by side: they read the same rows at about the same time.
+// The items of the row chunks that start in rows s .. s + m_rows - 1 of a parent, counted from its child j, which begins at
+// s; x is the parent's first.  The entry tiles of one chunk stand side by side: they read the same rows at about the same time.
 __device__ __forceinline__ void put_items(const Level& v, int64_t x, int32_t slot, int32_t m, int j, int64_t s, int64_t m_rows) {
     const int32_t tiles = (m + kM - 1) / kM;
     for (int64_t c = (s + kN - 1) / kN; c * kN < s + m_rows; ++c)
@@ -124,28 +125,20 @@ __device__ __forceinline__ void put_items(const Level& v, int64_t x, int32_t slo
             v.items[x + c * tiles + t] = Item{slot, t * kM, min(kM, m - t * kM), (int32_t)(c * kN), j, (int32_t)(c * kN - s)};
 }
 
-// A parent of a few children, by one thread ...
+// A parent of a few children, by one thread (its items' rows are all counted from the first child) ...
 constexpr int kThreadChildren = 32;
-__device__ __forceinline__ void add_items(const Level& v, int32_t slot, int32_t P, int32_t m) {
+__device__ __forceinline__ void add_items(const Level& v, int32_t slot, int32_t P, int32_t m, int nch) {
     int64_t rows = 0;
-    const int nch = n_children(v.a, P);
     for (int j = 0; j < nch; ++j) rows += child_rows(v.a, P, j);
     const int64_t x = take_items(v, rows, m);
-    if (x < 0) return;
-    int64_t s = 0;
-    for (int j = 0; j < nch; ++j) {
-        const int64_t r = child_rows(v.a, P, j);
-        put_items(v, x, slot, m, j, s, r);
-        s += r;
-    }
+    if (x >= 0) put_items(v, x, slot, m, 0, 0, rows);
 }
 
 // ... and of many, by a warp, 8 a lane at a time, whose look-ups overlap (a flat tree of 300,000 roots would keep one thread
 // for seconds).
 constexpr int kLaneChildren = 8;
-__device__ __forceinline__ void add_items_wide(const Level& v, int32_t slot, int32_t P, int32_t m, int lane) {
+__device__ __forceinline__ void add_items_wide(const Level& v, int32_t slot, int32_t P, int32_t m, int nch, int lane) {
     int64_t rows = 0;
-    const int nch = n_children(v.a, P);
 #pragma unroll 8
     for (int j = lane; j < nch; j += 32) rows += child_rows(v.a, P, j);
     for (int o = 16; o; o >>= 1) rows += __shfl_xor_sync(0xffffffffu, rows, o);
@@ -199,7 +192,7 @@ __global__ void entries_kernel(const Level v) {
         if (v.L > 0) P = v.paths[at(r, b, v.L - 1)];
         nch = n_children(v.a, P);
         if (nch > kMaxChildren) {
-            *v.flag = v.L + 1;
+            *v.flag = 1;
             nch = 0;
         }
     }
@@ -215,7 +208,7 @@ __global__ void entries_kernel(const Level v) {
     if (lane == 0 && total) p0 = (long long)atomicAdd(v.counters + kCntPairs, (unsigned long long)total);
     p0 = __shfl_sync(0xffffffffu, p0, 0);
     if (p0 + total > v.max_pairs) {
-        if (lane == 0) *v.flag = v.L + 1;
+        if (lane == 0) *v.flag = 1;
         return;  // the whole warp
     }
     if (!on) return;
@@ -256,13 +249,14 @@ __global__ void parents_kernel(const Level v) {
             v.tab_off[h] = (int32_t)atomicAdd(v.counters + kCntEntries, (unsigned long long)m);
         }
     }
-    const bool wide = m && n_children(v.a, P) > kThreadChildren;
-    if (m && !wide) add_items(v, slot, P, m);
+    const int nch = m ? n_children(v.a, P) : 0;
+    const bool wide = nch > kThreadChildren;
+    if (m && !wide) add_items(v, slot, P, m, nch);
     __syncwarp();
     for (uint32_t w = __ballot_sync(0xffffffffu, wide); w; w &= w - 1) {
         const int from = __ffs(w) - 1;
         add_items_wide(v, __shfl_sync(0xffffffffu, slot, from), __shfl_sync(0xffffffffu, P, from),
-                       __shfl_sync(0xffffffffu, m, from), lane);
+                       __shfl_sync(0xffffffffu, m, from), __shfl_sync(0xffffffffu, nch, from), lane);
     }
 }
 
@@ -466,7 +460,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
                 };
                 for (int i = 0; i < end_a; i += 4) four(i, end_a, n_ent);
                 for (int i = kTasksA; i < end_b; i += 4) four(i, end_b, kM + n_cols);
-                if (out) *v.flag = v.L + 1;
+                if (out) *v.flag = 1;
                 tc::fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&sm.full[stage]);
@@ -584,7 +578,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
                 double m[2] = {0, 0};
                 for (int w = 0; w < kM / 32; ++w)
                     for (int i = 0; i < 2; ++i) m[i] = fmax(m[i], (double)sm.norm_max[i][w]);
-                if (m[0] * m[1] > 281474976710656.0) *v.flag = v.L + 1;  // |q| |r| <= 2^24 for every pair of the item
+                if (m[0] * m[1] > 281474976710656.0) *v.flag = 1;  // |q| |r| <= 2^24 for every pair of the item
             }
             epi_sync();
             if (row == 0) t.seg[t.n_seg] = t.n_cols;
@@ -665,7 +659,7 @@ __global__ void __launch_bounds__(kThreadsId, 1) score_tc_kernel(const Level v) 
         tc::tmem_dealloc(tmem, 512);
     }
     if (tid == 0 && sm.err) {
-        *v.flag = v.L + 1;
+        *v.flag = 1;
         atomicCAS(v.status, 0, 100 + sm.err);
     }
 }
@@ -686,6 +680,7 @@ __global__ void select_kernel(const Level v) {
         }
         if (tid < kCounters) v.counters[tid] = 0;
     }
+    if (tid == 0 && *v.flag && *v.from == 0) *v.from = v.L + 1;
     if (r >= v.nq) return;
     if (__shfl_sync(0xffffffffu, lane == 0 ? v.done[r] | *v.flag : 0, 0)) return;
     const IdentifyArgs& a = v.a;
@@ -817,7 +812,8 @@ int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t 
     if (v.max_pairs > 0x7fffffff - 65536) return HDC_OK;
     auto carve_all = [&](uint8_t* base) {
         uint8_t* cur = base;
-        v.flag = carve<int32_t>(cur, 1);
+        v.flag = carve<int32_t>(cur, 2);
+        v.from = v.flag + 1;
         v.counters = carve<unsigned long long>(cur, kCounters);
         v.nbeam = carve<int32_t>(cur, nq);
         v.done = carve<int32_t>(cur, nq);
@@ -864,7 +860,7 @@ int launch_identify_grouped(hdc_context* ctx, const IdentifyArgs& args, int64_t 
         *workspace = nullptr;
         return cuda_fail(e, "identify: grouped launch");
     }
-    *from = IdentifyState{v.flag, v.done, v.nbeam, v.paths, v.scores};
+    *from = IdentifyState{v.from, v.done, v.nbeam, v.paths, v.scores};
     return HDC_OK;
 }
 
