@@ -1437,27 +1437,27 @@ struct MmPlan {
 // query tiles fill L2 about 5 % (60,000 references, 38,912 queries: 22.4 ms with 38 tiles a group, 23.6 with 152).
 MmPlan mm_plan(int sms, int64_t nq, int64_t nr, int dim, bool f4, int limbs) {
     MmPlan best;
-    const int64_t qt = (nq + kMmQueryTile - 1) / kMmQueryTile;
+    const int qt = (int)((nq + kMmQueryTile - 1) / kMmQueryTile);  // (32-bit divisions below: a call plans several times)
     const double steps = f4 ? (double)limbs * ((dim + 63) / 64) : (double)((dim + 15) / 16);
     double best_cost = 0;
     auto consider = [&](int CL, int n, double col_cycles) {
-        const int64_t rt = (nr + n - 1) / n;
+        const int rt = (int)((nr + n - 1) / n);
         const double tile = steps * n * col_cycles + 2500, row_bytes = f4 ? 0.5 * dim : 2.0 * dim;
-        const int64_t g_max = std::min<int64_t>(sms / CL * CL, (qt + CL - 1) / CL * CL);
-        for (int64_t G = CL; G <= g_max; G += CL) {
-            const int64_t S = std::min<int64_t>(std::min<int64_t>(sms / G, rt), 32 * kMergeHeads);
+        const int g_max = std::min(sms / CL * CL, (qt + CL - 1) / CL * CL);
+        for (int G = CL; G <= g_max; G += CL) {
+            const int S = std::min(std::min(sms / G, rt), 32 * kMergeHeads);
             if (S < 1) break;
-            const int64_t groups = (qt + G - 1) / G, tiles = (rt + S - 1) / S;
+            const int groups = (qt + G - 1) / G, tiles = (rt + S - 1) / S;
             const double in_l2 = std::min(1.0, (double)G * kMmQueryTile * row_bytes / 1e8);
             const double cost = (double)groups * ((double)tiles * tile + 20000) * (1 + 0.001 * (double)S + 0.05 * in_l2);
             if (best_cost == 0 || cost < best_cost) {
                 best_cost = cost;
                 best.CL = CL;
-                best.n_qtiles = (int)qt;
-                best.n_rtiles = (int)rt;
-                best.G = (int)G;
-                best.S = (int)S;
-                best.n_groups = (int)groups;
+                best.n_qtiles = qt;
+                best.n_rtiles = rt;
+                best.G = G;
+                best.S = S;
+                best.n_groups = groups;
             }
         }
     };
