@@ -81,8 +81,6 @@ CONFIGS = {
 #   grouped descent, c5 (one call's 5 descent_tc_kernel launches + the leaf-level score_kernel,
 #     38,912 reads): 3.64798e10 B with every row int32, 2.03567e10 B with int16 leaf rows
 TRAFFIC_SEARCH = {(38912, 200000): 116.88e9 + 22.80e6}  # (reads, references) -> bytes
-# block-scaled e2m1 MMAs (256 x 224 x 64, CTA pairs) on resident operands: the rate of the digits' search
-FP4_TFLOPS = 9160.0
 
 
 def base8_digits(max_abs):
@@ -261,8 +259,7 @@ class Form:
                     torch.empty((B, K), dtype=torch.int32, device=dev),
                     torch.empty((B, K), dtype=torch.float64, device=dev),
                     torch.empty((B, K), dtype=torch.int64, device=dev))
-        # encode, [norms], then (plain, one chunk of references) two conversions, norm tables, search, merge
-        self.launches = 6 if cfg["bipolar"] else 7
+        self.launches = 0  # kernels of a step, known after the first
         # the reference's NORM scale by default; --score-mode dot/cos for kernel studies
         self.mode = {"norm": H.SCORE_NORM, "cos": H.SCORE_COS, "dot": H.SCORE_DOT}[cfg.get("score_mode", "norm")]
 
@@ -274,11 +271,13 @@ class Form:
             ev[0].record(stream)
         if self.name == "tc":
             ctx.search_tc(self.db, self.q, qn, self.maxq, self.K, self.mode, work=self.work, out=self.out)
-            # encode, [norms], then the search kernels and merges the library reports (one or two parts)
-            self.launches = (1 if self.cfg["bipolar"] else 2) + ctx.tc_last_shape()[4]
+            search = ctx.tc_last_shape()[4]
         else:
             ctx.search_plain(self.q, qn, self.maxq, self.refs, self.rn, self.maxr, self.K, self.mode,
                              work=self.work, out=self.out)
+            search = ctx.plain_last_form()[1]
+        # encode, [norms], then the kernels that the library reports
+        self.launches = (1 if self.cfg["bipolar"] else 2) + search
         if ev is not None:
             ev[1].record(stream)
         return self.out
@@ -886,15 +885,20 @@ def run_reference(args, cfg):
     return float(np.median(vals)), threads, per_call
 
 
+def digits_roofline(achieved, digits, pk):
+    """Roofline keys of a search on base-8 digits: 2*D*R a read against the measured bf16 peak.  The fraction can pass 1: a
+    value's digits are block-scaled e2m1, which the tensor pipe takes at about four times bf16's rate."""
+    return {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
+            "frac": achieved / pk["bf16_tflops"], "digits": digits, "e2m1_tflops": achieved * digits}
+
+
 def batching_line(args, b, refs_host, pk):
     """The batching form measured inside the c3 run (same database): reads/s
     resident and end to end, its search's roofline, the autotuned schedule and
     the oracle's parity sample on the first reads of its batch."""
     cfg = b["cfg"]
     B = args.batch
-    digits = base8_digits(b["maxr"])
-    flops = 2.0 * cfg["dim"] * b["refs"] * digits * B
-    achieved = flops / (b["search_ms"] / 1e3) / 1e12
+    achieved = 2.0 * cfg["dim"] * b["refs"] * B / (b["search_ms"] / 1e3) / 1e12
     out = {"workload": "c4 reads on this database: log-normal lengths (median %d bp, sigma %.1f, %d-%d bp), %d%% "
                        "with %d%% sub:ins:del 3:1:1, top-%d, CUDA-graph encode -> search -> top-k" % (
                            cfg["read_len"], cfg["sigma"], cfg["min_read"], cfg["max_read"], 100 * cfg["mixed_frac"],
@@ -902,8 +906,7 @@ def batching_line(args, b, refs_host, pk):
            "value": B / (b["ms"] / 1e3), "unit": "reads/s", "batch_reads": B, "ms_per_step": b["ms"],
            "e2e": {"value": B / (b["e2e_ms"] / 1e3), "unit": "reads/s", "h2d_bytes_per_step": b["h2d"],
                    "d2h_bytes_per_step": b["d2h"]},
-           "search_roofline": {"bound": "tensor", "achieved": achieved, "peak": FP4_TFLOPS, "unit": "TFLOP/s",
-                               "frac": achieved / FP4_TFLOPS, "digits": digits},
+           "search_roofline": digits_roofline(achieved, base8_digits(b["maxr"]), pk),
            "autotuned_schedule": b["tuned"], "mean_read_len": b["mean_len"], "top1_accuracy": b["top1_accuracy"],
            "gpu_launches": b["launches"], "clocks": b["clocks"]}
     if refs_host is not None:
@@ -1325,19 +1328,17 @@ def main():
     value = B / (r["ms"] / 1e3)
     dim, nr = cfg["dim"], r["refs"]
     if args.form in ("tc", "pipe"):
-        # tensor work per read: 2*D*R, times the digits for +1/-1 reads (one e2m1 MMA step each)
+        # tensor work per read: 2*D*R (+1/-1 reads: in several digits a value, one e2m1 MMA step each)
         digits = base8_digits(r["maxr"]) if cfg["bipolar"] else 0
-        flops = 2.0 * dim * nr * max(1, digits) * B
-        achieved = flops / (r["search_ms"] / 1e3) / 1e12
-        peak = FP4_TFLOPS if digits else pk["bf16_tflops"]
-        roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                "frac": achieved / peak, "traffic": TRAFFIC_SEARCH.get((B, nr)),
-                "traffic_source": "ncu DRAM bytes of the search kernel of one call of this size",
-                "algorithmic_tflops": 2.0 * dim * nr * B / (r["search_ms"] / 1e3) / 1e12,
-                "peak_source": "block-scaled e2m1 MMAs on resident operands, measured" if digits else
-                               "%s dense bf16/fp16 burst (MEASURED_PEAKS.json)" % src,
-                "kernel": "mm_search_kernel + packing + merge; algorithmic 2*D*R per read" +
-                          (" for each of %d base-8 digits" % digits if digits else " on fp16 rows")}
+        achieved = 2.0 * dim * nr * B / (r["search_ms"] / 1e3) / 1e12
+        roof = digits_roofline(achieved, digits, pk) if digits else {
+            "bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
+            "frac": achieved / pk["bf16_tflops"]}
+        roof.update({"traffic": TRAFFIC_SEARCH.get((B, nr)),
+                     "traffic_source": "ncu DRAM bytes of the search kernel of one call of this size",
+                     "peak_source": "%s dense bf16/fp16 burst (MEASURED_PEAKS.json)" % src,
+                     "kernel": "mm_search_kernel + packing + merge; algorithmic 2*D*R per read" +
+                               (", in %d base-8 digits a value (block-scaled e2m1)" % digits if digits else " on fp16 rows")})
         dtype = ("e2m1 digits, block-scaled" if digits else "fp16 integers") + \
             ", fp32 accumulators (exact integer dots), FP64 scores"
     else:
