@@ -20,9 +20,12 @@
 // otherwise keeps the entries scoring >= threshold, at most `beam`
 // (:191-199).
 //
-// One CTA per read: the read's int16 hypervector is staged in shared memory
+// One CTA per read here: the read's int16 hypervector is staged in shared memory
 // once, and the CTA's warps split each candidate node's rows (coalesced
-// 16-byte loads of a row per warp step); dots are exact int64.
+// 16-byte loads of a row per warp step); dots are exact int64.  Batches of reads
+// are grouped by parent on the tensor cores instead (identify_grouped.cu) where
+// that is faster (launch_identify), and come back to this kernel at the level
+// that does not fit there.
 #include <algorithm>
 
 #include "hdc_internal.cuh"

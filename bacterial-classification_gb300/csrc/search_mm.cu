@@ -774,9 +774,9 @@ __global__ void __launch_bounds__(kThreadsMm, 1)
 // ---------------------------------------------------------------- small problems: the K loop split over CTAs
 // A problem with fewer tiles than SMs leaves most of them idle, and its time is one tile's K loop (157 K blocks of 330
 // cycles at D = 10,000, bound by the issuer's waits and commits) plus lists, thresholds and a merge made for thousands of
-// tiles.  Here the CTAs of a tile share its K blocks, each stores the whole dots of its part (at most 5 MB in all), and
-// one CTA a query adds the parts up and selects.  48 x 2,000 at D = 10,000: 80 -> 40 us with
-// its conversion; 190 x 567 at D = 1,024, top-32: 200 -> 36.
+// tiles.  Here the CTAs of a tile share its K blocks, each stores the whole dots of its part (at most a tile a CTA: 5 MB
+// in all on fp16 rows, 9 MB on digits), and one CTA a query adds the parts up and selects.  48 x 2,000 at D = 10,000:
+// 80 -> 40 us with its conversion; 190 x 567 at D = 1,024, top-32: 200 -> 36.
 constexpr int kDotThreads = 192;   // producer, MMA issuer, four drain warps
 constexpr int kSplitRefs = 12288;  // a query's dots and keys in shared memory
 constexpr int kMinSplitBlocks = 4; // K blocks that a CTA is worth starting for

@@ -5,14 +5,14 @@
 
 namespace hdc {
 
-// How a search's operands reach the tensor cores.  F16: queries and references as fp16 integers (|v| <= 2048),
-// row-major.  F4: +1/0/-1 queries and references split into balanced base-8 digits (-4 .. 4), both as packed e2m1
-// in the tile order of mm_pack_*; the digits' weights are the MMA's power-of-two scales.
 // Largest squared norms of a set of rows: of whole rows, and of any 64 dims of a K block.
 struct alignas(16) MmNorms {
     unsigned long long row, block;
 };
 
+// How a search's operands reach the tensor cores.  F16: queries and references as fp16 integers (|v| <= 2048),
+// row-major.  F4: +1/0/-1 queries and references split into balanced base-8 digits (-4 .. 4), both as packed e2m1
+// in the tile order of mm_pack_*; the digits' weights are the MMA's power-of-two scales.
 struct MmOperands {
     bool f4 = false;
     const void* a = nullptr;    // F16: [nq][lda] fp16; F4: mm_pack_queries' tiles

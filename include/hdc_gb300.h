@@ -174,9 +174,10 @@ size_t hdc_search_workspace_min_bytes(const hdc_context* ctx, int64_t nq, int64_
  * |element| of queries / references (from hdc_norms); products must satisfy
  * max_abs_q * max_abs_r <= 2^20 (else HDC_ERR_RANGE).  d_qnorm2 / d_rnorm2 come from hdc_norms.
  * d_work should hold hdc_search_workspace_bytes(nq, nr, k) bytes, 256-byte
- * aligned; it must hold hdc_search_workspace_min_bytes.  Rows of |v| <= 2048 (and +1/0/-1 queries against |r| <= 18724) are
- * converted in the workspace and searched on the tensor cores, exactly; larger
- * values take CUDA cores. */
+ * aligned; it must hold hdc_search_workspace_min_bytes.  Rows of |v| <= 2048
+ * (and +1/0/-1 queries against |r| <= 18724) are converted in the workspace and
+ * searched on the tensor cores, exactly, where the workspace is the full one and
+ * aligned; larger values take CUDA cores. */
 int hdc_search_plain(hdc_context* ctx, const int16_t* d_q, const int64_t* d_qnorm2, int64_t nq,
                      int32_t max_abs_q, const int16_t* d_r, const int64_t* d_rnorm2, int64_t nr,
                      int32_t max_abs_r, int k, int score_mode, float* d_score, int32_t* d_idx,
@@ -244,8 +245,14 @@ size_t hdc_search_tc_workspace_bytes(const hdc_context* ctx, const hdc_refdb* db
 
 /* Precision form: exact cosine top-k of fp16 integer queries (normally the
  * +1/-1 read hypervectors of HDC_OUT_BIPOLAR_F16, max_abs_q = 1) against a
- * tensor-core database, on tcgen05 tensor cores with fp32 accumulators per
- * limb (exact while dim * max|q| * max|limb| <= 2^24, else HDC_ERR_RANGE).
+ * tensor-core database, on tcgen05 tensor cores.  Queries for which the
+ * database has a search form (see hdc_refdb_create) run on it, in one exact
+ * fp32 accumulator a pair, emptied into integers where 2^24 would not hold a
+ * dot; the others on the limbs, with an accumulator each (exact while dim *
+ * max|q| * max|limb| <= 2^24, else HDC_ERR_RANGE, whichever form runs).
+ * max_abs_q must bound the queries' magnitudes (status 201 otherwise, on
+ * digits).  d_work: hdc_search_tc_workspace_bytes, 256-byte aligned; a smaller
+ * or unaligned one that holds the limb search's lists takes the limbs too.
  * Same ranking rule, outputs and score modes as hdc_search_plain, whose
  * results it reproduces exactly; the replacement for launch_cosine_topk
  * (src/cosine.cu:441-496) at scale. */
@@ -257,9 +264,12 @@ int hdc_search_tc(hdc_context* ctx, const hdc_refdb* db, const void* d_q, const 
 #define HDC_NOALLOC_SCRATCH_BYTES (16u << 20)
 
 /* hdc_search_plain without any device allocation, by this library or by the
- * caller: the same search, arguments, results and errors, except that the
- * workspace is a fixed HDC_NOALLOC_SCRATCH_BYTES array that the library
- * places in device memory once, when the GPU loads it.  It has no
+ * caller: the same arguments, results and errors, except that the workspace
+ * is a fixed HDC_NOALLOC_SCRATCH_BYTES array that the library places in device
+ * memory once, when the GPU loads it.  A search whose converted rows and lists
+ * fit there (some 800 queries and references in all at dim 8,192) runs on the
+ * tensor cores, a larger one on CUDA cores (30 to 60 times slower than
+ * hdc_search_plain with its full workspace).  It has no
  * counterpart in the reference (whose launch_cosine_topk allocates and frees
  * its buffers on every call, src/cosine.cu:455-494).
  *
@@ -292,7 +302,11 @@ int hdc_search_plain_noalloc(hdc_context* ctx, const int16_t* d_q, const int64_t
                              double* d_cos, int64_t* d_dot, void* stream);
 
 /* Schedule of hdc_search_tc on this context (no reference counterpart; the
- * knobs an autotuner varies): group_tiles = query tiles of 128 that run
+ * knobs an autotuner varies).  The search forms of a database plan themselves:
+ * these settings, and the HDC_TC_* ones below but HDC_TC_SCATTER, are the limb
+ * search's, and any of them other than automatic (0, -1, 0, 0; tile_n 128 counts
+ * as automatic too) selects it, at less than half the speed where the database
+ * has a form.  group_tiles = query tiles of 128 that run
  * together (0: automatic), the persistent grid being group_tiles x
  * (SMs / group_tiles) CTAs, each group's reference tiles dealt round-robin
  * to the SMs / group_tiles lanes; l2_policy = 0 no L2 hint, 1 query tiles
@@ -529,7 +543,9 @@ int hdc_pipeline_run(hdc_pipeline* p, const char* bytes, const int64_t* off, con
 int hdc_pipeline_launch_resident(hdc_pipeline* p);
 void* hdc_pipeline_stream(hdc_pipeline* p);
 /* Time the tensor-core schedules of hdc_search_tc_tuning on the pipeline's
- * buffers, keep the fastest on the context and re-capture the graphs.
+ * buffers, keep the fastest on the context and re-capture the graphs: the
+ * automatic one first (0, -1, 128, 0), which wins where the database has a
+ * search form, then the limb search's.
  * Outputs (optional): the chosen knobs and the search time in ms. */
 int hdc_pipeline_autotune(hdc_pipeline* p, int* group_tiles, int* l2_policy, int* tile_n, int* m_blocks,
                           float* ms);
